@@ -190,7 +190,9 @@ template <class T> struct Dft<T, 16> {
 // complex values the stride-R stores of the early Stockham stages and the
 // unit-stride loads both spread over all banks.
 __device__ __forceinline__ int fpad(int i) { return i + (i >> 3); }
-__host__ __device__ __forceinline__ int fft_buf_len(int M) { return M + (M >> 3) + 4; }
+// (An even count: a transform's second buffer, where rows are staged by 16-byte
+// copies, then starts on 16 bytes in FP32 too.)
+__host__ __device__ __forceinline__ int fft_buf_len(int M) { return (M + (M >> 3) + 5) & ~1; }
 // fpad(i + r S) for a compile-time stride S: when S is a multiple of 8 the
 // pad of i + r S is the pad of i plus r S / 8, so the index is affine in r
 // (one address per butterfly, constant offsets for its R values).
