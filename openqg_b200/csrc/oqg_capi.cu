@@ -168,13 +168,47 @@ static int ysolve_warps(int ny, long long ncols) {
     return W;
 }
 
+// The stages of a box transform of length M (oqg_odd.cuh): the radices of the
+// L = M / R0 points of a subsequence, then R0.
+static bool odd_radices(int M, std::vector<int> &rad) {
+    const int r0 = odd_r0(M), L = M / r0;
+    if (odd_ct_len(M)) {
+        rad = {odd_ra(L)};
+        if (L > rad[0]) rad.push_back(L / rad[0]);
+    } else if (!fft_radices(L, rad)) {
+        return false;
+    }
+    rad.push_back(r0);
+    return true;
+}
+
 // The transform kernels' instance for a basin's transform length: one built
 // for each length of the configurations' grids (boxes of 65 to 2049 points,
 // the 193-point channel; only that FFT plan in its code), the any-length one
-// otherwise (and for ensembles).
+// otherwise.  M = 0: an ensemble of several lengths.
 #define OQG_XLENS(X) X(128) X(192) X(256) X(384) X(512) X(1024) X(2048) X(4096)
+template <class T>
+static void (*bfwd_kernel(int M))(const BasinDev *, const Work *, int) {
+    switch (M) {
+#define OQG_BF(MM) case MM: return k_bfwd<T, MM>;
+        OQG_XLENS(OQG_BF)
+#undef OQG_BF
+        case 0: return k_bfwd<T, 0>;
+        default: return k_bfwd<T, -1>;
+    }
+}
+template <class T>
+static void (*binv_kernel(int M))(const BasinDev *, const Work *, int, int, int, double, T *) {
+    switch (M) {
+#define OQG_BI(MM) case MM: return k_binv<T, MM>;
+        OQG_XLENS(OQG_BI)
+#undef OQG_BI
+        case 0: return k_binv<T, 0>;
+        default: return k_binv<T, -1>;
+    }
+}
 template <class T, int E>
-static void (*xfwd_kernel(int M))(const BasinDev *, const Work *, const void *) {
+static void (*xfwd_kernel(int M))(const BasinDev *, const Work *, int) {
     // FP32 storage keeps the any-length instances below the in-place lengths:
     // at 513^2 the step measured 44.5 us with them against 48.1 us with the
     // per-length ones (which take 80 registers instead of 128), while at
@@ -188,15 +222,49 @@ static void (*xfwd_kernel(int M))(const BasinDev *, const Work *, const void *) 
         default: return k_xfwd<T, E>;
     }
 }
-template <class T, int NL, int E>
+template <class T, int E>
 static void (*xinv_rows_kernel(int M))(const BasinDev *, const Work *, int, int, int, double, T *) {
     if (std::is_same<T, float>::value && !fft_inplace_len(M)) M = 0;      // as xfwd_kernel
     switch (M) {
-#define OQG_XI(MM) case MM: return k_xinv_rows<T, NL, E, MM>;
+#define OQG_XI(MM) case MM: return k_xinv_rows<T, E, MM>;
         OQG_XLENS(OQG_XI)
 #undef OQG_XI
-        default: return k_xinv_rows<T, NL, E>;
+        default: return k_xinv_rows<T, E>;
     }
+}
+
+// The launches of the x-transforms.  cyclic: a channel's kernels; M: the
+// transform length (0: an ensemble of several); G: transforms per CTA (0: an
+// ensemble's members count their own); pdl: with programmatic stream
+// serialisation.
+struct XGeo {
+    bool cyclic;
+    int M, grid, block, G;
+    size_t smem;
+    cudaStream_t st;
+    const BasinDev *bas;
+    const Work *work;
+    bool pdl;
+};
+template <typename... KArgs, typename... Args>
+static void launch_x(const XGeo &x, int extra, void (*kern)(KArgs...), Args... args) {
+    if (x.pdl) launch_pdl(kern, x.grid + extra, x.block, x.smem, x.st, args...);
+    else kern<<<x.grid + extra, x.block, x.smem, x.st>>>(static_cast<KArgs>(args)...);
+}
+template <class T, int E>
+static void launch_fwd(const XGeo &x) {
+    if (x.cyclic) launch_x(x, 0, xfwd_kernel<T, E>(x.M), x.bas, x.work, x.G);
+    else launch_x(x, 0, bfwd_kernel<T>(x.M), x.bas, x.work, x.G);
+}
+// scal: scalar CTAs after the transforms'; out: the solve-only mode
+template <class T, int E>
+static void launch_inv(const XGeo &x, int scal, int par, double tdt, T *out) {
+    if (x.cyclic) launch_x(x, scal, xinv_rows_kernel<T, E>(x.M), x.bas, x.work, x.G, scal, par, tdt, out);
+    else launch_x(x, scal, binv_kernel<T>(x.M), x.bas, x.work, x.G, scal, par, tdt, out);
+}
+static XGeo xgeo(oqg_handle *h, bool fp64, bool pdl) {
+    return XGeo{h->hb.cyclic != 0, h->hb.M, h->nx, rup(h->xthreads, 32), h->xg, fp64 ? h->smem_x64 : h->smem_x, h->st,
+                fp64 ? h->d_bas64 : h->d_bas, h->d_wx, pdl};
 }
 
 // The vorticity kernel instance of a tile height (vort_tile_ok).
@@ -226,12 +294,12 @@ static void apply_xinv_sep(oqg_handle *h, bool on) {
 template <class T, int NL, int E>
 static void launch_step_t(oqg_handle *h, int par, double tdt) {
     const BasinDev &b = h->hb;
+    const XGeo x = xgeo(h, false, true);
     launch_pdl(vort_kernel<T, NL>(h->hb.vty), h->nv, VTHREADS, h->smem_v, h->st, h->d_bas, h->d_wv, par, tdt);
-    launch_pdl(xfwd_kernel<T, E>(b.M), h->nx, h->xthreads, h->smem_x, h->st, h->d_bas, h->d_wx, (const void *)nullptr);
+    launch_fwd<T, E>(x);
     launch_ysolve<T>(b.cyclic, h->yW, h->nys, h->smem_y, h->st, h->d_bas, h->d_wy, true);
     if (b.xinv_sep) {
-        launch_pdl(xinv_rows_kernel<T, NL, E>(b.M), h->nx + 1, rup(h->xthreads, 32), h->smem_x, h->st, h->d_bas, h->d_wx,
-                   h->xg, 1, par, tdt, (T *)nullptr);
+        launch_inv<T, E>(x, 1, par, tdt, nullptr);
         launch_pdl(k_xinv_asm<T, NL>, h->na, 256, 0, h->st, h->d_bas, (const Work *)h->d_wa, par);
     } else {
         launch_pdl(k_xinv<T, NL>, h->ni, h->xi_threads, h->smem_i, h->st, h->d_bas, h->d_wi, par, tdt,
@@ -245,23 +313,12 @@ static void launch_step_t(oqg_handle *h, int par, double tdt) {
 // in griddepcontrol.wait before its first dependent read).
 template <int NL, int E>
 static void launch_solve_t(oqg_handle *h, double *out, bool pdl) {
-    if (pdl) {
-        launch_pdl(xfwd_kernel<double, E>(h->hb.M), h->nx, h->xthreads, h->smem_x64, h->st, h->d_bas64, h->d_wx,
-                   (const void *)nullptr);
-        launch_ysolve<double>(h->hb.cyclic, h->yW, h->nys, h->smem_y, h->st, h->d_bas64, h->d_wy, true);
-        if (h->hb.xinv_sep)
-            launch_pdl(xinv_rows_kernel<double, NL, E>(h->hb.M), h->nx, rup(h->xthreads, 32), h->smem_x64, h->st, h->d_bas64,
-                       h->d_wx, h->xg, 0, 0, 0.0, out);
-        else
-            launch_pdl(k_xinv<double, NL>, h->ni, h->xi_threads, h->smem_i64, h->st, h->d_bas64, h->d_wi, 0, 0.0,
-                       out);
-        return;
-    }
-    xfwd_kernel<double, E>(h->hb.M)<<<h->nx, h->xthreads, h->smem_x64, h->st>>>(h->d_bas64, h->d_wx, nullptr);
-    launch_ysolve<double>(h->hb.cyclic, h->yW, h->nys, h->smem_y, h->st, h->d_bas64, h->d_wy, false);
-    if (h->hb.xinv_sep)
-        xinv_rows_kernel<double, NL, E>(h->hb.M)<<<h->nx, rup(h->xthreads, 32), h->smem_x64, h->st>>>(h->d_bas64, h->d_wx, h->xg,
-                                                                                        0, 0, 0.0, out);
+    const XGeo x = xgeo(h, true, pdl);
+    launch_fwd<double, E>(x);
+    launch_ysolve<double>(h->hb.cyclic, h->yW, h->nys, h->smem_y, h->st, h->d_bas64, h->d_wy, pdl);
+    if (h->hb.xinv_sep) launch_inv<double, E>(x, 0, 0, 0.0, out);
+    else if (pdl)
+        launch_pdl(k_xinv<double, NL>, h->ni, h->xi_threads, h->smem_i64, h->st, h->d_bas64, h->d_wi, 0, 0.0, out);
     else
         k_xinv<double, NL><<<h->ni, h->xi_threads, h->smem_i64, h->st>>>(h->d_bas64, h->d_wi, 0, 0.0, out);
 }
@@ -297,23 +354,28 @@ static void raise_ysolve_smem(size_t y) {
     raise_smem((const void *)k_ysolve<T, false, 4>, y);
 }
 
+template <class T, int E>
+static void raise_x_smem(bool cyclic, int M, size_t x) {
+    if (cyclic) {
+        raise_smem((const void *)xfwd_kernel<T, E>(M), x);
+        raise_smem((const void *)xinv_rows_kernel<T, E>(M), x);
+    } else {
+        raise_smem((const void *)bfwd_kernel<T>(M), x);
+        raise_smem((const void *)binv_kernel<T>(M), x);
+    }
+}
 template <class T, int NL, int E>
-static void raise_step_smem(size_t v, size_t x, size_t y, size_t i) {
+static void raise_step_smem(bool cyclic, int M, size_t v, size_t x, size_t y, size_t i) {
     for (int vt : {8, 12, 16}) raise_smem((const void *)vort_kernel<T, NL>(vt), v);
-    raise_smem((const void *)k_xfwd<T, E>, x);
-    raise_smem((const void *)k_xinv_rows<T, NL, E>, x);
-#define OQG_RX(MM) raise_smem((const void *)k_xfwd<T, E, MM>, x); raise_smem((const void *)k_xinv_rows<T, NL, E, MM>, x);
-    OQG_XLENS(OQG_RX)
-#undef OQG_RX
+    raise_x_smem<T, E>(cyclic, M, x);
     raise_ysolve_smem<T>(y);
     raise_smem((const void *)k_xinv<T, NL>, i);
 }
 
 template <class T, int NL, int E>
 static void set_attrs_t(oqg_handle *h) {
-    raise_step_smem<T, NL, E>(h->smem_v, h->smem_x, h->smem_y, h->smem_i);
-    raise_smem((const void *)xfwd_kernel<double, E>(h->hb.M), h->smem_x64);
-    raise_smem((const void *)xinv_rows_kernel<double, NL, E>(h->hb.M), h->smem_x64);
+    raise_step_smem<T, NL, E>(h->hb.cyclic, h->hb.M, h->smem_v, h->smem_x, h->smem_y, h->smem_i);
+    raise_x_smem<double, E>(h->hb.cyclic, h->hb.M, h->smem_x64);
     raise_ysolve_smem<double>(h->smem_y);
     raise_smem((const void *)k_xinv<double, NL>, h->smem_i64);
 }
@@ -614,12 +676,10 @@ static void launch_phase_t(oqg_handle *h, int phase, int par, double tdt) {
     const BasinDev &b = h->hb;
     switch (phase) {
         case 0: vort_kernel<T, NL>(b.vty)<<<h->nv, VTHREADS, h->smem_v, h->st>>>(h->d_bas, h->d_wv, par, tdt); break;
-        case 1: xfwd_kernel<T, E>(b.M)<<<h->nx, h->xthreads, h->smem_x, h->st>>>(h->d_bas, h->d_wx, nullptr); break;
+        case 1: launch_fwd<T, E>(xgeo(h, false, false)); break;
         case 2: launch_ysolve<T>(b.cyclic, h->yW, h->nys, h->smem_y, h->st, h->d_bas, h->d_wy, false); break;
         case 3:
-            if (b.xinv_sep)
-                xinv_rows_kernel<T, NL, E>(b.M)<<<h->nx + 1, rup(h->xthreads, 32), h->smem_x, h->st>>>(h->d_bas, h->d_wx, h->xg,
-                                                                                           1, par, tdt, nullptr);
+            if (b.xinv_sep) launch_inv<T, E>(xgeo(h, false, false), 1, par, tdt, nullptr);
             else
                 k_xinv<T, NL><<<h->ni, h->xi_threads, h->smem_i, h->st>>>(h->d_bas, h->d_wi, par, tdt, nullptr);
             break;
@@ -678,15 +738,13 @@ struct oqg_ensemble {
 template <class T, int NL, int E>
 static void launch_ens_step_t(oqg_ensemble *e, int par) {
     launch_pdl(vort_kernel<T, NL>(e->hb[0].vty), e->nv, VTHREADS, e->smem_v, e->st, e->d_bas, e->d_wv, par, 0.0);
-    // members of one transform length take that length's instance
-    launch_pdl(xfwd_kernel<T, E>(e->Mu), e->nx, e->xthreads, e->smem_x, e->st, e->d_bas, e->d_wx,
-               (const void *)nullptr);
+    // members of one transform length take that length's instance; each
+    // member's transforms per CTA follow from the CTA's threads (G = 0)
+    const XGeo x{e->cyclic != 0, e->Mu, e->nx, e->xthreads, 0, e->smem_x, e->st, e->d_bas, e->d_wx, true};
+    launch_fwd<T, E>(x);
     launch_ysolve<T>(e->cyclic, e->yW, e->nys, e->smem_y, e->st, e->d_bas, e->d_wy, true);
     if (e->sep) {
-        // per-member transform groups (G = 0) and one scalar CTA per member
-        const int nm = (int)e->m.size();
-        launch_pdl(xinv_rows_kernel<T, NL, E>(e->Mu), e->nx + nm, e->xthreads, e->smem_x, e->st, e->d_bas, e->d_wx,
-                   0, nm, par, 0.0, (T *)nullptr);
+        launch_inv<T, E>(x, (int)e->m.size(), par, 0.0, nullptr);    // one scalar CTA per member
         launch_pdl(k_xinv_asm<T, NL>, e->na, 256, 0, e->st, e->d_bas, (const Work *)e->d_wa, par);
     } else {
         launch_pdl(k_xinv<T, NL>, e->ni, e->xi_threads, e->smem_i, e->st, e->d_bas, e->d_wi, par, 0.0,
@@ -695,7 +753,7 @@ static void launch_ens_step_t(oqg_ensemble *e, int par) {
 }
 template <class T, int NL, int E>
 static void raise_ens_smem_t(oqg_ensemble *e) {
-    raise_step_smem<T, NL, E>(e->smem_v, e->smem_x, e->smem_y, e->smem_i);
+    raise_step_smem<T, NL, E>(e->cyclic, e->Mu, e->smem_v, e->smem_x, e->smem_y, e->smem_i);
 }
 static void launch_ens_step(oqg_ensemble *e, int par) { OQG_DISPATCH_E(launch_ens_step_t, e, e, par); }
 
@@ -899,6 +957,24 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     }
     CK(cudaMemcpy(d_tw64, tw.data(), tw.size() * sizeof(double), cudaMemcpyHostToDevice));
     b.tw = d_tw;
+    double *d_otw64 = nullptr;
+    if (!b.cyclic) {
+        std::vector<int> orad;
+        if (!odd_radices(b.M, orad) || (int)orad.size() > OQG_MAXRAD)
+            return bail(OQG_EUNSUPPORTED, "x-transform length must factor into 2, 3 and 5");
+        b.norad = (int)orad.size();
+        std::copy(orad.begin(), orad.end(), b.orad);
+        fft_stage_twiddles(b.M, orad, tw);
+        d_otw64 = dalloc<double>(h, tw.size());
+        CK(cudaMemcpy(d_otw64, tw.data(), tw.size() * sizeof(double), cudaMemcpyHostToDevice));
+        b.otw = d_otw64;
+        if (h->mixed) {
+            float *d_otw32 = dalloc<float>(h, tw.size());
+            std::vector<float> tf(tw.begin(), tw.end());
+            CK(cudaMemcpy(d_otw32, tf.data(), tf.size() * sizeof(float), cudaMemcpyHostToDevice));
+            b.otw = d_otw32;
+        }
+    }
     double *d_pt = dalloc<double>(h, pt.tab.size());
     int *d_po = dalloc<int>(h, pt.off.size()), *d_pl = dalloc<int>(h, pt.len.size());
     CK(cudaMemcpy(d_pt, pt.tab.data(), pt.tab.size() * sizeof(double), cudaMemcpyHostToDevice));
@@ -935,8 +1011,7 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     // ---- launch geometry
     // 16 values per transform thread: one radix-16 butterfly per stage
     h->E = 16;
-    const int TT = (b.M + h->E - 1) / h->E;
-    const size_t t2 = 2 * h->esz;
+    const int TT = b.cyclic ? (b.M + h->E - 1) / h->E : odd_tt(b.M);
     const int npm = (b.ny + 1) / 2;
     h->nv = b.tiles_x * b.tiles_y;
     // forward transform: one row pair per group, CTAs of >= 128 threads; a
@@ -959,8 +1034,12 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     const int LB = fft_buf_len(b.M);
     // the long lengths transform in place: one buffer plus two staged rows per group
     const size_t xrow = (size_t)((b.nxin + 3) & ~3);
-    h->smem_x = fft_inplace_len(b.M) ? (size_t)GX * (LB * t2 + 2 * xrow * h->esz) : (size_t)GX * 2 * LB * t2;
-    h->smem_x64 = fft_inplace_len(b.M) ? (size_t)GX * (LB * 16 + 2 * xrow * 8) : (size_t)GX * 2 * LB * 16;
+    auto xsmem = [&](size_t esz) -> size_t {
+        if (!b.cyclic) return (size_t)GX * odd_smem_len(b.M) * 2 * esz;
+        return fft_inplace_len(b.M) ? (size_t)GX * (LB * 2 * esz + 2 * xrow * esz) : (size_t)GX * 2 * LB * 2 * esz;
+    };
+    h->smem_x = xsmem(h->esz);
+    h->smem_x64 = xsmem(8);
     h->smem_y = (size_t)LDy * h->KB * vsz;
     // rows of an assembly CTA: k4_rows interior rows plus at most one wall row
     const int nra = (b.ny > b.k4_rows) ? b.k4_rows + 1 : b.ny + 2;
@@ -1018,6 +1097,7 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     make_tmaps(h);
     h->hb64 = b;
     h->hb64.tw = d_tw64;
+    h->hb64.otw = d_otw64;
     h->d_bas = dalloc<BasinDev>(h, 1);
     h->d_bas64 = dalloc<BasinDev>(h, 1);
     set_attrs(h);
@@ -1752,7 +1832,8 @@ int oqg_ensemble_create(const oqg_params *members, int nmembers, oqg_ensemble **
     // longest member if that is longer
     e->E = 16;
     e->xthreads = 128;
-    for (oqg_handle *h : e->m) e->xthreads = std::max(e->xthreads, rup((h->hb.M + e->E - 1) / e->E, 32));
+    auto xtt = [&](const BasinDev &b) { return b.cyclic ? (b.M + e->E - 1) / e->E : odd_tt(b.M); };
+    for (oqg_handle *h : e->m) e->xthreads = std::max(e->xthreads, rup(xtt(h->hb), 32));
     const size_t esz = e->m[0]->esz, t2 = 2 * esz, vsz = e->cyclic ? 16 : 8;
     // launch sizes per member, with the ensemble's E and fixed block sizes
     std::vector<int> order(nmembers);
@@ -1778,7 +1859,7 @@ int oqg_ensemble_create(const oqg_params *members, int nmembers, oqg_ensemble **
     }
     for (int i : order) {
         const BasinDev &b = e->m[i]->hb;
-        const int TT = (b.M + e->E - 1) / e->E;
+        const int TT = xtt(b);
         const int G = std::max(1, e->xthreads / TT);
         const int LB = fft_buf_len(b.M);
         const int npm = (b.ny + 1) / 2;
@@ -1794,7 +1875,8 @@ int oqg_ensemble_create(const oqg_params *members, int nmembers, oqg_ensemble **
         const int nra = (b.ny > b.k4_rows) ? b.k4_rows + 1 : b.ny + 2;
         e->smem_v = std::max(e->smem_v, vort_smem_bytes(b.vty, (int)esz));
         const size_t xrow = (size_t)((b.nxin + 3) & ~3);
-        e->smem_x = std::max(e->smem_x, fft_inplace_len(b.M) ? (size_t)G * (LB * t2 + 2 * xrow * esz)
+        e->smem_x = std::max(e->smem_x, !b.cyclic ? (size_t)G * odd_smem_len(b.M) * t2
+                                        : fft_inplace_len(b.M) ? (size_t)G * (LB * t2 + 2 * xrow * esz)
                                                                : (size_t)G * 2 * LB * t2);
         e->smem_y = std::max(e->smem_y, (size_t)ysolve_ld(b.ny, e->yW) * 4 * vsz);
         e->smem_i = std::max(e->smem_i, xinv_smem(b.M, b.nl, nra, b.nxp, nfft_e, esz, e->m[i]->xinv_split_needed));

@@ -84,6 +84,8 @@ struct BasinDev {
     void *rhs;                  // [nl][ny][pr] T
     void *spec;                 // [nl][ny][pk] T or T2
     const void *tw;             // [M] T2 per-stage FFT twiddles (fft_stage_twiddles)
+    const void *otw;            // box: [M] T2 twiddles of the pruned plan (oqg_odd.cuh)
+    int norad, orad[OQG_MAXRAD];   // its radices, the outer one last
     const double *piv_tab;      // Thomas pivots 1/(b - a gam), compressed
     const int *piv_off;         // [nl*nk] offset into piv_tab
     const int *piv_len;         // [nl*nk] stored length (beyond: fixed point)

@@ -28,6 +28,7 @@
 
 #include "oqg_dev.cuh"
 #include "oqg_fft.cuh"
+#include "oqg_odd.cuh"
 #include "oqg_tma.cuh"
 
 #include <type_traits>
@@ -650,16 +651,19 @@ k_vort(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
 // expanded into the first.  The stage twiddles are read from global memory.
 __host__ __device__ __forceinline__ int round16(int bytes) { return (bytes + 15) & ~15; }
 
-// MC > 0: an instance for transforms of length MC only (the host picks it
-// for a basin of that length); MC = 0 serves any length (ensembles).
+// A channel's forward transform (r2c of two rows by one complex FFT).  MC > 0:
+// an instance for transforms of length MC only (the host picks it for a basin
+// of that length); MC = 0 serves any length (ensembles).  G: transforms per
+// CTA (<= 0: an ensemble, as many as the CTA's threads serve).
 template <class T, int E, int MC = 0>
 __global__ void __launch_bounds__(256, 2)
-k_xfwd(const BasinDev *__restrict__ bas, const Work *__restrict__ work, const void *rhs_override) {
+k_xfwd(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int G) {
     typedef typename C2<T>::t T2;
     const Work w = work[blockIdx.x];
     const BasinDev &b = bas[w.member];
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int M = MC > 0 ? MC : b.M, TT = (M + E - 1) / E, G = blockDim.x / TT;
+    const int M = MC > 0 ? MC : b.M, TT = (M + E - 1) / E;
+    if (G <= 0) G = blockDim.x / TT;
     const int g = threadIdx.x / TT, t = threadIdx.x - g * TT;
     const int LB = fft_buf_len(M);
     T2 *zs = reinterpret_cast<T2 *>(smem_raw);
@@ -678,8 +682,7 @@ k_xfwd(const BasinDev *__restrict__ bas, const Work *__restrict__ work, const vo
     T2 *zb = za + LB;
     T *raw = ip ? reinterpret_cast<T *>(zs + (size_t)G * LB) + (size_t)(g < G ? g : 0) * 2 * RO
                 : reinterpret_cast<T *>(zb);
-    const T *R = (const T *)(rhs_override ? rhs_override : b.rhs);
-    const T *x = R + ((size_t)m * b.ny + j) * b.pr;
+    const T *x = (const T *)b.rhs + ((size_t)m * b.ny + j) * b.pr;
     pdl_trigger();
     pdl_wait();
     if (live) {
@@ -689,31 +692,11 @@ k_xfwd(const BasinDev *__restrict__ bas, const Work *__restrict__ work, const vo
     cp_async_commit_wait_all();
     __syncthreads();
     if (live) {
-        if (!b.cyclic) {
-            // odd extension of two rows: z_0 = z_{n+1} = 0, z_{M-jj} = -z_jj
-            if (t == 0) {
-                T2 zero;
-                zero.x = (T)0;
-                zero.y = (T)0;
-                za[fpad(0)] = zero;
-                za[fpad(n + 1)] = zero;
-            }
-            for (int jj = 1 + t; jj <= n; jj += TT) {
-                T2 v, vm;
-                v.x = raw[jj - 1];
-                v.y = two ? raw[RO + jj - 1] : (T)0;
-                vm.x = -v.x;
-                vm.y = -v.y;
-                za[fpad(jj)] = v;
-                za[fpad(M - jj)] = vm;
-            }
-        } else {
-            for (int jj = t; jj < M; jj += TT) {
-                T2 v;
-                v.x = raw[jj];
-                v.y = two ? raw[RO + jj] : (T)0;
-                za[fpad(jj)] = v;
-            }
+        for (int jj = t; jj < M; jj += TT) {
+            T2 v;
+            v.x = raw[jj];
+            v.y = two ? raw[RO + jj] : (T)0;
+            za[fpad(jj)] = v;
         }
     }
     __syncthreads();
@@ -721,32 +704,83 @@ k_xfwd(const BasinDev *__restrict__ bas, const Work *__restrict__ work, const vo
     if (ip) fft_inplace<T, MC>(za, M, (const T2 *)b.tw, live ? t : M, 0, 0);
     else z = fft_run<T, E, MC>(za, zb, M, b.rad, b.nrad, (const T2 *)b.tw, live ? t : TT, TT, 0, 0);
     if (!live) return;
-    if (!b.cyclic) {
-        T *S = (T *)b.spec;
-        T *sx = S + ((size_t)m * b.ny + j) * b.pk;
-        T *sy = sx + b.pk;
-        for (int kk = t; kk < n; kk += TT) {
-            const T2 v = z[fpad(kk + 1)];
-            sx[kk] = -v.y;
-            if (two) sy[kk] = v.x;
+    T2 *S = (T2 *)b.spec;
+    T2 *sx = S + ((size_t)m * b.ny + j) * b.pk;
+    T2 *sy = sx + b.pk;
+    for (int kk = t; kk < b.nk; kk += TT) {
+        const T2 a = z[fpad(kk)], c = z[fpad((M - kk) % M)];
+        T2 X, Y;
+        X.x = (T)0.5 * (a.x + c.x);
+        X.y = (T)0.5 * (a.y - c.y);
+        // (a - conj(c)) / (2i)
+        const T dx_ = (T)0.5 * (a.x - c.x), dy_ = (T)0.5 * (a.y + c.y);
+        Y.x = dy_;
+        Y.y = -dx_;
+        sx[kk] = X;
+        if (two) sy[kk] = Y;
+    }
+}
+
+// ------------------------------------------------------------------ k_bfwd
+// Stages a row pair x, y (n values each, times f) as the complex input of one
+// box transform (oqg_odd.cuh): value i at zpad<4>(i + 1), zero at both ends.
+// Eight loads of each row are in flight per thread; they bypass L1 (every
+// value is read once).
+template <class T>
+__device__ __forceinline__ void odd_stage_rows(typename C2<T>::t *z, const T *__restrict__ x, const T *__restrict__ y,
+                                               bool two, int n, T f, int t, int TT) {
+    constexpr int U = 8;
+    typename C2<T>::t zero;
+    zero.x = zero.y = (T)0;
+    if (t == 0) { z[0] = zero; z[zpad<4>(n + 1)] = zero; }
+    for (int i0 = t; i0 < n; i0 += U * TT) {
+        T a[U], c[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = i0 + u * TT;
+            a[u] = i < n ? __ldcg(x + i) : (T)0;
+            c[u] = two && i < n ? __ldcg(y + i) : (T)0;
         }
-    } else {
-        T2 *S = (T2 *)b.spec;
-        T2 *sx = S + ((size_t)m * b.ny + j) * b.pk;
-        T2 *sy = sx + b.pk;
-        for (int kk = t; kk < b.nk; kk += TT) {
-            const T2 a = z[fpad(kk)], c = z[fpad((M - kk) % M)];
-            T2 X, Y;
-            X.x = (T)0.5 * (a.x + c.x);
-            X.y = (T)0.5 * (a.y - c.y);
-            // (a - conj(c)) / (2i)
-            const T dx_ = (T)0.5 * (a.x - c.x), dy_ = (T)0.5 * (a.y + c.y);
-            Y.x = dy_;
-            Y.y = -dx_;
-            sx[kk] = X;
-            if (two) sy[kk] = Y;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int i = i0 + u * TT;
+            typename C2<T>::t v;
+            v.x = f * a[u];
+            v.y = f * c[u];
+            if (i < n) z[zpad<4>(i + 1)] = v;
         }
     }
+}
+
+// A box's forward transform: DST-I of the modal right-hand side's row pairs
+// (oqg_odd.cuh).  A CTA holds G = b.xg transforms (an ensemble: as many as
+// its threads serve, G <= 0), numbered with the mode fastest.
+template <class T, int MC = 0>
+__global__ void __launch_bounds__(256, 2)
+k_bfwd(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int G) {
+    typedef typename C2<T>::t T2;
+    const Work w = work[blockIdx.x];
+    const BasinDev &b = bas[w.member];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int M = MC > 0 ? MC : b.M, TT = odd_tt(M);
+    if (G <= 0) G = blockDim.x / TT;
+    const int g = threadIdx.x / TT, t = threadIdx.x - g * TT;
+    const int npm = (b.ny + 1) >> 1;          // row pairs per mode
+    const int tr = w.block * G + g;
+    const bool live = g < G && tr < b.nl * npm;
+    const int pair = live ? tr / b.nl : 0, m = live ? tr - pair * b.nl : 0, j = 2 * pair;
+    const bool two = j + 1 < b.ny;
+    T2 *z = reinterpret_cast<T2 *>(smem_raw) + (size_t)(g < G ? g : 0) * odd_smem_len(M);
+    const T *x = (const T *)b.rhs + ((size_t)m * b.ny + j) * b.pr;
+    T *sx = (T *)b.spec + ((size_t)m * b.ny + j) * b.pk, *sy = sx + b.pk;
+    pdl_trigger();
+    pdl_wait();
+    if (live) odd_stage_rows<T>(z, x, x + b.pr, two, b.nxin, (T)1, t, TT);
+    __syncthreads();
+    odd_fft<T, MC>(z, M, b.orad, b.norad, (const T2 *)b.otw, t, TT, live, [&](int i, T2 v) {
+        sx[i - 1] = -v.y;
+        if (two) sy[i - 1] = v.x;
+    });
 }
 
 // ------------------------------------------------------------------ k_ysolve
@@ -1280,35 +1314,90 @@ __device__ __noinline__ void scalar_phase(const BasinDev &b, double tdt, int par
 
 // ------------------------------------------------------------------ k_xinv_rows
 // The inverse x-transforms of the y-solved spectral rows as a launch of
-// their own, shaped like k_xfwd (one row pair per group, the 2048- and
-// 4096-point box lengths in place), into the modal rows b.inh_g, which
-// k_xinv_asm assembles.  A box's inverse DST-I is the forward transform
-// scaled by ftnorm (inhomog.F90:200-211): the modal row j + 1 of mode m gets
-// the n interior values and zeros on both walls.  A channel's c2r
-// (inhomog.F90:214-255) fills every column, the last repeating the first.
-// The first and last row
-// pairs of a mode clear the wall rows 0 and nyp - 1 (into out instead of
-// inh_g when out != null: the solve-only mode).  A scalar CTA after the
-// transforms' runs a basin's scalar phase once into b.scal_g (the assembly
-// reads it there) and writes the basin's next scalar state.
-// G: transforms per CTA (the forward launch's; <= 0: blockDim / TT, per
-// member of an ensemble), blockDim >= G TT rounded up to whole warps so the
-// scalar CTAs have a full warp.  scal: the last scal CTAs run the scalar
-// phase of member 0, 1, ... (0: none).
-template <class T, int NL, int E, int MC = 0>
+// their own, shaped like the forward one, into the modal rows b.inh_g, which
+// k_xinv_asm assembles (into out instead when out != null: the solve-only
+// mode).  The first and last row pairs of a mode clear the wall rows 0 and
+// nyp - 1.  The last scal CTAs run the scalar phase of member 0, 1, ... once
+// into its b.scal_g (the assembly reads it there) and write the member's next
+// scalar state (scal = 0: none).
+template <class T>
+__device__ __forceinline__ bool xinv_scalar_cta(const BasinDev *__restrict__ bas, int scal, int par, double tdt) {
+    if (scal <= 0 || (int)blockIdx.x < (int)gridDim.x - scal) return false;
+    pdl_trigger();
+    pdl_wait();
+    if (threadIdx.x < 32) {
+        const BasinDev &b = bas[blockIdx.x - (gridDim.x - scal)];
+        const double dt = tdt != 0.0 ? tdt : b.tdt_m;
+        XinvScal *sc = (XinvScal *)b.scal_g;
+        if (b.nl == 2) scalar_phase<T, 2>(b, dt, par, true, sc);
+        else if (b.nl == 3) scalar_phase<T, 3>(b, dt, par, true, sc);
+        else scalar_phase<T, 4>(b, dt, par, true, sc);
+    }
+    return true;
+}
+template <class T>
+__device__ __forceinline__ void xinv_wall_rows(const BasinDev &b, T *inh, int m, int j, int t, int TT) {
+    const int nxp = b.nxp, px = b.px;
+    if (j == 0) {
+        T *first = inh + (size_t)m * b.nyp * px;
+        for (int i = t; i < nxp; i += TT) first[i] = (T)0;
+    }
+    if (j + 2 >= b.ny) {
+        T *last = inh + ((size_t)m * b.nyp + b.nyp - 1) * px;
+        for (int i = t; i < nxp; i += TT) last[i] = (T)0;
+    }
+}
+
+// A box: the inverse DST-I is the forward transform scaled by ftnorm
+// (inhomog.F90:200-211); the modal row j + 1 gets the n interior values and
+// zeros on both walls.  G: transforms per CTA as in k_bfwd; the scalar CTAs
+// need a full warp, so blockDim is a multiple of 32.
+template <class T, int MC = 0>
+__global__ void __launch_bounds__(256, 2)
+k_binv(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int G, int scal, int par, double tdt, T *out) {
+    typedef typename C2<T>::t T2;
+    if (xinv_scalar_cta<T>(bas, scal, par, tdt)) return;
+    const Work w = work[blockIdx.x];
+    const BasinDev &b = bas[w.member];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int M = MC > 0 ? MC : b.M, TT = odd_tt(M);
+    if (G <= 0) G = blockDim.x / TT;
+    const int g = threadIdx.x / TT, t = threadIdx.x - g * TT;
+    const int npm = (b.ny + 1) >> 1;
+    const int tr = w.block * G + g;
+    const bool live = g < G && tr < b.nl * npm;
+    const int pair = live ? tr / b.nl : 0, m = live ? tr - pair * b.nl : 0, j = 2 * pair;
+    const bool two = j + 1 < b.ny;
+    T2 *z = reinterpret_cast<T2 *>(smem_raw) + (size_t)(g < G ? g : 0) * odd_smem_len(M);
+    const T *x = (const T *)b.spec + ((size_t)m * b.ny + j) * b.pk;
+    T *inh = out ? out : (T *)b.inh_g;
+    const int n = b.nxin, px = b.px;
+    T *ox = inh + ((size_t)m * b.nyp + j + 1) * px, *oy = ox + px;
+    pdl_trigger();
+    pdl_wait();
+    if (live) odd_stage_rows<T>(z, x, x + b.pk, two, n, (T)b.ftnorm, t, TT);
+    __syncthreads();
+    odd_fft<T, MC>(z, M, b.orad, b.norad, (const T2 *)b.otw, t, TT, live, [&](int i, T2 v) {
+        ox[i] = -v.y;
+        if (two) oy[i] = v.x;
+    });
+    if (!live) return;
+    if (t == 0) {
+        ox[0] = ox[n + 1] = (T)0;
+        if (two) oy[0] = oy[n + 1] = (T)0;
+    }
+    xinv_wall_rows(b, inh, m, j, t, TT);
+}
+
+// A channel: the c2r (inhomog.F90:214-255) of two rows by one complex
+// transform fills every column, the last repeating the first.  G <= 0:
+// blockDim / TT, per member of an ensemble.
+template <class T, int E, int MC = 0>
 __global__ void __launch_bounds__(256, 2)
 k_xinv_rows(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int G, int scal, int par,
             double tdt, T *out) {
     typedef typename C2<T>::t T2;
-    if (scal > 0 && (int)blockIdx.x >= (int)gridDim.x - scal) {
-        pdl_trigger();
-        pdl_wait();
-        if (threadIdx.x < 32) {
-            const BasinDev &b = bas[blockIdx.x - (gridDim.x - scal)];
-            scalar_phase<T, NL>(b, tdt != 0.0 ? tdt : b.tdt_m, par, true, (XinvScal *)b.scal_g);
-        }
-        return;
-    }
+    if (xinv_scalar_cta<T>(bas, scal, par, tdt)) return;
     const Work w = work[blockIdx.x];
     const BasinDev &b = bas[w.member];
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1323,21 +1412,15 @@ k_xinv_rows(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int
     const int m = live ? pair / npm : 0;
     const int j = live ? 2 * (pair - m * npm) : 0;
     const bool two = live && (j + 1 < b.ny);
-    const int n = b.nxin, nxp = b.nxp, px = b.px;
-    // a spectral row: n reals (box) or nk complex values (channel); a channel
-    // transforms through the ping-pong pair, whose second buffer holds both
-    const bool cyc = b.cyclic != 0;
-    const int rowbytes = cyc ? b.nk * (int)sizeof(T2) : n * (int)sizeof(T);
+    const int px = b.px;
+    // a spectral row: nk complex values, staged in the second buffer
+    const int rowbytes = b.nk * (int)sizeof(T2);
     const int RO = round16(rowbytes) / (int)sizeof(T);   // offset of the second row (16-byte aligned)
-    const bool ip = E == 16 && !cyc && fft_inplace_len(M);
-    T2 *za = zs + (size_t)(g < G ? g : 0) * (ip ? LB : 2 * LB);
+    T2 *za = zs + (size_t)(g < G ? g : 0) * 2 * LB;
     T2 *zb = za + LB;
-    T *raw = ip ? reinterpret_cast<T *>(zs + (size_t)G * LB) + (size_t)(g < G ? g : 0) * 2 * RO
-                : reinterpret_cast<T *>(zb);
-    const size_t pitchb = (size_t)b.pk * (cyc ? sizeof(T2) : sizeof(T));
+    T *raw = reinterpret_cast<T *>(zb);
+    const size_t pitchb = (size_t)b.pk * sizeof(T2);
     const char *x = (const char *)b.spec + ((size_t)m * b.ny + j) * pitchb;
-    // out != null: solve-only mode, the modal solutions go straight to out
-    // ([nl][nyp][px], the same layout)
     T *inh = out ? out : (T *)b.inh_g;
     const T ftn = (T)b.ftnorm;
     pdl_trigger();
@@ -1348,9 +1431,8 @@ k_xinv_rows(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int
     }
     cp_async_commit_wait_all();
     __syncthreads();
-    if (live && cyc) {
-        // c2r by one complex transform of two rows: the Hermitian extension
-        // of X + iY, conjugated (inhomog.F90:214-255)
+    if (live) {
+        // the Hermitian extension of X + iY, conjugated
         const T2 *xr = reinterpret_cast<const T2 *>(raw), *yr = reinterpret_cast<const T2 *>(raw + RO);
         for (int kk = t; kk < M; kk += TT) {
             T2 X, Y;
@@ -1365,64 +1447,24 @@ k_xinv_rows(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int
             v.y = -(ftn * X.y + ftn * Y.x);
             za[fpad(kk)] = v;
         }
-    } else if (live) {
-        if (t == 0) {
-            T2 zero;
-            zero.x = (T)0;
-            zero.y = (T)0;
-            za[fpad(0)] = zero;
-            za[fpad(n + 1)] = zero;
-        }
-        for (int jj = 1 + t; jj <= n; jj += TT) {
-            T2 v, vm;
-            v.x = ftn * raw[jj - 1];
-            v.y = two ? ftn * raw[RO + jj - 1] : (T)0;
-            vm.x = -v.x;
-            vm.y = -v.y;
-            za[fpad(jj)] = v;
-            za[fpad(M - jj)] = vm;
-        }
     }
     __syncthreads();
-    T2 *z = za;
-    if (ip) fft_inplace<T, MC>(za, M, (const T2 *)b.tw, live ? t : M, 0, 0);
-    else z = fft_run<T, E, MC>(za, zb, M, b.rad, b.nrad, (const T2 *)b.tw, live ? t : TT, TT, 0, 0);
+    const T2 *z = fft_run<T, E, MC>(za, zb, M, b.rad, b.nrad, (const T2 *)b.tw, live ? t : TT, TT, 0, 0);
     if (!live) return;
     T *ox = inh + ((size_t)m * b.nyp + j + 1) * px;
     T *oy = ox + px;
-    if (cyc) {
-        // every column; column nxp-1 = M repeats column 0 (inhomog.F90:250)
-        for (int i = t; i < M; i += TT) {
-            const T2 v = z[fpad(i)];
-            ox[i] = v.x;
-            if (two) oy[i] = -v.y;
-        }
-        if (t == 0) {
-            const T2 v = z[fpad(0)];
-            ox[M] = v.x;
-            if (two) oy[M] = -v.y;
-        }
-    } else {
-        for (int kk = t; kk < n; kk += TT) {
-            const T2 v = z[fpad(kk + 1)];
-            ox[kk + 1] = -v.y;
-            if (two) oy[kk + 1] = v.x;
-        }
+    // every column; column nxp-1 = M repeats column 0 (inhomog.F90:250)
+    for (int i = t; i < M; i += TT) {
+        const T2 v = z[fpad(i)];
+        ox[i] = v.x;
+        if (two) oy[i] = -v.y;
     }
-    if (t == 0 && !cyc) {
-        ox[0] = (T)0;
-        ox[nxp - 1] = (T)0;
-        if (two) { oy[0] = (T)0; oy[nxp - 1] = (T)0; }
+    if (t == 0) {
+        const T2 v = z[fpad(0)];
+        ox[M] = v.x;
+        if (two) oy[M] = -v.y;
     }
-    // the wall rows (zonal walls of either geometry)
-    T *wrow = nullptr;
-    if (j == 0) wrow = inh + (size_t)m * b.nyp * px;
-    if (j + 2 >= b.ny) {
-        T *last = inh + ((size_t)m * b.nyp + b.nyp - 1) * px;
-        for (int i = t; i < nxp; i += TT) last[i] = (T)0;
-    }
-    if (wrow)
-        for (int i = t; i < nxp; i += TT) wrow[i] = (T)0;
+    xinv_wall_rows(b, inh, m, j, t, TT);
 }
 
 // ------------------------------------------------------------------ k_xinv
