@@ -47,6 +47,11 @@ __attribute__((visibility("hidden"))) int host_fail(int code, const char *msg) {
 
 static inline int rup(int v, int m) { return (v + m - 1) / m * m; }
 
+// The y-solve instance for R rows per thread and KB columns per group, in the
+// box (real) or channel (complex) form.
+struct YGeo {
+    int R, KB, grid, block;
+};
 struct oqg_handle {
     int dev = 0;
     cudaStream_t st = nullptr;
@@ -58,14 +63,15 @@ struct oqg_handle {
     std::vector<void *> allocs;
     Work *d_wv = nullptr, *d_wx = nullptr, *d_wy = nullptr, *d_wi = nullptr;
     Work *d_wa = nullptr;                // k_xinv_asm work items
-    int nv = 0, nx = 0, nys = 0, ni = 0;
-    int E = 8, KB = 16, xthreads = 128, xi_threads = 64;
-    int yW = 1;                          // warps per y-solve column
+    int nv = 0, nx = 0, ni = 0;
+    int E = 8, xthreads = 128, xi_threads = 64;
+    int yW = 1;                          // spread of a y-solve column as set or tuned
+    YGeo yg{};                           // the y-solve's launch
     bool xinv_split_needed = false;      // the modal rows do not fit in shared memory
     size_t smem_i_full = 0, smem_i64_full = 0;   // k_xinv's shared memory when it transforms
     int na = 0;                          // CTAs of k_xinv_asm
     int xg = 1;                          // transforms per CTA of k_xfwd and k_xinv_rows
-    size_t smem_v = 0, smem_x = 0, smem_x64 = 0, smem_y = 0, smem_i = 0, smem_i64 = 0;
+    size_t smem_v = 0, smem_x = 0, smem_x64 = 0, smem_i = 0, smem_i64 = 0;
     double *stage[2] = {nullptr, nullptr};
     double *hrow = nullptr;     // contiguous host-order copy buffer [nl][nyp][nxp]
     double *dg = nullptr;       // qg_diagno scratch, made on its first call
@@ -134,38 +140,44 @@ static void launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem,
     cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
-// The y-solve instance for a column spread over W warps (1, 2 or 4) in the
-// box (real) or channel (complex) form.
-template <class T, bool CPLX, int W>
-static void ysolve_w(int grid, size_t smem, cudaStream_t st, const BasinDev *bas, const Work *wy, bool pdl) {
-    if (pdl) launch_pdl(k_ysolve<T, CPLX, W>, grid, 128 * W, smem, st, bas, wy);
-    else k_ysolve<T, CPLX, W><<<grid, 128 * W, smem, st>>>(bas, wy);
+template <class T, bool CPLX>
+static void (*ysolve_kernel(int R, int KB))(const BasinDev *, const Work *) {
+    constexpr int K = CPLX ? 4 : 8;
+    if (KB == 1) return k_ysolve<T, CPLX, YS_ROWS, 1>;
+    if (KB == 2) return k_ysolve<T, CPLX, YS_ROWS, 2>;
+    if (KB < K) return k_ysolve<T, CPLX, YS_ROWS, K / 2>;
+    return R == 4 ? k_ysolve<T, CPLX, 4, K> : R == 8 ? k_ysolve<T, CPLX, 8, K> : k_ysolve<T, CPLX, YS_ROWS, K>;
 }
 template <class T>
-static void launch_ysolve(bool cplx, int W, int grid, size_t smem, cudaStream_t st, const BasinDev *bas,
-                          const Work *wy, bool pdl) {
-    if (cplx) {
-        if (W == 4) ysolve_w<T, true, 4>(grid, smem, st, bas, wy, pdl);
-        else if (W == 2) ysolve_w<T, true, 2>(grid, smem, st, bas, wy, pdl);
-        else ysolve_w<T, true, 1>(grid, smem, st, bas, wy, pdl);
-    } else {
-        if (W == 4) ysolve_w<T, false, 4>(grid, smem, st, bas, wy, pdl);
-        else if (W == 2) ysolve_w<T, false, 2>(grid, smem, st, bas, wy, pdl);
-        else ysolve_w<T, false, 1>(grid, smem, st, bas, wy, pdl);
-    }
+static void launch_ysolve(bool cplx, const YGeo &y, cudaStream_t st, const BasinDev *bas, const Work *wy, bool pdl) {
+    auto fn = cplx ? ysolve_kernel<T, true>(y.R, y.KB) : ysolve_kernel<T, false>(y.R, y.KB);
+    if (pdl) launch_pdl(fn, y.grid, y.block, 0, st, bas, wy);
+    else fn<<<y.grid, y.block, 0, st>>>(bas, wy);
 }
-// Warps per y-solve column for ncols columns of ny rows: enough that the
-// columns put about 20 warps on each of the 148 SMs, as long as every warp
-// keeps 4 or more rows per lane and no lane more than 8 (the register path
-// within the instance's register budget).
+// The y-solve's shape for ncb column groups of ny rows spread by W: several
+// groups share a CTA of about 128 threads where that leaves a CTA to every SM.
+static YGeo ysolve_geo(int ny, int nk, int nl, bool cplx, int W) {
+    YGeo y;
+    y.KB = ysolve_kb(ny, cplx);
+    y.R = ysolve_rows(ny, cplx, W);
+    const int wg = ysolve_group_warps(ny, y.R, y.KB), ncb = nl * ((nk + y.KB - 1) / y.KB);
+    const int G = std::max(1, std::min(4 / wg, ncb / 148));
+    y.block = 32 * wg * G;
+    y.grid = (ncb + G - 1) / G;
+    return y;
+}
+// Column groups of a basin (the work list has room for one per CTA).
+static int ysolve_groups(const BasinDev &b) { return b.nl * ((b.nk + b.ykb - 1) / b.ykb); }
+// Spread of a y-solve column (oqg_set_ysolve_warps): the middle one.
 static int ysolve_warps(int ny, long long ncols) {
-    int W = 1;
-    while (W < 4 && ncols * W < 148LL * 20) {
-        const int W2 = 2 * W;
-        if (ny <= 32 * W * 4 || ny > 32 * W2 * 8) break;
-        W = W2;
-    }
-    return W;
+    (void)ny;
+    (void)ncols;
+    return 2;
+}
+// Whether this build takes columns of ny rows at spread W (values of vsz bytes).
+static bool ysolve_fits(int ny, int W, int vsz) {
+    const int L = 32 * W, s = ny <= 4 * L ? 4 : ny <= 8 * L ? 8 : ny <= 16 * L ? 16 : (ny + L - 1) / L;
+    return (size_t)std::max((ny + 32) | 1, (L * (s + 1) + 1) | 1) * 4 * vsz <= 227 * 1024;
 }
 
 // The stages of a box transform of length M (oqg_odd.cuh): the radices of the
@@ -297,7 +309,7 @@ static void launch_step_t(oqg_handle *h, int par, double tdt) {
     const XGeo x = xgeo(h, false, true);
     launch_pdl(vort_kernel<T, NL>(h->hb.vty), h->nv, VTHREADS, h->smem_v, h->st, h->d_bas, h->d_wv, par, tdt);
     launch_fwd<T, E>(x);
-    launch_ysolve<T>(b.cyclic, h->yW, h->nys, h->smem_y, h->st, h->d_bas, h->d_wy, true);
+    launch_ysolve<T>(b.cyclic, h->yg, h->st, h->d_bas, h->d_wy, true);
     if (b.xinv_sep) {
         launch_inv<T, E>(x, 1, par, tdt, nullptr);
         launch_pdl(k_xinv_asm<T, NL>, h->na, 256, 0, h->st, h->d_bas, (const Work *)h->d_wa, par);
@@ -315,7 +327,7 @@ template <int NL, int E>
 static void launch_solve_t(oqg_handle *h, double *out, bool pdl) {
     const XGeo x = xgeo(h, true, pdl);
     launch_fwd<double, E>(x);
-    launch_ysolve<double>(h->hb.cyclic, h->yW, h->nys, h->smem_y, h->st, h->d_bas64, h->d_wy, pdl);
+    launch_ysolve<double>(h->hb.cyclic, h->yg, h->st, h->d_bas64, h->d_wy, pdl);
     if (h->hb.xinv_sep) launch_inv<double, E>(x, 0, 0, 0.0, out);
     else if (pdl)
         launch_pdl(k_xinv<double, NL>, h->ni, h->xi_threads, h->smem_i64, h->st, h->d_bas64, h->d_wi, 0, 0.0, out);
@@ -344,16 +356,6 @@ static void raise_smem(const void *fn, size_t bytes) {
         g_smem_set.push_back({{dev, fn}, (int)bytes});
 }
 
-template <class T>
-static void raise_ysolve_smem(size_t y) {
-    raise_smem((const void *)k_ysolve<T, true, 1>, y);
-    raise_smem((const void *)k_ysolve<T, true, 2>, y);
-    raise_smem((const void *)k_ysolve<T, true, 4>, y);
-    raise_smem((const void *)k_ysolve<T, false, 1>, y);
-    raise_smem((const void *)k_ysolve<T, false, 2>, y);
-    raise_smem((const void *)k_ysolve<T, false, 4>, y);
-}
-
 template <class T, int E>
 static void raise_x_smem(bool cyclic, int M, size_t x) {
     if (cyclic) {
@@ -365,18 +367,16 @@ static void raise_x_smem(bool cyclic, int M, size_t x) {
     }
 }
 template <class T, int NL, int E>
-static void raise_step_smem(bool cyclic, int M, size_t v, size_t x, size_t y, size_t i) {
+static void raise_step_smem(bool cyclic, int M, size_t v, size_t x, size_t i) {
     for (int vt : {8, 12, 16}) raise_smem((const void *)vort_kernel<T, NL>(vt), v);
     raise_x_smem<T, E>(cyclic, M, x);
-    raise_ysolve_smem<T>(y);
     raise_smem((const void *)k_xinv<T, NL>, i);
 }
 
 template <class T, int NL, int E>
 static void set_attrs_t(oqg_handle *h) {
-    raise_step_smem<T, NL, E>(h->hb.cyclic, h->hb.M, h->smem_v, h->smem_x, h->smem_y, h->smem_i);
+    raise_step_smem<T, NL, E>(h->hb.cyclic, h->hb.M, h->smem_v, h->smem_x, h->smem_i);
     raise_x_smem<double, E>(h->hb.cyclic, h->hb.M, h->smem_x64);
-    raise_ysolve_smem<double>(h->smem_y);
     raise_smem((const void *)k_xinv<double, NL>, h->smem_i64);
 }
 
@@ -677,7 +677,7 @@ static void launch_phase_t(oqg_handle *h, int phase, int par, double tdt) {
     switch (phase) {
         case 0: vort_kernel<T, NL>(b.vty)<<<h->nv, VTHREADS, h->smem_v, h->st>>>(h->d_bas, h->d_wv, par, tdt); break;
         case 1: launch_fwd<T, E>(xgeo(h, false, false)); break;
-        case 2: launch_ysolve<T>(b.cyclic, h->yW, h->nys, h->smem_y, h->st, h->d_bas, h->d_wy, false); break;
+        case 2: launch_ysolve<T>(b.cyclic, h->yg, h->st, h->d_bas, h->d_wy, false); break;
         case 3:
             if (b.xinv_sep) launch_inv<T, E>(xgeo(h, false, false), 1, par, tdt, nullptr);
             else
@@ -709,10 +709,11 @@ struct oqg_ensemble {
     int na = 0;                        // k_xinv_asm work items
     bool sep = false;                  // boxes: k_xinv_rows + k_xinv_asm
     int Mu = 0;                        // the members' common transform length, else 0
-    int nv = 0, nx = 0, nys = 0, ni = 0;
-    size_t smem_v = 0, smem_x = 0, smem_y = 0, smem_i = 0;
+    int nv = 0, nx = 0, ni = 0;
+    size_t smem_v = 0, smem_x = 0, smem_i = 0;
     int xi_threads = 64, xthreads = 128;
-    int yW = 1;                        // warps per y-solve column, one for every member
+    int yW = 1;                        // spread of a y-solve column, one for every member
+    YGeo yg{};                         // the y-solve's launch
     int par = 0;
     cudaGraphExec_t gexec[2] = {nullptr, nullptr};
     std::vector<void *> allocs;
@@ -742,7 +743,7 @@ static void launch_ens_step_t(oqg_ensemble *e, int par) {
     // member's transforms per CTA follow from the CTA's threads (G = 0)
     const XGeo x{e->cyclic != 0, e->Mu, e->nx, e->xthreads, 0, e->smem_x, e->st, e->d_bas, e->d_wx, true};
     launch_fwd<T, E>(x);
-    launch_ysolve<T>(e->cyclic, e->yW, e->nys, e->smem_y, e->st, e->d_bas, e->d_wy, true);
+    launch_ysolve<T>(e->cyclic, e->yg, e->st, e->d_bas, e->d_wy, true);
     if (e->sep) {
         launch_inv<T, E>(x, (int)e->m.size(), par, 0.0, nullptr);    // one scalar CTA per member
         launch_pdl(k_xinv_asm<T, NL>, e->na, 256, 0, e->st, e->d_bas, (const Work *)e->d_wa, par);
@@ -753,9 +754,14 @@ static void launch_ens_step_t(oqg_ensemble *e, int par) {
 }
 template <class T, int NL, int E>
 static void raise_ens_smem_t(oqg_ensemble *e) {
-    raise_step_smem<T, NL, E>(e->cyclic, e->Mu, e->smem_v, e->smem_x, e->smem_y, e->smem_i);
+    raise_step_smem<T, NL, E>(e->cyclic, e->Mu, e->smem_v, e->smem_x, e->smem_i);
 }
 static void launch_ens_step(oqg_ensemble *e, int par) { OQG_DISPATCH_E(launch_ens_step_t, e, e, par); }
+
+// Column groups of a member in a y-solve CTA of the ensemble.
+static int ens_ygroups(const oqg_ensemble *e, const BasinDev &b) {
+    return std::max(1, e->yg.block / 32 / ysolve_group_warps(b.ny, e->yg.R, e->yg.KB));
+}
 
 static void ens_free(oqg_ensemble *e) {
     if (!e) return;
@@ -816,6 +822,25 @@ static void record_vty(const oqg_params &P, bool mixed, int vty) {
             return;
         }
     g_tuned.push_back(TunedVty{P.nxp, P.nyp, P.nl, P.cyclic != 0, (int)mixed, vty});
+}
+
+// The pivots of YS_PIVB adjacent wavenumbers interleaved row by row, up to the
+// longest of their lengths (k_ysolve reads them so); the columns past the last
+// wavenumber repeat it.
+static PivotTable pivot_blocks(const PivotTable &pt, int nl, int nk) {
+    PivotTable r;
+    for (int m = 0; m < nl; ++m)
+        for (int k0 = 0; k0 < nk; k0 += YS_PIVB) {
+            auto at = [&](int c) { return m * nk + std::min(k0 + c, nk - 1); };
+            int len = 0;
+            for (int c = 0; c < YS_PIVB; ++c) len = std::max(len, pt.len[at(c)]);
+            r.off.push_back((int)r.tab.size());
+            r.len.push_back(len);
+            for (int j = 0; j < len; ++j)
+                for (int c = 0; c < YS_PIVB; ++c)
+                    r.tab.push_back(pt.tab[pt.off[at(c)] + std::min(j, pt.len[at(c)] - 1)]);
+        }
+    return r;
 }
 
 static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
@@ -975,6 +1000,7 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
             b.otw = d_otw32;
         }
     }
+    pt = pivot_blocks(pt, b.nl, b.nk);
     double *d_pt = dalloc<double>(h, pt.tab.size());
     int *d_po = dalloc<int>(h, pt.off.size()), *d_pl = dalloc<int>(h, pt.len.size());
     CK(cudaMemcpy(d_pt, pt.tab.data(), pt.tab.size() * sizeof(double), cudaMemcpyHostToDevice));
@@ -1022,12 +1048,11 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     h->xthreads = GX * TT;
     h->xg = GX;
     h->nx = (b.nl * npm + GX - 1) / GX;
-    const size_t vsz = (size_t)(b.cyclic ? 16 : 8);
-    // y-solve: 4 columns (warps) per CTA; the padded column tile (pivots come through L1)
-    h->KB = 4;
     h->yW = ysolve_warps(b.ny, (long long)b.nl * b.nk);
-    const int LDy = ysolve_ld(b.ny, h->yW);
-    h->nys = b.nl * ((b.nk + h->KB - 1) / h->KB);
+    if (!ysolve_fits(b.ny, 1, b.cyclic ? 16 : 8))
+        return bail(OQG_EUNSUPPORTED, "grid too large for this build's shared-memory tiling");
+    h->yg = ysolve_geo(b.ny, b.nk, b.nl, b.cyclic, h->yW);
+    b.ykb = h->yg.KB;
     b.k4_rows = 2;
     h->ni = (b.ny + b.k4_rows - 1) / b.k4_rows;
     h->smem_v = vort_smem_bytes(b.vty, (int)h->esz);
@@ -1040,7 +1065,6 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     };
     h->smem_x = xsmem(h->esz);
     h->smem_x64 = xsmem(8);
-    h->smem_y = (size_t)LDy * h->KB * vsz;
     // rows of an assembly CTA: k4_rows interior rows plus at most one wall row
     const int nra = (b.ny > b.k4_rows) ? b.k4_rows + 1 : b.ny + 2;
     int nfft_i = xinv_fft_threads(b.M, b.nl);
@@ -1074,13 +1098,13 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     // 513^2 and the only form once the modal rows leave shared memory);
     // channels start with the one-kernel form (oqg_autotune_xinv measures both)
     apply_xinv_sep(h, !b.cyclic || split);
-    if (h->smem_i64_full > 227 * 1024 || h->smem_x64 > 227 * 1024 || h->smem_y > 227 * 1024)
+    if (h->smem_i64_full > 227 * 1024 || h->smem_x64 > 227 * 1024)
         return bail(OQG_EUNSUPPORTED, "grid too large for this build's shared-memory tiling");
-    std::vector<Work> wv(h->nv), wx(h->nx), wy(h->nys), wi(h->ni), wa(h->na);
+    std::vector<Work> wv(h->nv), wx(h->nx), wy(ysolve_groups(b)), wi(h->ni), wa(h->na);
     for (int i = 0; i < h->na; ++i) wa[i] = Work{0, i};
     for (int i = 0; i < h->nv; ++i) wv[i] = Work{0, i};
     for (int i = 0; i < h->nx; ++i) wx[i] = Work{0, i};
-    for (int i = 0; i < h->nys; ++i) wy[i] = Work{0, i};
+    for (size_t i = 0; i < wy.size(); ++i) wy[i] = Work{0, (int)i};
     for (int i = 0; i < h->ni; ++i) wi[i] = Work{0, i};
     h->d_wv = dalloc<Work>(h, (size_t)b.tiles_x * ((P.nyp + 7) / 8));
     h->d_wx = dalloc<Work>(h, wx.size());
@@ -1700,7 +1724,7 @@ int oqg_launch_floor(oqg_handle *h, int nsteps, double *us_per_step) {
     if (!h || !us_per_step || nsteps < 1) return fail(OQG_EINVAL, "bad argument");
     struct Shape { int grid, block; size_t smem; };
     std::vector<Shape> sh = {{h->nv, VTHREADS, h->smem_v}, {h->nx, h->xthreads, h->smem_x},
-                             {h->nys, 128 * h->yW, h->smem_y}};
+                             {h->yg.grid, h->yg.block, 0}};
     if (h->hb.xinv_sep) {
         sh.push_back({h->nx + 1, rup(h->xthreads, 32), h->smem_x});
         sh.push_back({h->na, 256, 0});
@@ -1834,7 +1858,7 @@ int oqg_ensemble_create(const oqg_params *members, int nmembers, oqg_ensemble **
     e->xthreads = 128;
     auto xtt = [&](const BasinDev &b) { return b.cyclic ? (b.M + e->E - 1) / e->E : odd_tt(b.M); };
     for (oqg_handle *h : e->m) e->xthreads = std::max(e->xthreads, rup(xtt(h->hb), 32));
-    const size_t esz = e->m[0]->esz, t2 = 2 * esz, vsz = e->cyclic ? 16 : 8;
+    const size_t esz = e->m[0]->esz, t2 = 2 * esz;
     // launch sizes per member, with the ensemble's E and fixed block sizes
     std::vector<int> order(nmembers);
     for (int i = 0; i < nmembers; ++i) order[i] = i;
@@ -1856,6 +1880,11 @@ int oqg_ensemble_create(const oqg_params *members, int nmembers, oqg_ensemble **
         int ny_max = 0;
         for (oqg_handle *h : e->m) { cols += (long long)h->hb.nl * h->hb.nk; ny_max = std::max(ny_max, h->hb.ny); }
         e->yW = ysolve_warps(ny_max, cols);
+        // one shape for every member: the tallest's, with CTAs of its threads
+        // (shorter columns pack several groups into one)
+        e->yg = ysolve_geo(ny_max, 1, 1, e->cyclic, e->yW);
+        e->yg.block = std::max(e->yg.block, 128);
+        for (oqg_handle *h : e->m) h->hb.ykb = h->hb64.ykb = e->yg.KB;
     }
     for (int i : order) {
         const BasinDev &b = e->m[i]->hb;
@@ -1865,7 +1894,7 @@ int oqg_ensemble_create(const oqg_params *members, int nmembers, oqg_ensemble **
         const int npm = (b.ny + 1) / 2;
         const int nvb = b.tiles_x * b.tiles_y;
         const int nxb = (b.nl * npm + G - 1) / G;
-        const int nyb = b.nl * ((b.nk + 3) / 4);
+        const int nyb = (ysolve_groups(b) + ens_ygroups(e, b) - 1) / ens_ygroups(e, b);
         const int nib = (b.ny + b.k4_rows - 1) / b.k4_rows;
         for (int k = 0; k < nvb; ++k) wv.push_back(Work{i, k});
         for (int k = 0; k < nxb; ++k) wx.push_back(Work{i, k});
@@ -1878,14 +1907,13 @@ int oqg_ensemble_create(const oqg_params *members, int nmembers, oqg_ensemble **
         e->smem_x = std::max(e->smem_x, !b.cyclic ? (size_t)G * odd_smem_len(b.M) * t2
                                         : fft_inplace_len(b.M) ? (size_t)G * (LB * t2 + 2 * xrow * esz)
                                                                : (size_t)G * 2 * LB * t2);
-        e->smem_y = std::max(e->smem_y, (size_t)ysolve_ld(b.ny, e->yW) * 4 * vsz);
         e->smem_i = std::max(e->smem_i, xinv_smem(b.M, b.nl, nra, b.nxp, nfft_e, esz, e->m[i]->xinv_split_needed));
     }
     if (e->smem_x > 227 * 1024 || e->smem_i > 227 * 1024 || e->smem_v > 227 * 1024) {
         ens_free(e);
         return fail(OQG_EUNSUPPORTED, "ensemble member too large for the shared-memory tiling");
     }
-    e->nv = (int)wv.size(); e->nx = (int)wx.size(); e->nys = (int)wy.size(); e->ni = (int)wi.size();
+    e->nv = (int)wv.size(); e->nx = (int)wx.size(); e->yg.grid = (int)wy.size(); e->ni = (int)wi.size();
     e->na = (int)wa.size();
     e->wv_cap = wv.size();
     auto up = [&](const void *src, size_t bytes) -> void * {
@@ -2431,14 +2459,11 @@ static int set_vty(oqg_handle *h, int vt) {
     return push_desc(h);
 }
 
-// The y-solve spread over W warps per column: launch shape, shared memory,
-// the graphs.
+// The y-solve's columns spread by W: the launch shape, the graphs.
 static int set_ysolve_w(oqg_handle *h, int W) {
-    const size_t smem = (size_t)ysolve_ld(h->hb.ny, W) * h->KB * (h->hb.cyclic ? 16 : 8);
-    if (smem > 227 * 1024) return fail(OQG_EUNSUPPORTED, "y-solve tile too large");
+    if (!ysolve_fits(h->hb.ny, W, h->hb.cyclic ? 16 : 8)) return fail(OQG_EUNSUPPORTED, "y-solve tile too large");
     h->yW = W;
-    h->smem_y = smem;
-    set_attrs(h);
+    h->yg = ysolve_geo(h->hb.ny, h->hb.nk, h->hb.nl, h->hb.cyclic, W);
     drop_graphs(h);
     return OQG_OK;
 }

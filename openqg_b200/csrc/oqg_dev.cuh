@@ -86,15 +86,17 @@ struct BasinDev {
     const void *tw;             // [M] T2 per-stage FFT twiddles (fft_stage_twiddles)
     const void *otw;            // box: [M] T2 twiddles of the pruned plan (oqg_odd.cuh)
     int norad, orad[OQG_MAXRAD];   // its radices, the outer one last
-    const double *piv_tab;      // Thomas pivots 1/(b - a gam), compressed
-    const int *piv_off;         // [nl*nk] offset into piv_tab
-    const int *piv_len;         // [nl*nk] stored length (beyond: fixed point)
+    // Thomas pivots 1/(b - a gam) of blocks of 8 adjacent wavenumbers of a mode:
+    // [piv_len][8] from piv_off, up to the longest column's fixed point
+    const double *piv_tab;
+    const int *piv_off, *piv_len;   // [nl * ceil(nk / 8)]
     const double *dst_w;        // [nk] sum_i of the inverse DST basis (box)
     const void *hsb;            // box: [nl-1][nyp][px] T hom_sol_bc
     const double *hbt;          // channel: [nyp] barotropic homogeneous solution
     const double *hbc1, *hbc2;  // channel: [nl][nyp]
     double *part_tile;          // [tiles][nl][OQG_NQ]
-    double *part_col;           // [y-solve CTAs][2]: dst_w-weighted column sums and
+    int ykb;                    // columns of a y-solve group
+    double *part_col;           // [y-solve groups][2]: dst_w-weighted column sums and
                                 // their compensations
     DevState *st;               // [2] by step parity
     DevForcing *frc;

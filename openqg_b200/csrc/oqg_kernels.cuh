@@ -8,7 +8,7 @@
 //   k_xfwd   forward x-transform of solve_inhomog_box / _cyclic
 //            (qg/inhomog.F90:170-255): DST-I (box) or r2c FFT (channel).
 //   k_ysolve Thomas solve in y per (mode, wavenumber) (inhomog.F90:187-199),
-//            one to four warps per column as a warp-parallel affine scan.
+//            chunks of rows in registers, their affine maps scanned.
 //   k_xinv   inverse x-transform + homogeneous correction + modes_to_layers
 //            (modes.F90:268-284) + ocqbdy (vorsubs.F90:58-114) +
 //            suppress_comp_mode (driver.F90:174-189).  One warp of each CTA
@@ -784,19 +784,33 @@ k_bfwd(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int G) {
 }
 
 // ------------------------------------------------------------------ k_ysolve
-// One warp per wavenumber column; blockDim = 32*KB.  Tile [ny][KB] (FP64) in
-// shared memory; the forward and back substitutions of the Thomas algorithm
-// are affine recurrences, solved by a per-lane chunk pass, a warp scan of the
-// chunk maps and a second chunk pass.
+// Thomas solves in y (inhomog.F90:187-199), one column per (mode, wavenumber).
+// The lanes of a warp lie along the wavenumber: KB adjacent columns (64 bytes of
+// FP64) times 32 / KB chunks of R rows, so every load and store of a row is
+// whole sectors and a column's values stay in the registers of its threads
+// from load to store.  Both substitutions are affine recurrences with the same
+// coefficients e_j = -a beta_j:
+//   down   u_j = beta_j f_j + e_j u_{j-1},   up   w_j = u_j + e_j w_{j+1}.
+// A thread runs its R rows from a zero input (v_j) and keeps the products
+// P_j = e_s .. e_j; then u_j = v_j + P_j u_in, and the chunk's map of the up
+// sweep is known at once: w_s = sum P_{j-1} v_j + u_in sum P_{j-1} P_j + P w_in.
+// The chunk maps are scanned across the lanes by shuffles and across the warps
+// of a column group through shared memory (two barriers in all).
+//
+// Bound by latency.  The kernel this replaces staged four columns per CTA in
+// shared memory (32-byte rows; 16-byte ones in FP32 storage, half of each
+// sector unused) with the lanes along y: strided pivot loads and six passes
+// over the tile.
 template <class T, bool CPLX> struct YT;
 template <class T> struct YT<T, false> { typedef double v; typedef T g; };
 template <class T> struct YT<T, true> { typedef double2 v; typedef typename C2<T>::t g; };
 
 __device__ __forceinline__ double yt_zero(double) { return 0.0; }
 __device__ __forceinline__ double2 yt_zero(double2) { return make_double2(0.0, 0.0); }
-__device__ __forceinline__ double yt_axpy(double c, double d, double x) { return c + d * x; }
+// c + d x
+__device__ __forceinline__ double yt_axpy(double c, double d, double x) { return fma(d, x, c); }
 __device__ __forceinline__ double2 yt_axpy(double2 c, double d, double2 x) {
-    return make_double2(c.x + d * x.x, c.y + d * x.y);
+    return make_double2(fma(d, x.x, c.x), fma(d, x.y, c.y));
 }
 __device__ __forceinline__ double yt_scale(double f, double s) { return f * s; }
 __device__ __forceinline__ double2 yt_scale(double2 f, double s) { return make_double2(f.x * s, f.y * s); }
@@ -808,259 +822,170 @@ __device__ __forceinline__ double yt_load(float v) { return (double)v; }
 __device__ __forceinline__ double yt_load(double v) { return v; }
 __device__ __forceinline__ double2 yt_load(float2 v) { return make_double2(v.x, v.y); }
 __device__ __forceinline__ double2 yt_load(double2 v) { return v; }
-template <class G> __device__ __forceinline__ G yt_store(double v);
-template <> __device__ __forceinline__ double yt_store<double>(double v) { return v; }
-template <> __device__ __forceinline__ float yt_store<float>(double v) { return (float)v; }
-template <class G> __device__ __forceinline__ G yt_store2(double2 v);
-template <> __device__ __forceinline__ double2 yt_store2<double2>(double2 v) { return v; }
-template <> __device__ __forceinline__ float2 yt_store2<float2>(double2 v) { return make_float2((float)v.x, (float)v.y); }
-__device__ __forceinline__ double yt_re(double v) { return v; }
-__device__ __forceinline__ double yt_re(double2 v) { return v.x; }
-
-// The maps of the two sweeps compose across the lanes of a column: lane l's
-// rows give an affine map u_out = C + D u_in, and the lanes' maps are scanned
-// in sweep order.  A column spread over W warps also composes across them:
-// each warp publishes its aggregate map (lane 31 going down the rows, lane 0
-// going up) and a warp's carry-in is the composition of the warps before it.
-// Returns this lane's input value: its exclusive prefix applied to the carry.
-// Every thread of the CTA calls it (a CTA barrier when W > 1).
-template <class V, int W, bool DOWN>
-__device__ __forceinline__ V ysolve_scan(V C, double D, int lane, int wc, V *sC, double *sD) {
-    for (int q = 1; q < 32; q <<= 1) {
-        const V Co = DOWN ? yt_up(C, q) : yt_dn(C, q);
-        const double Do = DOWN ? shfl_up_d(D, q) : shfl_dn_d(D, q);
-        if (DOWN ? lane >= q : lane + q < 32) { C = yt_axpy(C, D, Co); D = D * Do; }
-    }
-    V Ce = DOWN ? yt_up(C, 1) : yt_dn(C, 1);
-    if constexpr (W == 1) {
-        if (lane == (DOWN ? 0 : 31)) Ce = yt_zero(V());
-        return Ce;
-    } else {
-        double De = DOWN ? shfl_up_d(D, 1) : shfl_dn_d(D, 1);
-        if (lane == (DOWN ? 0 : 31)) { Ce = yt_zero(V()); De = 1.0; }
-        if (lane == (DOWN ? 31 : 0)) { sC[wc] = C; sD[wc] = D; }
-        __syncthreads();
-        V u = yt_zero(V());
-        if (DOWN) { for (int v = 0; v < wc; ++v) u = yt_axpy(sC[v], sD[v], u); }
-        else { for (int v = W - 1; v > wc; --v) u = yt_axpy(sC[v], sD[v], u); }
-        return yt_axpy(Ce, De, u);
-    }
+template <class G> __device__ __forceinline__ G yt_store(double v) { return (G)v; }
+template <class G> __device__ __forceinline__ G yt_store(double2 v) {
+    G g;
+    g.x = v.x;
+    g.y = v.y;
+    return g;
 }
 
-// The column solve with each lane's rows [s, s+SM) held in registers through
-// all four passes: forward elimination as an affine scan (chunk pass, scan
-// of the chunk maps, chunk pass), then back substitution the same way from
-// the bottom.  Rows at or beyond ny are padding: their value and pivot are
-// zero, so they map everything to zero in both sweeps and the last row's
-// zero neighbour below needs no special case; the passes then run without
-// per-row predicates.  col: the column in shared memory at padded offset o;
-// piv: its pivots (global, plen stored); sC/sD: the column's W carry slots
-// of each sweep.
-#define YREG 16
-template <class V, int W, int SM>
-__device__ __forceinline__ void ysolve_chunk_regs(V *col, const double *__restrict__ piv, int plen, double a,
-                                                  int lane, int wc, int s, int o, int ny, V *sC, double *sD,
-                                                  CSum &colsum) {
-    V x[SM];
-    double bt[SM];
-#pragma unroll
-    for (int t = 0; t < SM; ++t) {
-        const bool in = s + t < ny;
-        x[t] = in ? col[o + t] : yt_zero(V());
-        bt[t] = in ? __ldg(piv + min(s + t, plen - 1)) : 0.0;
-    }
-    // forward elimination: u_j = f_j beta_j - a beta_j u_{j-1}
-    V C = yt_zero(V());
-    double D = 1.0;
-#pragma unroll
-    for (int t = 0; t < SM; ++t) {
-        C = yt_axpy(yt_scale(x[t], bt[t]), -a * bt[t], C);
-        D = -a * bt[t] * D;
-    }
-    V uu = ysolve_scan<V, W, true>(C, D, lane, wc, sC, sD);
-#pragma unroll
-    for (int t = 0; t < SM; ++t) {
-        uu = yt_axpy(yt_scale(x[t], bt[t]), -a * bt[t], uu);
-        x[t] = uu;
-    }
-    // back substitution: u_j = u'_j - a beta_j u_{j+1}
-    C = yt_zero(V());
-    D = 1.0;
-#pragma unroll
-    for (int t = SM - 1; t >= 0; --t) {
-        const double ej = -a * bt[t];
-        C = yt_axpy(x[t], ej, C);
-        D = ej * D;
-    }
-    uu = ysolve_scan<V, W, false>(C, D, lane, wc, sC + W, sD + W);
-#pragma unroll
-    for (int t = SM - 1; t >= 0; --t) {
-        const double ej = -a * bt[t];
-        uu = yt_axpy(x[t], ej, uu);
-        x[t] = uu;
-        // the box's dst_w-weighted column sum (a channel has none)
-        if constexpr (std::is_same<V, double>::value) colsum.add(yt_re(uu));
-    }
-#pragma unroll
-    for (int t = 0; t < SM; ++t)
-        if (s + t < ny) col[o + t] = x[t];
+#define YS_THREADS 512      // most threads of a CTA
+#define YS_PIVB 8           // columns of a pivot-table block
+#define YS_ROWS 16          // most rows per thread (values and pivots in registers)
+// Columns per group: 64 bytes of FP64, fewer when the rows need more threads.
+__host__ __device__ __forceinline__ int ysolve_kb(int ny, int cplx) {
+    for (int k = cplx ? 4 : 8; k > 1; k /= 2)
+        if ((ny + YS_ROWS - 1) / YS_ROWS * k <= YS_THREADS) return k;
+    return 1;
+}
+// Rows per thread of a column spread over about 25 W chunks: W = 1, 2, 4 trade
+// the length of a thread's chain for threads.  At W = 2 a step took (us, rows
+// 4 / 8 / 16): 257^2 29.8 / 30.0 / 30.6, 361 x 287 - / 42.7 / 43.7, 513^2
+// - / 51.4 / 50.2; 32 rows do not fit the registers (1025^2: 168 against 147
+// with 16).
+__host__ __device__ __forceinline__ int ysolve_rows(int ny, int cplx, int W) {
+    const int kb = ysolve_kb(ny, cplx);
+    int R = 4;
+    while (R < YS_ROWS && (R * 25 * W < ny || (ny + R - 1) / R * kb > YS_THREADS)) R *= 2;
+    return R;
+}
+// Warps of a group of kb columns.
+__host__ __device__ __forceinline__ int ysolve_group_warps(int ny, int R, int kb) {
+    return ((ny + R - 1) / R * kb + 31) / 32;
 }
 
-// Rows per lane of a column spread over W warps and the padded column
-// length of its tile: up to 32 W YREG rows the smallest of 4, 8 and 16 rows
-// per lane that covers them (the register path, one instance each), beyond
-// that ceil(ny / 32 W) rows per lane through shared memory.
-__host__ __device__ __forceinline__ int ysolve_rows_per_lane(int ny, int W) {
-    const int L = 32 * W;
-    return ny <= 4 * L ? 4 : ny <= 8 * L ? 8 : ny <= YREG * L ? YREG : (ny + L - 1) / L;
-}
-__host__ __device__ __forceinline__ int ysolve_ld(int ny, int W) {
-    const int s = ysolve_rows_per_lane(ny, W);
-    const int need = 32 * W * (s + 1) + 1;             // 32 W lanes of s rows, one pad each
-    const int ld = (ny + 32) | 1;
-    return ld > need ? ld : (need | 1);
-}
-
-// One column per W warps, 4 columns per CTA (blockDim = 128 W).  More warps
-// per column cut the rows each lane carries through the sweeps and put more
-// warps on the SMs when the grid has few columns.
-template <class T, bool CPLX, int W>
-__global__ void __launch_bounds__(128 * W, W == 1 ? 1 : W == 2 ? 3 : 1)
+template <class T, bool CPLX, int R, int KB>
+__global__ void __launch_bounds__(YS_THREADS, 1)
 k_ysolve(const BasinDev *__restrict__ bas, const Work *__restrict__ work) {
     typedef typename YT<T, CPLX>::v V;
     typedef typename YT<T, CPLX>::g Gm;
-    constexpr int KB = 4;                       // columns per CTA
-    constexpr int NT = 128 * W;                 // threads
-    constexpr int CH = 16 / W;                  // loads in flight per thread and pass
+    constexpr int MAXW = YS_THREADS / 32;
     const Work w = work[blockIdx.x];
     const BasinDev &b = bas[w.member];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int c = wid / W, wc = wid - c * W;    // column of the CTA, warp within it
-    const int nk = b.nk, ny = b.ny, pk = b.pk;
-    const int nkb = (nk + KB - 1) / KB;
-    const int m = w.block / nkb, k0 = (w.block - m * nkb) * KB;
-    // Lane l of warp wc owns rows [(32 wc + l) S, +S).  Columns are stored
-    // with one pad word per S rows (row j at j + j / S), so the 32 lanes of a
-    // warp reading their chunks hit distinct banks.
-    const int S_ = ysolve_rows_per_lane(ny, W);
-    const int LD = ysolve_ld(ny, W);            // > 32 W (S + 1), odd
-    const FastDiv fdS(S_);
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    V *tile = reinterpret_cast<V *>(smem_raw);                 // [KB][LD]
-    __shared__ V sC[KB][2 * W];                 // carries of the two sweeps
-    __shared__ double sD[KB][2 * W];
-    const int k = k0 + c;
-    const bool live = k < nk;
-    const int pidx = m * nk + (live ? k : 0);
-    // this column's pivots (constant data, read through L1); beyond the
-    // stored length a pivot repeats its fixed point
-    const double *__restrict__ piv = b.piv_tab + b.piv_off[pidx];
-    const int plen = b.piv_len[pidx];
-    Gm *S = (Gm *)b.spec + (size_t)m * ny * pk;
+    const int nk = b.nk, ny = b.ny, pk = b.pk, nl = b.nl;
+    const int WG = ysolve_group_warps(ny, R, KB), G = max(1, (int)(blockDim.x >> 5) / WG);
+    const int g = wid / WG, wg = wid - g * WG;  // group of the CTA, warp within it
+    const int ncb = (nk + KB - 1) / KB, cb = w.block * G + g;
+    const bool live = g < G && cb < nl * ncb;
+    const int m = live ? cb / ncb : 0, k0 = live ? (cb - m * ncb) * KB : 0;
+    const int col = lane % KB, rc = lane / KB, k = k0 + col;
+    const int s = (wg * (32 / KB) + rc) * R;    // this thread's first row
+    const bool on = live && k < nk;
+    __shared__ V sC[2][MAXW][KB];
+    __shared__ double sD[2][MAXW][KB];
+    __shared__ double part[2][MAXW];
+    // pivots of the table block's columns, [plen][YS_PIVB]; beyond the stored
+    // length a pivot repeats its fixed point
+    const int pb = m * ((nk + YS_PIVB - 1) / YS_PIVB) + k0 / YS_PIVB;
+    const int plen = b.piv_len[pb];
+    const double *__restrict__ piv = b.piv_tab + b.piv_off[pb] + k0 % YS_PIVB + col;
+    const double a = b.a_tri;
+    const bool flat = s >= plen - 1;            // every row of the thread has the fixed point
+    const double bt0 = __ldg(piv + (size_t)min(s, plen - 1) * YS_PIVB);
+    double bt[R];                               // zero, as the value, in rows at or beyond ny
+#pragma unroll
+    for (int t = 0; t < R; ++t)
+        bt[t] = s + t >= ny ? 0.0 : flat ? bt0 : __ldg(piv + (size_t)min(s + t, plen - 1) * YS_PIVB);
+    Gm *S = (Gm *)b.spec + ((size_t)m * ny + s) * pk + k;
     pdl_trigger();
     pdl_wait();
-    // load the spectral columns: thread -> (row, column), coalesced along k
-    for (int i0 = threadIdx.x; i0 < ny * KB; i0 += NT * CH) {
-        V v[CH];
+    V x[R];
+    {
+        Gm raw[R];
 #pragma unroll
-        for (int u = 0; u < CH; ++u) {
-            const int idx = i0 + NT * u;
-            const int jj = idx >> 2, cc = idx & 3, kk = k0 + cc;
-            v[u] = (idx < ny * KB && kk < nk) ? yt_load(S[(size_t)jj * pk + kk]) : yt_zero(V());
-        }
+        for (int t = 0; t < R; ++t)
+            if (on && s + t < ny) raw[t] = __ldcg(S + (size_t)t * pk);
 #pragma unroll
-        for (int u = 0; u < CH; ++u) {
-            const int idx = i0 + NT * u;
-            const int jj = idx >> 2, cc = idx & 3;
-            if (idx < ny * KB) tile[cc * LD + jj + fdS.div(jj)] = v[u];
-        }
+        for (int t = 0; t < R; ++t) x[t] = on && s + t < ny ? yt_load(raw[t]) : yt_zero(V());
     }
-    __syncthreads();
-
-    // Every warp runs the sweeps (a column past nk solves zeros) so that the
-    // carry barriers are uniform over the CTA.
-    const double a = b.a_tri;
-    V *col = tile + c * LD;
-    const int gl = wc * 32 + lane;
-    const int s = gl * S_, e = min(s + S_, ny);
-    const int o = gl * (S_ + 1);                // padded offset of row s
-    const int n = max(e - s, 0);
-    CSum colsum;
-    if (S_ == 4) ysolve_chunk_regs<V, W, 4>(col, piv, plen, a, lane, wc, s, o, ny, sC[c], sD[c], colsum);
-    else if (S_ == 8) ysolve_chunk_regs<V, W, 8>(col, piv, plen, a, lane, wc, s, o, ny, sC[c], sD[c], colsum);
-    // (16 rows per lane with one warp per column, and with four for the
-    // box; the two-warp instances run at most 8 within their register budget)
-    else if ((W == 1 || (W == 4 && !CPLX)) && S_ == YREG)
-        ysolve_chunk_regs<V, W, YREG>(col, piv, plen, a, lane, wc, s, o, ny, sC[c], sD[c], colsum);
-    else {
-        // forward elimination: u_j = f_j beta_j - a beta_j u_{j-1}
-        V C = yt_zero(V());
-        double D = 1.0;
-#pragma unroll 8
-        for (int t = 0; t < n; ++t) {
-            const double bt = __ldg(piv + min(s + t, plen - 1));
-            C = yt_axpy(yt_scale(col[o + t], bt), -a * bt, C);
-            D = -a * bt * D;
-        }
-        V uu = ysolve_scan<V, W, true>(C, D, lane, wc, sC[c], sD[c]);
-#pragma unroll 8
-        for (int t = 0; t < n; ++t) {
-            const double bt = __ldg(piv + min(s + t, plen - 1));
-            uu = yt_axpy(yt_scale(col[o + t], bt), -a * bt, uu);
-            col[o + t] = uu;
-        }
-        // back substitution: u_j = u'_j - a beta_j u_{j+1}
-        C = yt_zero(V());
-        D = 1.0;
-#pragma unroll 8
-        for (int t = n - 1; t >= 0; --t) {
-            const double ej = (s + t == ny - 1) ? 0.0 : -a * __ldg(piv + min(s + t, plen - 1));
-            C = yt_axpy(col[o + t], ej, C);
-            D = ej * D;
-        }
-        uu = ysolve_scan<V, W, false>(C, D, lane, wc, sC[c] + W, sD[c] + W);
-#pragma unroll 8
-        for (int t = n - 1; t >= 0; --t) {
-            const double ej = (s + t == ny - 1) ? 0.0 : -a * __ldg(piv + min(s + t, plen - 1));
-            uu = yt_axpy(col[o + t], ej, uu);
-            col[o + t] = uu;
-            if constexpr (std::is_same<V, double>::value) colsum.add(yt_re(uu));
-        }
-    }
-    // dst_w-weighted column sum (box), one compensated partial per warp
-    CSum wsum;
-    if (!CPLX) {
-        const CSum cw = csum_warp(colsum);
-        if (live) {
-            const double wk = b.dst_w[k];
-            wsum.add_prod(wk, cw.s);
-            wsum.add_prod(wk, cw.c);
-        }
-    }
-    __syncthreads();
-    for (int i0 = threadIdx.x; i0 < ny * KB; i0 += NT * CH) {
+    // the chunk from a zero input, and its map of the up sweep
+    V v = yt_zero(V()), A = yt_zero(V());
+    double P = 1.0, S2 = 0.0;
 #pragma unroll
-        for (int u = 0; u < CH; ++u) {
-            const int idx = i0 + NT * u;
-            const int jj = idx >> 2, cc = idx & 3, kk = k0 + cc;
-            if (idx < ny * KB && kk < nk) {
-                if constexpr (CPLX) S[(size_t)jj * pk + kk] = yt_store2<Gm>(tile[cc * LD + jj + fdS.div(jj)]);
-                else S[(size_t)jj * pk + kk] = yt_store<Gm>(tile[cc * LD + jj + fdS.div(jj)]);
-            }
-        }
+    for (int t = 0; t < R; ++t) {
+        const double be = bt[t], e = -a * be;
+        v = yt_axpy(yt_scale(x[t], be), e, v);
+        x[t] = v;
+        A = yt_axpy(A, P, v);
+        const double Pn = P * e;
+        S2 = fma(P, Pn, S2);
+        P = Pn;
     }
-    if (!CPLX) {
-        // the CTA's partial (sum, compensation), its warps merged in a fixed
-        // order
-        __shared__ double wpart[2 * KB * W];
-        if (lane == 0) { wpart[wid] = wsum.s; wpart[KB * W + wid] = wsum.c; }
+    // scan down: C + D u over the chunks above
+    V u;
+    {
+        V C = v;
+        double D = P;
+#pragma unroll
+        for (int o = KB; o < 32; o <<= 1) {
+            const V Co = yt_up(C, o);
+            const double Do = shfl_up_d(D, o);
+            if (lane >= o) { C = yt_axpy(C, D, Co); D *= Do; }
+        }
+        V Ce = yt_up(C, KB);
+        double De = shfl_up_d(D, KB);
+        if (rc == 0) { Ce = yt_zero(V()); De = 1.0; }
+        if (lane >= 32 - KB) { sC[0][wid][col] = C; sD[0][wid][col] = D; }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            CSum t;
+        u = yt_zero(V());
+        const int w0 = wid - wg;
+        for (int y = 0; y < wg; ++y) u = yt_axpy(sC[0][w0 + y][col], sD[0][w0 + y][col], u);
+        u = yt_axpy(Ce, De, u);
+    }
+    // scan up: the chunks below
+    V win;
+    {
+        V C = yt_axpy(A, S2, u);
+        double D = P;
 #pragma unroll
-            for (int x = 0; x < KB * W; ++x) t.merge(wpart[x], wpart[KB * W + x]);
-            b.part_col[2 * w.block] = t.s;
-            b.part_col[2 * w.block + 1] = t.c;
+        for (int o = KB; o < 32; o <<= 1) {
+            const V Co = yt_dn(C, o);
+            const double Do = shfl_dn_d(D, o);
+            if (lane + o < 32) { C = yt_axpy(C, D, Co); D *= Do; }
+        }
+        V Ce = yt_dn(C, KB);
+        double De = shfl_dn_d(D, KB);
+        if (rc == 32 / KB - 1) { Ce = yt_zero(V()); De = 1.0; }
+        if (lane < KB) { sC[1][wid][col] = C; sD[1][wid][col] = D; }
+        __syncthreads();
+        win = yt_zero(V());
+        const int w0 = wid - wg;
+        for (int y = WG - 1; y > wg; --y)
+            if (w0 + y < MAXW) win = yt_axpy(sC[1][w0 + y][col], sD[1][w0 + y][col], win);
+        win = yt_axpy(Ce, De, win);
+    }
+    P = 1.0;
+#pragma unroll
+    for (int t = 0; t < R; ++t) {
+        P *= -a * bt[t];
+        x[t] = yt_axpy(x[t], P, u);
+    }
+    CSum sum;
+#pragma unroll
+    for (int t = R - 1; t >= 0; --t) {
+        win = yt_axpy(x[t], -a * bt[t], win);
+        if (on && s + t < ny) __stcg(S + (size_t)t * pk, yt_store<Gm>(win));
+        // the box's dst_w-weighted column sum (a channel has none)
+        if constexpr (!CPLX) sum.add(win);
+    }
+    if constexpr (!CPLX) {
+        // the group's partial (sum, compensation), merged in a fixed order
+        CSum ws;
+        if (on) {
+            const double wk = b.dst_w[k];
+            ws.add_prod(wk, sum.s);
+            ws.add_prod(wk, sum.c);
+        }
+        ws = csum_warp(ws);
+        if (lane == 0) { part[0][wid] = ws.s; part[1][wid] = ws.c; }
+        __syncthreads();
+        if (live && wg == 0 && lane == 0) {
+            CSum t;
+            for (int y = 0; y < WG; ++y) t.merge(part[0][wid + y], part[1][wid + y]);
+            b.part_col[2 * cb] = t.s;
+            b.part_col[2 * cb + 1] = t.c;
         }
     }
 }
@@ -1156,7 +1081,7 @@ __device__ __noinline__ void scalar_phase(const BasinDev &b, double tdt, int par
     double imode[NL];
     double (*S)[OQG_NQ] = out->S;
     if (!b.cyclic) {
-        const int nkb = (b.nk + 3) / 4;       // y-solve CTAs per mode (4 columns each)
+        const int nkb = (b.nk + b.ykb - 1) / b.ykb;       // y-solve column groups per mode
 #pragma unroll
         for (int m = 0; m < NL; ++m) {
             CSum s;
