@@ -221,12 +221,9 @@ static void (*binv_kernel(int M))(const BasinDev *, const Work *, int, int, int,
 }
 template <class T, int E>
 static void (*xfwd_kernel(int M))(const BasinDev *, const Work *, int) {
-    // FP32 storage keeps the any-length instances below the in-place lengths:
-    // at 513^2 the step measured 44.5 us with them against 48.1 us with the
-    // per-length ones (which take 80 registers instead of 128), while at
-    // 2049^2 the per-length forward transform measured 72 against 79 us;
-    // FP64 measured 51.0 against 53.8 us at 513^2 the other way round
-    if (std::is_same<T, float>::value && !fft_inplace_len(M)) M = 0;
+    // FP32 storage keeps the any-length instances: at 513 points the step
+    // measured 44.5 us with them against 48.1 us with the per-length ones
+    if (std::is_same<T, float>::value) M = 0;
     switch (M) {
 #define OQG_XF(MM) case MM: return k_xfwd<T, E, MM>;
         OQG_XLENS(OQG_XF)
@@ -236,7 +233,7 @@ static void (*xfwd_kernel(int M))(const BasinDev *, const Work *, int) {
 }
 template <class T, int E>
 static void (*xinv_rows_kernel(int M))(const BasinDev *, const Work *, int, int, int, double, T *) {
-    if (std::is_same<T, float>::value && !fft_inplace_len(M)) M = 0;      // as xfwd_kernel
+    if (std::is_same<T, float>::value) M = 0;      // as xfwd_kernel
     switch (M) {
 #define OQG_XI(MM) case MM: return k_xinv_rows<T, E, MM>;
         OQG_XLENS(OQG_XI)
@@ -1057,11 +1054,8 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     h->ni = (b.ny + b.k4_rows - 1) / b.k4_rows;
     h->smem_v = vort_smem_bytes(b.vty, (int)h->esz);
     const int LB = fft_buf_len(b.M);
-    // the long lengths transform in place: one buffer plus two staged rows per group
-    const size_t xrow = (size_t)((b.nxin + 3) & ~3);
     auto xsmem = [&](size_t esz) -> size_t {
-        if (!b.cyclic) return (size_t)GX * odd_smem_len(b.M) * 2 * esz;
-        return fft_inplace_len(b.M) ? (size_t)GX * (LB * 2 * esz + 2 * xrow * esz) : (size_t)GX * 2 * LB * 2 * esz;
+        return (size_t)GX * (b.cyclic ? 2 * LB : odd_smem_len(b.M)) * 2 * esz;
     };
     h->smem_x = xsmem(h->esz);
     h->smem_x64 = xsmem(8);
@@ -1903,10 +1897,7 @@ int oqg_ensemble_create(const oqg_params *members, int nmembers, oqg_ensemble **
         for (int k = 0; k < (b.nxp * b.nyp + XASM_ENS_POINTS - 1) / XASM_ENS_POINTS; ++k) wa.push_back(Work{i, k});
         const int nra = (b.ny > b.k4_rows) ? b.k4_rows + 1 : b.ny + 2;
         e->smem_v = std::max(e->smem_v, vort_smem_bytes(b.vty, (int)esz));
-        const size_t xrow = (size_t)((b.nxin + 3) & ~3);
-        e->smem_x = std::max(e->smem_x, !b.cyclic ? (size_t)G * odd_smem_len(b.M) * t2
-                                        : fft_inplace_len(b.M) ? (size_t)G * (LB * t2 + 2 * xrow * esz)
-                                                               : (size_t)G * 2 * LB * t2);
+        e->smem_x = std::max(e->smem_x, (size_t)G * (b.cyclic ? 2 * LB : odd_smem_len(b.M)) * t2);
         e->smem_i = std::max(e->smem_i, xinv_smem(b.M, b.nl, nra, b.nxp, nfft_e, esz, e->m[i]->xinv_split_needed));
     }
     if (e->smem_x > 227 * 1024 || e->smem_i > 227 * 1024 || e->smem_v > 227 * 1024) {

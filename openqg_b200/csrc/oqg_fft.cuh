@@ -337,69 +337,6 @@ __device__ __forceinline__ typename C2<T>::t *fft_ct_from(typename C2<T>::t *src
     }
 }
 
-// ---- in-place stages for the long power-of-two lengths: one padded buffer
-// per transform, so two transforms of 4096 FP64 values fit where the
-// ping-pong pair fits one.  Each thread holds the inputs of all its
-// butterflies in registers (E = M / TT values, E a multiple of every radix of
-// the plan), the group synchronises, then the thread computes and stores.
-template <class T, int R, int Ns, int M, int TT>
-__device__ __forceinline__ void fft_stage_ip(typename C2<T>::t *buf, const typename C2<T>::t *__restrict__ tws,
-                                             int t, bool live, int bar_id, int nbar) {
-    typedef typename C2<T>::t T2;
-    constexpr int nb = M / R, NB = nb / TT;
-    static_assert(nb % TT == 0, "in-place stages need whole butterflies per thread");
-    T2 v[NB][R];
-    if (live) {
-#pragma unroll
-        for (int u = 0; u < NB; ++u)
-#pragma unroll
-            for (int r = 0; r < R; ++r) v[u][r] = buf[fpad_step<nb>(t + u * TT, r)];
-    }
-    bar_sync(bar_id, nbar);
-    if (live) {
-#pragma unroll
-        for (int u = 0; u < NB; ++u) {
-            const int j = t + u * TT;
-            const int q = j / Ns, jm = j - q * Ns;
-            if (Ns > 1 && jm != 0) {
-#pragma unroll
-                for (int r = 1; r < R; ++r) v[u][r] = c_mul(v[u][r], __ldg(tws + (r - 1) * Ns + jm));
-            }
-            Dft<T, R>::run(v[u]);
-            const int d = q * Ns * R + jm;
-#pragma unroll
-            for (int r = 0; r < R; ++r) buf[fpad_step<Ns>(d, r)] = v[u][r];
-        }
-    }
-    bar_sync(bar_id, nbar);
-}
-template <class T, int M, int TT, int Ns>
-__device__ __forceinline__ void fft_ip_from(typename C2<T>::t *buf, const typename C2<T>::t *__restrict__ tw, int t,
-                                            bool live, int bar_id, int nbar) {
-    if constexpr (Ns < M) {
-        constexpr int R = fft_next_radix(M / Ns);
-        fft_stage_ip<T, R, Ns, M, TT>(buf, tw + (Ns - 1), t, live, bar_id, nbar);
-        fft_ip_from<T, M, TT, Ns * R>(buf, tw, t, live, bar_id, nbar);
-    }
-}
-// The lengths that transform in place (16 values per thread).
-__host__ __device__ constexpr bool fft_inplace_len(int M) { return M == 2048 || M == 4096; }
-// In-place forward FFT of length M (fft_inplace_len) by groups of TT = M / 16
-// threads (t >= TT: barriers only); the input is in buf, the barrier after
-// its writes taken.
-// MC > 0: the kernel is built for that one length, and only its plan is
-// compiled.
-template <class T, int MC = 0>
-__device__ __forceinline__ void fft_inplace(typename C2<T>::t *buf, int M, const typename C2<T>::t *__restrict__ tw,
-                                            int t, int bar_id, int nbar) {
-    if constexpr (MC == 2048 || MC == 4096) {
-        fft_ip_from<T, MC, MC / 16, 1>(buf, tw, t, t < MC / 16, bar_id, nbar);
-    } else if constexpr (MC == 0) {
-        if (M == 2048) fft_ip_from<T, 2048, 128, 1>(buf, tw, t, t < 128, bar_id, nbar);
-        else if (M == 4096) fft_ip_from<T, 4096, 256, 1>(buf, tw, t, t < 256, bar_id, nbar);
-    }
-}
-
 // Forward FFT of length M by groups of TT = M / E threads: the compile-time
 // stages for the lengths of the configurations' grids, the general stages
 // otherwise.  Same contract as fft_smem (t >= TT: barriers only).  MC > 0:

@@ -675,13 +675,10 @@ k_xfwd(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int G) {
     const bool two = live && (j + 1 < b.ny);
     const int n = b.nxin;
     const int RO = (n + 3) & ~3;              // offset of the second row (16-byte aligned)
-    // the long lengths transform in place: one buffer per group, the input
-    // rows staged after all the groups' buffers
-    const bool ip = E == 16 && fft_inplace_len(M);
-    T2 *za = zs + (size_t)(g < G ? g : 0) * (ip ? LB : 2 * LB);
+    // the input rows are staged in the second buffer
+    T2 *za = zs + (size_t)(g < G ? g : 0) * 2 * LB;
     T2 *zb = za + LB;
-    T *raw = ip ? reinterpret_cast<T *>(zs + (size_t)G * LB) + (size_t)(g < G ? g : 0) * 2 * RO
-                : reinterpret_cast<T *>(zb);
+    T *raw = reinterpret_cast<T *>(zb);
     const T *x = (const T *)b.rhs + ((size_t)m * b.ny + j) * b.pr;
     pdl_trigger();
     pdl_wait();
@@ -700,9 +697,7 @@ k_xfwd(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int G) {
         }
     }
     __syncthreads();
-    T2 *z = za;
-    if (ip) fft_inplace<T, MC>(za, M, (const T2 *)b.tw, live ? t : M, 0, 0);
-    else z = fft_run<T, E, MC>(za, zb, M, b.rad, b.nrad, (const T2 *)b.tw, live ? t : TT, TT, 0, 0);
+    const T2 *z = fft_run<T, E, MC>(za, zb, M, b.rad, b.nrad, (const T2 *)b.tw, live ? t : TT, TT, 0, 0);
     if (!live) return;
     T2 *S = (T2 *)b.spec;
     T2 *sx = S + ((size_t)m * b.ny + j) * b.pk;
