@@ -191,15 +191,12 @@ void fft_stage_twiddles(int M, const std::vector<int> &rad, std::vector<double> 
 }
 
 void dst_row_sums(int n, std::vector<double> &w) {
+    // the sine sum in closed form: cot(pi k / (2 (n+1))) for odd k, 0 for even
     const long double pi = 3.14159265358979323846264338327950288L;
-    w.resize(n);
-    for (int k = 1; k <= n; ++k) {
-        long double s = 0.0L;
-        for (int i = 1; i <= n; ++i) {
-            long long r = ((long long)i * k) % (2 * (n + 1));
-            s += sinl(pi * (long double)r / (long double)(n + 1));
-        }
-        w[k - 1] = (double)(2.0L * s);
+    w.assign(n, 0.0);
+    for (int k = 1; k <= n; k += 2) {
+        const long double a = pi * (long double)k / (2.0L * (long double)(n + 1));
+        w[k - 1] = (double)(2.0L * cosl(a) / sinl(a));
     }
 }
 
