@@ -68,10 +68,9 @@ struct oqg_handle {
     int yW = 1;                          // spread of a y-solve column as set or tuned
     YGeo yg{};                           // the y-solve's launch
     bool xinv_split_needed = false;      // the modal rows do not fit in shared memory
-    size_t smem_i_full = 0, smem_i64_full = 0;   // k_xinv's shared memory when it transforms
     int na = 0;                          // CTAs of k_xinv_asm
     int xg = 1;                          // transforms per CTA of k_xfwd and k_xinv_rows
-    size_t smem_v = 0, smem_x = 0, smem_x64 = 0, smem_i = 0, smem_i64 = 0;
+    size_t smem_v = 0, smem_x = 0, smem_x64 = 0, smem_i = 0;
     double *stage[2] = {nullptr, nullptr};
     double *hrow = nullptr;     // contiguous host-order copy buffer [nl][nyp][nxp]
     double *dg = nullptr;       // qg_diagno scratch, made on its first call
@@ -105,25 +104,17 @@ static X *dalloc(oqg_handle *h, size_t count) {
 
 // ----------------------------------------------------------- launch helpers
 
-// Launch with programmatic stream serialisation: the kernel may be scheduled
-// while its predecessor drains and waits in griddepcontrol.wait for its data.
-// Inverse-transform CTA: transform threads for all NL row pairs of a CTA in
-// one round where they fit (XINV_E values per thread), plus the scalar warp.
-static int xinv_fft_threads(int M, int nl) {
-    const int tt = (M + XINV_E - 1) / XINV_E;
-    int nfft = std::min(XINV_FFT_MAX, rup(nl * tt, 32));
-    return std::max(nfft, rup(tt, 32));
-}
-// Dynamic shared bytes of k_xinv for nfft transform threads (element size
-// esz); split: the modal rows live in global memory instead.
-static size_t xinv_smem(int M, int nl, int nra, int nxp, int nfft, size_t esz, bool split = false) {
-    const int tt = (M + XINV_E - 1) / XINV_E, G = nfft / tt;
-    const size_t set = (size_t)G * fft_buf_len(M) * 2 * esz;
-    if (split) return 2 * set;
-    const size_t inh = (size_t)nl * nra * nxp * esz;
-    return G >= nl ? std::max(2 * set, set + inh) : 2 * set + inh;
+// Whether a grid may take the one-kernel inverse (oqg_set_xinv_sep): two
+// buffers of nl transforms of M FP64 values, threads for them, and the modal
+// rows of a row pair and a wall row in shared memory.
+static bool xinv_fits(int M, int nl, int ny, int nxp) {
+    const int tt = (M + XINV_E - 1) / XINV_E, nfft = std::max(std::min(512, rup(nl * tt, 32)), rup(tt, 32)), G = nfft / tt;
+    const size_t set = (size_t)G * fft_buf_len(M) * 16, inh = (size_t)nl * (ny > 2 ? 3 : ny + 2) * nxp * 8;
+    return (G >= nl ? std::max(2 * set, set + inh) : 2 * set + inh) <= 227 * 1024;
 }
 
+// Launch with programmatic stream serialisation: the kernel may be scheduled
+// while its predecessor drains and waits in griddepcontrol.wait for its data.
 template <typename... KArgs, typename... Args>
 static void launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t st,
                        Args... args) {
@@ -276,43 +267,55 @@ static XGeo xgeo(oqg_handle *h, bool fp64, bool pdl) {
                 fp64 ? h->d_bas64 : h->d_bas, h->d_wx, pdl};
 }
 
-// The vorticity kernel instance of a tile height (vort_tile_ok).
+// The vorticity kernel instance of a tile height and its threads.  wide: no
+// more CTAs than SMs at the least height (us per step: 129^2 25.1 -> 22.5,
+// 193 x 97 channel 29.9 -> 26.7).
 typedef void (*VortFn)(const BasinDev *, const Work *, int, double);
 template <class T, int NL>
-static VortFn vort_kernel(int vt) {
+static VortFn vort_kernel(int vt, bool wide) {
     switch (vt) {
-        case 8: return k_vort<T, NL, 8>;
-        case 12: return k_vort<T, NL, 12>;
-        default: return k_vort<T, NL, 16>;
+        case 8: return wide ? k_vort<T, NL, 8, VWIDE> : k_vort<T, NL, 8, VSTRIPS>;
+        case 12: return k_vort<T, NL, 12, VSTRIPS>;
+        default: return k_vort<T, NL, 16, VSTRIPS>;
     }
 }
+static bool vort_wide(int vt, int ctas) { return vt == 8 && ctas <= 148; }
+static int vort_threads(int vt, bool wide) { return 64 * (vt == 8 && wide ? VWIDE : VSTRIPS); }
 
-// The inverse transforms as k_xinv_rows and the one-pass k_xinv_asm (box),
-// or inside k_xinv; k_xinv keeps its modal rows in global memory when they
-// run separately or do not fit in shared memory.
+// The one-kernel inverse's instance: a channel's length (FP64), or any.
+template <class T>
+static void (*xinv_kernel(bool cyclic, int M))(const BasinDev *, const Work *, int, double) {
+    if (!cyclic) return k_xinv<T, false, 0>;
+    if constexpr (sizeof(T) == 8) {
+        switch (M) {
+#define OQG_XK(MM) case MM: return k_xinv<T, true, MM>;
+            OQG_XLENS(OQG_XK)
+#undef OQG_XK
+        }
+    }
+    return k_xinv<T, true, 0>;
+}
+
+// The inverse transforms and the one-pass k_xinv_asm as two launches (on), or
+// k_xinv for both.
 static void apply_xinv_sep(oqg_handle *h, bool on) {
-    BasinDev &b = h->hb;
-    b.xinv_sep = on ? 1 : 0;
-    b.xinv_split = (on || h->xinv_split_needed) ? 1 : 0;
-    h->smem_i = on ? 0 : h->smem_i_full;
-    h->smem_i64 = on ? 0 : h->smem_i64_full;
-    h->hb64.xinv_sep = b.xinv_sep;
-    h->hb64.xinv_split = b.xinv_split;
+    h->hb.xinv_sep = on ? 1 : 0;
+    h->hb64.xinv_sep = h->hb.xinv_sep;
 }
 
 template <class T, int NL, int E>
 static void launch_step_t(oqg_handle *h, int par, double tdt) {
     const BasinDev &b = h->hb;
     const XGeo x = xgeo(h, false, true);
-    launch_pdl(vort_kernel<T, NL>(h->hb.vty), h->nv, VTHREADS, h->smem_v, h->st, h->d_bas, h->d_wv, par, tdt);
+    const bool vw = vort_wide(b.vty, h->nv);
+    launch_pdl(vort_kernel<T, NL>(b.vty, vw), h->nv, vort_threads(b.vty, vw), h->smem_v, h->st, h->d_bas, h->d_wv, par, tdt);
     launch_fwd<T, E>(x);
     launch_ysolve<T>(b.cyclic, h->yg, h->st, h->d_bas, h->d_wy, true);
     if (b.xinv_sep) {
         launch_inv<T, E>(x, 1, par, tdt, nullptr);
         launch_pdl(k_xinv_asm<T, NL>, h->na, 256, 0, h->st, h->d_bas, (const Work *)h->d_wa, par);
     } else {
-        launch_pdl(k_xinv<T, NL>, h->ni, h->xi_threads, h->smem_i, h->st, h->d_bas, h->d_wi, par, tdt,
-                   (double *)nullptr);
+        launch_pdl(xinv_kernel<T>(b.cyclic, b.M), h->ni, h->xi_threads, h->smem_i, h->st, h->d_bas, h->d_wi, par, tdt);
     }
 }
 
@@ -325,11 +328,7 @@ static void launch_solve_t(oqg_handle *h, double *out, bool pdl) {
     const XGeo x = xgeo(h, true, pdl);
     launch_fwd<double, E>(x);
     launch_ysolve<double>(h->hb.cyclic, h->yg, h->st, h->d_bas64, h->d_wy, pdl);
-    if (h->hb.xinv_sep) launch_inv<double, E>(x, 0, 0, 0.0, out);
-    else if (pdl)
-        launch_pdl(k_xinv<double, NL>, h->ni, h->xi_threads, h->smem_i64, h->st, h->d_bas64, h->d_wi, 0, 0.0, out);
-    else
-        k_xinv<double, NL><<<h->ni, h->xi_threads, h->smem_i64, h->st>>>(h->d_bas64, h->d_wi, 0, 0.0, out);
+    launch_inv<double, E>(x, 0, 0, 0.0, out);
 }
 
 // The dynamic shared-memory limit of a kernel is a property of the function
@@ -365,16 +364,16 @@ static void raise_x_smem(bool cyclic, int M, size_t x) {
 }
 template <class T, int NL, int E>
 static void raise_step_smem(bool cyclic, int M, size_t v, size_t x, size_t i) {
-    for (int vt : {8, 12, 16}) raise_smem((const void *)vort_kernel<T, NL>(vt), v);
+    for (int vt : {8, 12, 16}) raise_smem((const void *)vort_kernel<T, NL>(vt, false), v);
+    raise_smem((const void *)vort_kernel<T, NL>(8, true), v);
     raise_x_smem<T, E>(cyclic, M, x);
-    raise_smem((const void *)k_xinv<T, NL>, i);
+    if (i) raise_smem((const void *)xinv_kernel<T>(cyclic, M), i);
 }
 
 template <class T, int NL, int E>
 static void set_attrs_t(oqg_handle *h) {
     raise_step_smem<T, NL, E>(h->hb.cyclic, h->hb.M, h->smem_v, h->smem_x, h->smem_i);
     raise_x_smem<double, E>(h->hb.cyclic, h->hb.M, h->smem_x64);
-    raise_smem((const void *)k_xinv<double, NL>, h->smem_i64);
 }
 
 // dispatch over (T, NL); 16 values per transform thread
@@ -522,12 +521,11 @@ static EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-// Tensor maps of the closed-box tiles of k_vort (order in oqg_kernels.cuh).
+// Tensor maps of the tiles of k_vort (order in oqg_kernels.cuh).
 // Returns false when the driver cannot encode them; the kernel then loads
 // the tiles with cp.async.
 static bool make_tmaps(oqg_handle *h) {
     BasinDev &b = h->hb;
-    if (b.cyclic) return false;
     const char *env = std::getenv("OQG_NO_TMA");
     if (env && env[0] == '1') return false;
     EncodeTiledFn enc = encode_tiled();
@@ -672,13 +670,17 @@ template <class T, int NL, int E>
 static void launch_phase_t(oqg_handle *h, int phase, int par, double tdt) {
     const BasinDev &b = h->hb;
     switch (phase) {
-        case 0: vort_kernel<T, NL>(b.vty)<<<h->nv, VTHREADS, h->smem_v, h->st>>>(h->d_bas, h->d_wv, par, tdt); break;
+        case 0: {
+            const bool vw = vort_wide(b.vty, h->nv);
+            vort_kernel<T, NL>(b.vty, vw)<<<h->nv, vort_threads(b.vty, vw), h->smem_v, h->st>>>(h->d_bas, h->d_wv, par, tdt);
+            break;
+        }
         case 1: launch_fwd<T, E>(xgeo(h, false, false)); break;
         case 2: launch_ysolve<T>(b.cyclic, h->yg, h->st, h->d_bas, h->d_wy, false); break;
         case 3:
             if (b.xinv_sep) launch_inv<T, E>(xgeo(h, false, false), 1, par, tdt, nullptr);
             else
-                k_xinv<T, NL><<<h->ni, h->xi_threads, h->smem_i, h->st>>>(h->d_bas, h->d_wi, par, tdt, nullptr);
+                xinv_kernel<T>(b.cyclic, b.M)<<<h->ni, h->xi_threads, h->smem_i, h->st>>>(h->d_bas, h->d_wi, par, tdt);
             break;
         default: k_xinv_asm<T, NL><<<h->na, 256, 0, h->st>>>(h->d_bas, h->d_wa, par); break;
     }
@@ -701,14 +703,13 @@ struct oqg_ensemble {
     bool mixed = false;
     int nl = 3, E = 8, cyclic = 0;
     BasinDev *d_bas = nullptr;
-    Work *d_wv = nullptr, *d_wx = nullptr, *d_wy = nullptr, *d_wi = nullptr;
-    Work *d_wa = nullptr;              // k_xinv_asm work items (boxes)
+    Work *d_wv = nullptr, *d_wx = nullptr, *d_wy = nullptr;
+    Work *d_wa = nullptr;              // k_xinv_asm work items
     int na = 0;                        // k_xinv_asm work items
-    bool sep = false;                  // boxes: k_xinv_rows + k_xinv_asm
     int Mu = 0;                        // the members' common transform length, else 0
-    int nv = 0, nx = 0, ni = 0;
-    size_t smem_v = 0, smem_x = 0, smem_i = 0;
-    int xi_threads = 64, xthreads = 128;
+    int nv = 0, nx = 0;
+    size_t smem_v = 0, smem_x = 0;
+    int xthreads = 128;
     int yW = 1;                        // spread of a y-solve column, one for every member
     YGeo yg{};                         // the y-solve's launch
     int par = 0;
@@ -735,23 +736,18 @@ struct oqg_ensemble {
 // descriptor (tdt = 0).
 template <class T, int NL, int E>
 static void launch_ens_step_t(oqg_ensemble *e, int par) {
-    launch_pdl(vort_kernel<T, NL>(e->hb[0].vty), e->nv, VTHREADS, e->smem_v, e->st, e->d_bas, e->d_wv, par, 0.0);
+    launch_pdl(vort_kernel<T, NL>(e->hb[0].vty, false), e->nv, vort_threads(e->hb[0].vty, false), e->smem_v, e->st, e->d_bas, e->d_wv, par, 0.0);
     // members of one transform length take that length's instance; each
     // member's transforms per CTA follow from the CTA's threads (G = 0)
     const XGeo x{e->cyclic != 0, e->Mu, e->nx, e->xthreads, 0, e->smem_x, e->st, e->d_bas, e->d_wx, true};
     launch_fwd<T, E>(x);
     launch_ysolve<T>(e->cyclic, e->yg, e->st, e->d_bas, e->d_wy, true);
-    if (e->sep) {
-        launch_inv<T, E>(x, (int)e->m.size(), par, 0.0, nullptr);    // one scalar CTA per member
-        launch_pdl(k_xinv_asm<T, NL>, e->na, 256, 0, e->st, e->d_bas, (const Work *)e->d_wa, par);
-    } else {
-        launch_pdl(k_xinv<T, NL>, e->ni, e->xi_threads, e->smem_i, e->st, e->d_bas, e->d_wi, par, 0.0,
-                   (double *)nullptr);
-    }
+    launch_inv<T, E>(x, (int)e->m.size(), par, 0.0, nullptr);    // one scalar CTA per member
+    launch_pdl(k_xinv_asm<T, NL>, e->na, 256, 0, e->st, e->d_bas, (const Work *)e->d_wa, par);
 }
 template <class T, int NL, int E>
 static void raise_ens_smem_t(oqg_ensemble *e) {
-    raise_step_smem<T, NL, E>(e->cyclic, e->Mu, e->smem_v, e->smem_x, e->smem_i);
+    raise_step_smem<T, NL, E>(e->cyclic, e->Mu, e->smem_v, e->smem_x, 0);
 }
 static void launch_ens_step(oqg_ensemble *e, int par) { OQG_DISPATCH_E(launch_ens_step_t, e, e, par); }
 
@@ -820,6 +816,8 @@ static void record_vty(const oqg_params &P, bool mixed, int vty) {
         }
     g_tuned.push_back(TunedVty{P.nxp, P.nyp, P.nl, P.cyclic != 0, (int)mixed, vty});
 }
+
+static int vort_ctas(const BasinDev &b) { return vort_strips(b.nl, b.cyclic) + b.tiles_x * b.tiles_y; }
 
 // The pivots of YS_PIVB adjacent wavenumbers interleaved row by row, up to the
 // longest of their lengths (k_ysolve reads them so); the columns past the last
@@ -901,7 +899,7 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
         int best = 16;
         long best_cost = -1;
         for (int vt = 16; vt >= 8 && !batched; vt -= 4) {          // the compiled heights
-            const int ty = vort_tile_rows(P.nyp, P.cyclic, vt);
+            const int ty = vort_tile_rows(P.nyp, vt);
             const long waves = ((long)b.tiles_x * ty + slots - 1) / slots;
             const long cost = waves * (vt + 6);
             if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = vt; }
@@ -909,7 +907,7 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
         const int tuned = tuned_vty(P, h->mixed);
         if (tuned > 0 && !batched) best = tuned;
         b.vty = best;
-        b.tiles_y = vort_tile_rows(P.nyp, P.cyclic, b.vty);
+        b.tiles_y = vort_tile_rows(P.nyp, b.vty);
     }
     b.kt = P.k_topo - 1;
     b.wait_limit = OQG_WAIT_LIMIT;
@@ -1016,8 +1014,7 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
         b.hbc1 = dalloc<double>(h, (size_t)b.nl * b.nyp);
         b.hbc2 = dalloc<double>(h, (size_t)b.nl * b.nyp);
     }
-    // sized for the shortest tiles (8 rows), so oqg_autotune can retile in place
-    b.part_tile = dalloc<double>(h, (size_t)b.tiles_x * ((P.nyp + 7) / 8) * b.nl * OQG_NQ);
+    b.part_tile = dalloc<double>(h, (size_t)2 * b.nl * OQG_NSTRIP);
     b.part_col = dalloc<double>(h, 2 * (size_t)b.nl * b.nk);
     b.st = dalloc<DevState>(h, 2);
     b.frc = dalloc<DevForcing>(h, 1);
@@ -1036,7 +1033,7 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     h->E = 16;
     const int TT = b.cyclic ? (b.M + h->E - 1) / h->E : odd_tt(b.M);
     const int npm = (b.ny + 1) / 2;
-    h->nv = b.tiles_x * b.tiles_y;
+    h->nv = vort_ctas(b);
     // forward transform: one row pair per group, CTAs of >= 128 threads; a
     // grid whose row pairs would not fill the SMs that way spreads them over
     // more, smaller CTAs (each transform is a latency chain of FFT stages)
@@ -1050,8 +1047,7 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
         return bail(OQG_EUNSUPPORTED, "grid too large for this build's shared-memory tiling");
     h->yg = ysolve_geo(b.ny, b.nk, b.nl, b.cyclic, h->yW);
     b.ykb = h->yg.KB;
-    b.k4_rows = 2;
-    h->ni = (b.ny + b.k4_rows - 1) / b.k4_rows;
+    h->ni = npm;
     h->smem_v = vort_smem_bytes(b.vty, (int)h->esz);
     const int LB = fft_buf_len(b.M);
     auto xsmem = [&](size_t esz) -> size_t {
@@ -1059,40 +1055,24 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     };
     h->smem_x = xsmem(h->esz);
     h->smem_x64 = xsmem(8);
-    // rows of an assembly CTA: k4_rows interior rows plus at most one wall row
-    const int nra = (b.ny > b.k4_rows) ? b.k4_rows + 1 : b.ny + 2;
-    int nfft_i = xinv_fft_threads(b.M, b.nl);
-    bool split = false;
-    b.inh_g = nullptr;
-    if (xinv_smem(b.M, b.nl, nra, b.nxp, nfft_i, 8) > 227 * 1024) {
-        // wide grid: the modal rows go to a global buffer, and a round holds
-        // as many FP64 transforms as shared memory does
-        split = true;
-        const int tt = (b.M + XINV_E - 1) / XINV_E;
-        const size_t per = 2 * (size_t)fft_buf_len(b.M) * 16;
-        const int G = std::max(1, std::min(b.nl, (int)((227 * 1024) / per)));
-        nfft_i = std::min(XINV_FFT_MAX, rup(G * tt, 32));
-        if ((nfft_i / tt) * per > 227 * 1024) nfft_i = rup(tt, 32);
-    }
     // the buffers of the separate inverse transforms (the modal rows in
     // global memory, the step's scalars), kept at any width
     b.inh_g = dalloc<char>(h, (size_t)b.nl * b.nyp * b.px * 8);
     b.scal_g = dalloc<char>(h, sizeof(XinvScal));
     if (!b.inh_g || !b.scal_g) return bail(OQG_ECUDA, "out of device memory");
-    h->xi_threads = nfft_i + 32;
-    h->smem_i_full = xinv_smem(b.M, b.nl, nra, b.nxp, nfft_i, h->esz, split);
-    h->smem_i64_full = xinv_smem(b.M, b.nl, nra, b.nxp, nfft_i, 8, split);
-    h->xinv_split_needed = split;
+    h->xinv_split_needed = !xinv_fits(b.M, b.nl, b.ny, b.nxp);
+    h->xi_threads = xinv_threads(b.M, b.cyclic, b.nl) + 32;
+    h->smem_i = h->xinv_split_needed ? 0 : xinv_bytes(b.M, b.cyclic, b.nl, b.nxp, (int)h->esz);
     // one point per thread, at most 8 work items of 256 threads per SM (the
     // items stride over larger grids)
     b.asm_items = std::min((b.nxp * b.nyp + 255) / 256, 148 * 8);
     h->na = b.asm_items;
     // boxes: the inverse transforms run as a launch of their own, shaped like
-    // the forward one, then a one-pass assembly (oqg_set_xinv_sep; faster at
-    // 513^2 and the only form once the modal rows leave shared memory);
-    // channels start with the one-kernel form (oqg_autotune_xinv measures both)
-    apply_xinv_sep(h, !b.cyclic || split);
-    if (h->smem_i64_full > 227 * 1024 || h->smem_x64 > 227 * 1024)
+    // the forward one, then a one-pass assembly (oqg_set_xinv_sep; the only
+    // form once the modal rows leave shared memory); channels start with the
+    // one-kernel form
+    apply_xinv_sep(h, !b.cyclic || h->xinv_split_needed);
+    if (h->smem_x64 > 227 * 1024)
         return bail(OQG_EUNSUPPORTED, "grid too large for this build's shared-memory tiling");
     std::vector<Work> wv(h->nv), wx(h->nx), wy(ysolve_groups(b)), wi(h->ni), wa(h->na);
     for (int i = 0; i < h->na; ++i) wa[i] = Work{0, i};
@@ -1100,7 +1080,8 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     for (int i = 0; i < h->nx; ++i) wx[i] = Work{0, i};
     for (size_t i = 0; i < wy.size(); ++i) wy[i] = Work{0, (int)i};
     for (int i = 0; i < h->ni; ++i) wi[i] = Work{0, i};
-    h->d_wv = dalloc<Work>(h, (size_t)b.tiles_x * ((P.nyp + 7) / 8));
+    // room for the shortest tiles (8 rows), so oqg_autotune can retile in place
+    h->d_wv = dalloc<Work>(h, (size_t)vort_strips(b.nl, b.cyclic) + b.tiles_x * vort_tile_rows(P.nyp, 8));
     h->d_wx = dalloc<Work>(h, wx.size());
     h->d_wy = dalloc<Work>(h, wy.size());
     h->d_wi = dalloc<Work>(h, wi.size());
@@ -1717,7 +1698,7 @@ __global__ void k_chain_empty() {
 int oqg_launch_floor(oqg_handle *h, int nsteps, double *us_per_step) {
     if (!h || !us_per_step || nsteps < 1) return fail(OQG_EINVAL, "bad argument");
     struct Shape { int grid, block; size_t smem; };
-    std::vector<Shape> sh = {{h->nv, VTHREADS, h->smem_v}, {h->nx, h->xthreads, h->smem_x},
+    std::vector<Shape> sh = {{h->nv, vort_threads(h->hb.vty, vort_wide(h->hb.vty, h->nv)), h->smem_v}, {h->nx, h->xthreads, h->smem_x},
                              {h->yg.grid, h->yg.block, 0}};
     if (h->hb.xinv_sep) {
         sh.push_back({h->nx + 1, rup(h->xthreads, 32), h->smem_x});
@@ -1859,16 +1840,10 @@ int oqg_ensemble_create(const oqg_params *members, int nmembers, oqg_ensemble **
     std::stable_sort(order.begin(), order.end(), [&](int a, int c) {
         return (long)e->m[a]->hb.nxp * e->m[a]->hb.nyp > (long)e->m[c]->hb.nxp * e->m[c]->hb.nyp;
     });
-    std::vector<Work> wv, wx, wy, wi, wa;
-    // boxes invert as a transform launch and a one-pass assembly, as single
-    // handles do
-    e->sep = !e->cyclic;
+    std::vector<Work> wv, wx, wy, wa;
     e->Mu = e->m[0]->hb.M;
     for (oqg_handle *h : e->m)
         if (h->hb.M != e->Mu) e->Mu = 0;
-    int nfft_e = 32;
-    for (oqg_handle *h : e->m) nfft_e = std::max(nfft_e, xinv_fft_threads(h->hb.M, h->hb.nl));
-    e->xi_threads = nfft_e + 32;
     {
         long long cols = 0;
         int ny_max = 0;
@@ -1886,25 +1861,21 @@ int oqg_ensemble_create(const oqg_params *members, int nmembers, oqg_ensemble **
         const int G = std::max(1, e->xthreads / TT);
         const int LB = fft_buf_len(b.M);
         const int npm = (b.ny + 1) / 2;
-        const int nvb = b.tiles_x * b.tiles_y;
+        const int nvb = vort_ctas(b);
         const int nxb = (b.nl * npm + G - 1) / G;
         const int nyb = (ysolve_groups(b) + ens_ygroups(e, b) - 1) / ens_ygroups(e, b);
-        const int nib = (b.ny + b.k4_rows - 1) / b.k4_rows;
         for (int k = 0; k < nvb; ++k) wv.push_back(Work{i, k});
         for (int k = 0; k < nxb; ++k) wx.push_back(Work{i, k});
         for (int k = 0; k < nyb; ++k) wy.push_back(Work{i, k});
-        for (int k = 0; k < nib; ++k) wi.push_back(Work{i, k});
         for (int k = 0; k < (b.nxp * b.nyp + XASM_ENS_POINTS - 1) / XASM_ENS_POINTS; ++k) wa.push_back(Work{i, k});
-        const int nra = (b.ny > b.k4_rows) ? b.k4_rows + 1 : b.ny + 2;
         e->smem_v = std::max(e->smem_v, vort_smem_bytes(b.vty, (int)esz));
         e->smem_x = std::max(e->smem_x, (size_t)G * (b.cyclic ? 2 * LB : odd_smem_len(b.M)) * t2);
-        e->smem_i = std::max(e->smem_i, xinv_smem(b.M, b.nl, nra, b.nxp, nfft_e, esz, e->m[i]->xinv_split_needed));
     }
-    if (e->smem_x > 227 * 1024 || e->smem_i > 227 * 1024 || e->smem_v > 227 * 1024) {
+    if (e->smem_x > 227 * 1024 || e->smem_v > 227 * 1024) {
         ens_free(e);
         return fail(OQG_EUNSUPPORTED, "ensemble member too large for the shared-memory tiling");
     }
-    e->nv = (int)wv.size(); e->nx = (int)wx.size(); e->yg.grid = (int)wy.size(); e->ni = (int)wi.size();
+    e->nv = (int)wv.size(); e->nx = (int)wx.size(); e->yg.grid = (int)wy.size();
     e->na = (int)wa.size();
     e->wv_cap = wv.size();
     auto up = [&](const void *src, size_t bytes) -> void * {
@@ -1917,17 +1888,14 @@ int oqg_ensemble_create(const oqg_params *members, int nmembers, oqg_ensemble **
     e->hb.resize(nmembers);
     for (int i = 0; i < nmembers; ++i) {
         e->hb[i] = e->m[i]->hb;
-        e->hb[i].xinv_sep = e->sep ? 1 : 0;
-        e->hb[i].xinv_split = (e->sep || e->m[i]->xinv_split_needed) ? 1 : 0;
         e->hb[i].asm_items = (e->hb[i].nxp * e->hb[i].nyp + XASM_ENS_POINTS - 1) / XASM_ENS_POINTS;
     }
     e->d_bas = (BasinDev *)up(e->hb.data(), e->hb.size() * sizeof(BasinDev));
     e->d_wv = (Work *)up(wv.data(), wv.size() * sizeof(Work));
     e->d_wx = (Work *)up(wx.data(), wx.size() * sizeof(Work));
     e->d_wy = (Work *)up(wy.data(), wy.size() * sizeof(Work));
-    e->d_wi = (Work *)up(wi.data(), wi.size() * sizeof(Work));
     e->d_wa = (Work *)up(wa.data(), wa.size() * sizeof(Work));
-    if (!e->d_bas || !e->d_wv || !e->d_wx || !e->d_wy || !e->d_wi || !e->d_wa) {
+    if (!e->d_bas || !e->d_wv || !e->d_wx || !e->d_wy || !e->d_wa) {
         ens_free(e);
         return fail(OQG_ECUDA, "out of device memory");
     }
@@ -1955,8 +1923,6 @@ static int ens_member(oqg_ensemble *e, int member, oqg_handle **h) {
 static int ens_refresh(oqg_ensemble *e, int member) {
     const double tdt = e->hb[member].tdt_m;
     e->hb[member] = e->m[member]->hb;
-    e->hb[member].xinv_sep = e->sep ? 1 : 0;
-    e->hb[member].xinv_split = (e->sep || e->m[member]->xinv_split_needed) ? 1 : 0;
     e->hb[member].asm_items = (e->hb[member].nxp * e->hb[member].nyp + XASM_ENS_POINTS - 1) / XASM_ENS_POINTS;
     e->hb[member].tdt_m = tdt;
     CK(cudaMemcpyAsync(e->d_bas + member, &e->hb[member], sizeof(BasinDev), cudaMemcpyHostToDevice, e->st));
@@ -2435,8 +2401,8 @@ int oqg_get_forcing(oqg_handle *h, double *wekp, double *ent) {
 static int set_vty(oqg_handle *h, int vt) {
     BasinDev &b = h->hb;
     b.vty = vt;
-    b.tiles_y = vort_tile_rows(b.nyp, b.cyclic, vt);
-    h->nv = b.tiles_x * b.tiles_y;
+    b.tiles_y = vort_tile_rows(b.nyp, vt);
+    h->nv = vort_ctas(b);
     std::vector<Work> wv(h->nv);
     for (int i = 0; i < h->nv; ++i) wv[i] = Work{0, i};
     CK(cudaMemcpy(h->d_wv, wv.data(), wv.size() * sizeof(Work), cudaMemcpyHostToDevice));
@@ -2623,7 +2589,7 @@ static int ens_set_vty(oqg_ensemble *e, int vt) {
         oqg_handle *h = e->m[i];
         BasinDev &b = h->hb;
         b.vty = vt;
-        b.tiles_y = vort_tile_rows(b.nyp, b.cyclic, vt);
+        b.tiles_y = vort_tile_rows(b.nyp, vt);
         if (b.tmaps && !make_tmaps(h)) return fail(OQG_ECUDA, "tensor maps could not be encoded");
         h->hb64.vty = b.vty;
         h->hb64.tiles_y = b.tiles_y;
@@ -2636,7 +2602,7 @@ static int ens_set_vty(oqg_ensemble *e, int vt) {
         e->hb[i].tmaps = b.tmaps;
     }
     for (int i : order)
-        for (int k = 0; k < e->hb[i].tiles_x * e->hb[i].tiles_y; ++k) wv.push_back(Work{i, k});
+        for (int k = 0; k < vort_ctas(e->hb[i]); ++k) wv.push_back(Work{i, k});
     if (wv.size() > e->wv_cap) {
         void *d = nullptr;
         if (cudaMalloc(&d, wv.size() * sizeof(Work)) != cudaSuccess) return fail(OQG_ECUDA, "out of device memory");

@@ -37,8 +37,8 @@ struct DevForcing {
 // Device error bits
 #define OQG_DERR_TIMEOUT 2   // a bounded wait for a tile load ran out
 
-// Number of per-tile channel strip quantities per layer (vorticity kernel)
-#define OQG_NQ 10
+// Channel strip quantities per wall and layer (vorticity kernel)
+#define OQG_NSTRIP 5
 
 struct BasinDev {
     // geometry
@@ -80,7 +80,7 @@ struct BasinDev {
     const void *ent;            // [nl-1][nyp][px] T or null
     const double *ddyn;         // [nyp][px] or null
     const double *yprel;        // [nyp] y - yl/2 (box.F90:142-145)
-    const void *tmaps;          // box: OQG_NTMAP tensor maps (128 bytes each) or null
+    const void *tmaps;          // OQG_NTMAP tensor maps (128 bytes each) or null
     void *rhs;                  // [nl][ny][pr] T
     void *spec;                 // [nl][ny][pk] T or T2
     const void *tw;             // [M] T2 per-stage FFT twiddles (fft_stage_twiddles)
@@ -94,7 +94,7 @@ struct BasinDev {
     const void *hsb;            // box: [nl-1][nyp][px] T hom_sol_bc
     const double *hbt;          // channel: [nyp] barotropic homogeneous solution
     const double *hbc1, *hbc2;  // channel: [nl][nyp]
-    double *part_tile;          // [tiles][nl][OQG_NQ]
+    double *part_tile;          // channel: [2 walls][nl][OQG_NSTRIP] strip integrals
     int ykb;                    // columns of a y-solve group
     double *part_col;           // [y-solve groups][2]: dst_w-weighted column sums and
                                 // their compensations
@@ -106,10 +106,8 @@ struct BasinDev {
                                 // slots): wide grids, and every box (k_xinv_rows)
     int *err;                   // device error bits
     // launch bookkeeping
-    int k4_rows;                // interior rows per CTA of the assembly launch
     int xinv_sep;               // the inverse transforms run as k_xinv_rows and the
                                 // assembly as k_xinv_asm (boxes; always when wide)
-    int xinv_split;             // k_xinv keeps its modal rows in inh_g
     int asm_items;              // k_xinv_asm work items of this basin (256-point runs
                                 // interleaved over them)
     void *scal_g;               // with xinv_sep: the step's scalar phase results,

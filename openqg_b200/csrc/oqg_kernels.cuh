@@ -142,9 +142,9 @@ __device__ __forceinline__ double csum_block(CSum v, double *red) { return csum_
 // ------------------------------------------------------------------ k_vort
 #define VTX 60          // output columns of a vorticity tile
 #define VTYMAX 17       // output rows of a vorticity tile (at most)
-#define VTHREADS 256    // 64 column lanes x 4 row strips
-#define XINV_E 16           // complex values per transform thread in k_xinv
-#define XINV_FFT_MAX 512    // at most this many transform threads per k_xinv CTA
+#define VSTRIPS 4        // row strips of a tile (64 column lanes each)
+#define VWIDE 8          // the same where every SM has at most one tile
+#define XINV_E 16           // complex values per transform thread of a channel
 
 // Storage of q: FP64 handles keep q itself; FP32 handles keep the anomaly
 // q - beta yprel (the planetary vorticity is most of q, and in FP32 its
@@ -200,12 +200,13 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// Queues the copy of rows [jlo, jlo+nr) x cols [ilo, ilo+nc) of layer k of f
-// into s (leading dimension nc); outside the basin -> 0.  Channel columns of
-// a halo tile wrap with period nxp-1; an `own` tile (the CTA's output columns
-// only) reads columns < nxp as stored, including the duplicate column nxp-1,
-// and zeros beyond, so it never reads a column that another CTA writes.
-// Thread layout: 64 columns x 4 rows.
+// Queues the copy of rows [jlo, jlo+nr) x cols [ilo, ilo+nc) of layer k of a
+// channel's f into s (leading dimension nc); outside the basin -> 0.  Columns
+// of a halo tile wrap with period nxp-1 as far as the last output column's
+// halo; an `own` tile (the CTA's output columns only) reads columns < nxp as
+// stored, including the duplicate column nxp-1, and zeros beyond, so it never
+// reads a column that another CTA writes.
+// Thread layout: 64 columns x blockDim / 64 rows.
 template <class T, class G>
 __device__ __forceinline__ void load_tile_async(T *s, const T *__restrict__ f, const G &g, int px,
                                                 int k, int jlo, int nr, int ilo, int nc,
@@ -213,34 +214,29 @@ __device__ __forceinline__ void load_tile_async(T *s, const T *__restrict__ f, c
     const int N = g.nxp - 1;
     const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
     const T *fk = f + (size_t)k * g.nyp * px;
-    for (int r = ty; r < nr; r += 4) {
-        const int j = jlo + r;
-        const bool jv = (j >= 0 && j < g.nyp);
-        const T *row = fk + (size_t)(jv ? j : 0) * px;
-        for (int c = tx; c < nc; c += 64) {
-            int i = ilo + c;
-            bool v = jv;
-            if (g.cyclic && !own) {
-                while (i < 0) i += N;
-                while (i >= N) i -= N;
-            } else {
-                v = v && i >= 0 && i < g.nxp;
-            }
-            cp_async_el(s + r * nc + c, row + (v ? i : 0), v);
+    for (int c = tx; c < nc; c += 64) {
+        const int gi = ilo + c;
+        const bool cv = own ? gi < g.nxp : gi < g.nxp + 3;
+        const int i = !cv ? 0 : own ? gi : gi < 0 ? gi + N : gi >= N ? gi - N : gi;
+        for (int r = ty; r < nr; r += blockDim.x >> 6) {
+            const int j = jlo + r;
+            const bool v = cv && j >= 0 && j < g.nyp;
+            cp_async_el(s + r * nc + c, fk + (size_t)(v ? j : 0) * px + i, v);
         }
     }
 }
 
 // Tiles are VTX columns by b.vty rows (b.vty <= VTYMAX, chosen per basin so
-// that the tiles fill whole waves); a box's tile rows start at row 1.  Shared tiles per layer (origin, pitch):
+// that the tiles fill whole waves); tile rows start at row 1 (the walls are not
+// stepped).  Shared tiles per layer (origin, pitch):
 //   pm     rows j0-3 .. j0+vty+2, cols from i0-4   (LPQ = VTX+8 = 68)
 //   p, q   rows j0-1 .. j0+vty,   cols from i0-4   (LPQ)
 //   qm     rows j0 .. j0+vty-1,   cols from i0     (LO = VTX)
 //   d2     rows j0-2 .. j0+vty+1, cols from i0-2   (L2 = VTX+4 = 64), computed
 //   d4     rows j0-1 .. j0+vty,   cols from i0-1   (L1 = VTX+2), computed
 // The x-origins are multiples of 4 elements (16 bytes), as tensor loads need.
-// Closed-box tiles arrive by TMA (one thread issues, an mbarrier counts the
-// bytes); channel tiles wrap periodically and come by cp.async.  Thread
+// Tiles arrive by TMA (one thread issues, an mbarrier counts the bytes), but
+// for a channel's at the seam, which wrap and come by cp.async.  Thread
 // (lane x, strip y) owns column x of each phase and marches down a strip of
 // rows with a rolling window of the stencil in registers.
 struct VortLayout {
@@ -271,16 +267,16 @@ __host__ __device__ __forceinline__ VortLayout vort_layout(int vt, int esz) {
     L.total = L.by + vort_round(vt * 8 / esz + 1, esz);   // vt doubles
     return L;
 }
-// Rows of vorticity tiles: a box tiles its interior rows, a channel all.
-__host__ __device__ __forceinline__ int vort_tile_rows(int nyp, int cyclic, int vt) {
-    return cyclic ? (nyp + vt - 1) / vt : (nyp - 2 + vt - 1) / vt;
-}
+// Rows of vorticity tiles (of the interior rows) and CTAs of a basin: a
+// channel's strip integrals first (one CTA per wall and layer), then the tiles.
+__host__ __device__ __forceinline__ int vort_tile_rows(int nyp, int vt) { return (nyp - 2 + vt - 1) / vt; }
+__host__ __device__ __forceinline__ int vort_strips(int nl, int cyclic) { return cyclic ? 2 * nl : 0; }
 // Dynamic shared bytes of k_vort (plus slack to align the base to 128 bytes).
 __host__ __device__ __forceinline__ size_t vort_smem_bytes(int vt, int esz) {
     return (size_t)vort_layout(vt, esz).total * esz + 128;
 }
 
-// Tensor maps of a box basin, in this order: p/q-shaped boxes of F[0..3],
+// Tensor maps of a basin, in this order: p/q-shaped boxes of F[0..3],
 // pm-shaped boxes of F[0], F[1], qm-shaped boxes of F[2], F[3], wekp.
 #define OQG_TMAP_PQ 0
 #define OQG_TMAP_PM 4
@@ -289,21 +285,84 @@ __host__ __device__ __forceinline__ size_t vort_smem_bytes(int vt, int esz) {
 #define OQG_NTMAP 9
 #define OQG_TMAP_BYTES 128
 
+// The channel's strip integrands (vorticity.F90:84-101, numerics.F90:374-386)
+// along one wall of layer k, summed over x by one CTA: with rows counted from
+// the wall, q(0) dp(1), q(1) dp(1) (dp the zonal difference of p), the steps
+// of del2(pm), del4(pm) and (drag layer) pm from row 0 to row 1, signed
+// northward.  part: [2 walls][nl][OQG_NSTRIP].
+template <class T>
+__device__ __forceinline__ void vort_strip(const BasinDev &b, int side, int k, int par) {
+    const int N = b.nxp - 1, px = b.px;
+    const size_t lay = (size_t)k * b.nyp * px;
+    auto row = [&](const void *f, int d) { return (const T *)f + lay + (size_t)(side ? b.nyp - 1 - d : d) * px; };
+    const T *p1 = row(b.F[par], 1), *q0 = row(b.F[2 + par], 0), *q1 = row(b.F[2 + par], 1);
+    const T *m0 = row(b.F[1 - par], 0), *m1 = row(b.F[1 - par], 1), *m2 = row(b.F[1 - par], 2), *m3 = row(b.F[1 - par], 3);
+    const T fx = (T)b.fx, fy = (T)b.fy, fyb = (T)b.fy_bc;
+    const bool qa = q_anom_stored<T>();
+    const double by0 = qa ? b.beta * b.yprel[side ? b.nyp - 1 : 0] : 0.0;
+    const double by1 = qa ? b.beta * b.yprel[side ? b.nyp - 2 : 1] : 0.0;
+    double s[OQG_NSTRIP];
+#pragma unroll
+    for (int x = 0; x < OQG_NSTRIP; ++x) s[x] = 0.0;
+    for (int i = threadIdx.x; i < N; i += blockDim.x) {
+        auto wrap = [&](int c) { return c < 0 ? c + N : c >= N ? c - N : c; };
+        const int w2 = wrap(i - 2), w1 = wrap(i - 1), e1 = wrap(i + 1), e2 = wrap(i + 2);
+        const double dp = (double)(p1[e1] - p1[w1]);
+        s[0] += ((double)q0[i] + by0) * dp;
+        s[1] += ((double)q1[i] + by1) * dp;
+        auto lap = [&](T w, T e, T sv, T nv, T c) { return fx * (w + e - (T)2 * c) + fy * (sv + nv - (T)2 * c); };
+        const T d20 = fyb * (m1[i] - m0[i]);
+        const T d21 = lap(m1[w1], m1[e1], m0[i], m2[i], m1[i]);
+        const T d21w = lap(m1[w2], m1[i], m0[w1], m2[w1], m1[w1]), d21e = lap(m1[i], m1[e2], m0[e1], m2[e1], m1[e1]);
+        const T d22 = lap(m2[w1], m2[e1], m1[i], m3[i], m2[i]);
+        const T d40 = fyb * (d21 - d20), d41 = lap(d21w, d21e, d20, d22, d21);
+        s[2] += (double)(d21 - d20);
+        s[3] += (double)(d41 - d40);
+        if (k == b.kt) s[4] += (double)(m1[i] - m0[i]);
+    }
+    __shared__ double red[OQG_NSTRIP][2 * VWIDE];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int x = 0; x < OQG_NSTRIP; ++x) s[x] += __shfl_down_sync(0xffffffffu, s[x], o);
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+        for (int x = 0; x < OQG_NSTRIP; ++x) red[x][threadIdx.x >> 5] = s[x];
+    __syncthreads();
+    if (threadIdx.x < OQG_NSTRIP) {
+        const int x = threadIdx.x;
+        double v = red[x][0];
+        for (int u = 1; u < (int)blockDim.x / 32; ++u) v += red[x][u];
+        if (side && x >= 2) v = -v;
+        b.part_tile[((size_t)side * b.nl + k) * OQG_NSTRIP + x] = v;
+    }
+}
+
 // tdt = 0: each member steps with its own b.tdt_m (ensemble launches).
 // VT: the tile's rows (b.vty), a compile-time multiple of 4 (vort_tile_rows),
 // so every strip's row loop has a fixed trip count: the loops unroll with no
 // predicates and the rolling windows live in renamed registers.
-template <class T, int NL, int VT>
-__global__ void __launch_bounds__(VTHREADS, 2)
+// NS row strips of 64 threads: VSTRIPS, or VWIDE where the tiles are no more
+// than the SMs, so that a CTA has its SM to itself: the rows a thread marches
+// in each phase halve.
+template <class T, int NL, int VT, int NS>
+__global__ void __launch_bounds__(64 * NS, NS == VSTRIPS ? 2 : 1)
 k_vort(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par, double tdt) {
-    static_assert(VT % 4 == 0 && VT >= 8 && VT <= VTYMAX, "tile rows: a multiple of 4 in [8, VTYMAX]");
+    static_assert(VT % NS == 0 && VT >= 8 && VT <= VTYMAX, "tile rows: a multiple of the strips in [8, VTYMAX]");
     constexpr int LPQ = VTX + 8, L2 = VTX + 4, L1 = VTX + 2, LO = VTX;
     constexpr int HPM = VT + 6, H2 = VT + 4, H1 = VT + 2;
-    // rows per strip of each phase (4 strips); the last d4 strip starts
-    // early and recomputes a row or two of its neighbour (the same values)
-    constexpr int RMAX = VT / 4, R2MAX = H2 / 4, R1MAX = (H1 + 3) / 4;
+    // rows per strip of each phase; the last strips of d2 and d4 start early
+    // and recompute a row or two of their neighbours (the same values)
+    constexpr int RMAX = VT / NS, R2MAX = (H2 + NS - 1) / NS, R1MAX = (H1 + NS - 1) / NS;
     const Work w = work[blockIdx.x];
     const BasinDev &b = bas[w.member];
+    const int strips = vort_strips(NL, b.cyclic);
+    if (w.block < strips) {
+        pdl_trigger();
+        pdl_wait();
+        vort_strip<T>(b, w.block / NL, w.block % NL, par);
+        return;
+    }
     // uniform constants in shared memory: fx fy fxb fyb jac | c_ent1 c_wind
     // c_ent2 c_drag tdt | c2[k] | c4[k]; FP64 ctl2m
     __shared__ T sK[11 + 2 * OQG_NLMAX];
@@ -326,10 +385,8 @@ k_vort(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
     GeoS<T> g;
     g.nxp = b.nxp; g.nyp = b.nyp; g.cyclic = b.cyclic; g.K = sK;
     const VortLayout LY = vort_layout(VT, (int)sizeof(T));
-    const int tile_x = w.block % b.tiles_x, tile_y = w.block / b.tiles_x;
-    // a box's tiles cover its interior rows 1 .. nyp-2 (the walls are not
-    // stepped); a channel's start at row 0 (its strip integrals hold row 0)
-    const int i0 = tile_x * VTX, j0 = tile_y * VT + (g.cyclic ? 0 : 1);
+    const int tile = w.block - strips, tile_y = tile / b.tiles_x, tile_x = tile - tile_y * b.tiles_x;
+    const int i0 = tile_x * VTX, j0 = tile_y * VT + 1;
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *sm = reinterpret_cast<T *>(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
@@ -337,16 +394,15 @@ k_vort(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
     T *sD4 = sm + LY.d4;
     T *sWK = sm + LY.wk;
     double *sBY = reinterpret_cast<double *>(sm + LY.by);
-    __shared__ double red[32];
     __shared__ __align__(8) unsigned long long bars[2];
 
     T *QM = (T *)b.F[3 - par];
     const T *ENT = (const T *)b.ent;
     const double *__restrict__ DD = b.ddyn;
-    const int N = g.nxp - 1;
     const int nyp = g.nyp, nxp = g.nxp, px = b.px, kt = b.kt;
     const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
-    const bool tma = !g.cyclic && b.tmaps != nullptr;
+    // a channel's halo tile must lie in its N = nxp - 1 distinct columns as stored
+    const bool tma = b.tmaps != nullptr && (!g.cyclic || (i0 >= 4 && i0 + VTX + 4 <= nxp - 1));
     const unsigned char *tm = (const unsigned char *)b.tmaps;
 
     if (tma && threadIdx.x == 0) {
@@ -398,8 +454,6 @@ k_vort(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
 #pragma unroll
         for (int m = 0; m < NL; ++m) acc[u][m] = 0.0;
     const bool topo = b.topo_active != 0;
-    // channel strip integrals are formed by tiles holding rows 0, 1, nyp-2, nyp-1
-    const bool strips = g.cyclic && (j0 <= 1 || j0 + VT > nyp - 2);
     // in-domain test of a column (a channel has none outside)
     auto colok = [&](int gi) { return g.cyclic || (gi >= 0 && gi < nxp); };
     // the del2 region (rows j0-2 .. j0+VT+1, columns i0-2 .. i0+VTX+1) lies
@@ -444,7 +498,7 @@ k_vort(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
                 const int gi = i0 - 2 + tx, cs = tx + 2;          // column in the pm tile
                 const bool cv = colok(gi);
                 const bool wl = !g.cyclic && gi == 0, wr = !g.cyclic && gi == nxp - 1;
-                const int rb = ty * R2;          // H2 = 4 R2: the strips tile exactly
+                const int rb = min(ty * R2, H2 - R2);
                 const T *col = sPM + rb * LPQ + cs;
                 T sv = col[0], cv_ = col[LPQ];
     #pragma unroll
@@ -571,57 +625,6 @@ k_vort(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
         };
         if (interior) layer(std::true_type{});
         else layer(std::false_type{});
-        if (strips) {
-            // channel strip integrands (vorticity.F90:84-101, numerics.F90:374-386)
-            // of the rows 0, 1, nyp-2, nyp-1 held by this tile
-            double sq[OQG_NQ];
-#pragma unroll
-            for (int q = 0; q < OQG_NQ; ++q) sq[q] = 0.0;
-            const int gi = i0 + tx;
-            if (ty == 0 && tx < VTX && gi < N) {
-                for (int r = 0; r < VT; ++r) {
-                    const int gj = j0 + r;
-                    if (!(gj == 0 || gj == 1 || gj == nyp - 2 || gj == nyp - 1)) continue;
-                    const int c = tx + 4;                   // p/q tile column
-                    // q itself (FP32 storage holds q - beta y), in FP64
-                    const double qc = QA ? (double)sQ[(r + 1) * LPQ + c] + sBY[r] : (double)sQ[(r + 1) * LPQ + c];
-                    const T d2 = sD2[(r + 2) * L2 + tx + 2], d4 = sD4[(r + 1) * L1 + tx + 1];
-                    if (gj == 0) {
-                        sq[0] += qc * (double)(sP[(r + 2) * LPQ + c + 1] - sP[(r + 2) * LPQ + c - 1]);
-                        sq[4] += (double)(sD2[(r + 3) * L2 + tx + 2] - d2);
-                        sq[6] += (double)(sD4[(r + 2) * L1 + tx + 1] - d4);
-                        if (k == kt)
-                            sq[8] += (double)(sPM[(r + 4) * LPQ + tx + 4] - sPM[(r + 3) * LPQ + tx + 4]);
-                    }
-                    if (gj == 1) sq[1] += qc * (double)(sP[(r + 1) * LPQ + c + 1] - sP[(r + 1) * LPQ + c - 1]);
-                    if (gj == nyp - 1) {
-                        sq[2] += qc * (double)(sP[r * LPQ + c + 1] - sP[r * LPQ + c - 1]);
-                        sq[5] += (double)(d2 - sD2[(r + 1) * L2 + tx + 2]);
-                        sq[7] += (double)(d4 - sD4[r * L1 + tx + 1]);
-                        if (k == kt)
-                            sq[9] += (double)(sPM[(r + 3) * LPQ + tx + 4] - sPM[(r + 2) * LPQ + tx + 4]);
-                    }
-                    if (gj == nyp - 2) sq[3] += qc * (double)(sP[(r + 1) * LPQ + c + 1] - sP[(r + 1) * LPQ + c - 1]);
-                }
-            }
-            // only the row ty = 0 (warps 0 and 1) holds terms: reduce the
-            // OQG_NQ sums together in those two warps, then add warp 1's to
-            // warp 0's (the value block_sum gives, without its barriers)
-            double *pt = b.part_tile + ((size_t)w.block * b.nl + k) * OQG_NQ;
-            if (ty == 0) {
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                    for (int q = 0; q < OQG_NQ; ++q) sq[q] += __shfl_down_sync(0xffffffffu, sq[q], o);
-                if (threadIdx.x == 32)
-#pragma unroll
-                    for (int q = 0; q < OQG_NQ; ++q) red[q] = sq[q];
-            }
-            __syncthreads();
-            if (threadIdx.x == 0)
-#pragma unroll
-                for (int q = 0; q < OQG_NQ; ++q) pt[q] = sq[q] + red[q];
-        }
         __syncthreads();
     }
 
@@ -1051,32 +1054,53 @@ __device__ __forceinline__ void solve_ax_b_dev(const double (&A)[N * N], const d
 struct XinvScal {
     double alpha[OQG_NLMAX];                             // box
     double c_bt, c_bc1[OQG_NLMAX], c_bc2[OQG_NLMAX];     // channel
-    double S[OQG_NLMAX][OQG_NQ];                         // channel strip sums (scratch)
     int supp;
 };
 
-// The scalar phase of one step, run by one warp of every assembly CTA from
-// the current state st[par] (all CTAs compute the same values); CTA 0 also
-// writes the next state st[1-par].
+// Brings a basin's descriptor into L1 ahead of the dependency wait (a full
+// warp calls it): the scalar phase's loads of constants then hit.
+__device__ __forceinline__ void prefetch_basin(const BasinDev &b) {
+    for (int o = (threadIdx.x & 31) * 128; o < (int)sizeof(BasinDev); o += 32 * 128)
+        asm volatile("prefetch.global.L1 [%0];" ::"l"((const char *)&b + o));
+}
+
+// The scalar phase of one step, run by one warp from the current state st[par]
+// (every caller computes the same values); the writer also writes the next
+// state st[1-par].
 //   update_mass_constr (constraint.F90:167-179);
 //   box_homog's area integrals and 2x2 solve (homog.F90:331-366), from the
 //     dst_w-weighted spectral column sums of the y-solve (the inverse DST is
 //     linear, so the area integral of the modal solution is known before it);
 //   or, for a channel, the strip integrals of the vorticity kernel,
 //     step_constraints (constraint.F90:182-215) and cyclic_homog
-//     (homog.F90:280-329);
+//     (homog.F90:280-329), lane k holding layer k, then mode k;
 //   the suppress_comp_mode schedule and its scalar part (openqg.F90:485-487,
 //     driver.F90:183-188).
+// Bound by the latency of its loads and divisions: the assembly of a channel
+// waits for it, and with one lane looping over the layers it took two thirds
+// of the one-kernel inverse (k_xinv 18.8 us per launch on a 193 x 97 channel).
 template <class T, int NL>
 __device__ __noinline__ void scalar_phase(const BasinDev &b, double tdt, int par, bool writer,
                                           XinvScal *out) {
+    constexpr unsigned ALL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const DevState *st = b.st + par;
+    DevState *nx = b.st + (1 - par);
     const DevForcing *fr = b.frc;
-    double imode[NL];
-    double (*S)[OQG_NQ] = out->S;
+    const long long nt = st->nt;
+    const double ent_xn = fr->ent_xn;
+    // update_mass_constr (constraint.F90:167-179)
+    double dpi[NL], dpip[NL];
+#pragma unroll
+    for (int l = 0; l < NL - 1; ++l) {
+        dpi[l] = st->dpip[l] - tdt * b.gp[l] * (l == 0 ? ent_xn : 0.0);
+        dpip[l] = st->dpi[l];
+    }
+    const int per = b.suppress_period;
+    const bool supp = per > 0 && (nt >> 31 ? nt % per : (long long)((unsigned)nt % (unsigned)per)) == 0;
     if (!b.cyclic) {
         const int nkb = (b.nk + b.ykb - 1) / b.ykb;       // y-solve column groups per mode
+        double imode[NL];
 #pragma unroll
         for (int m = 0; m < NL; ++m) {
             CSum s;
@@ -1085,46 +1109,6 @@ __device__ __noinline__ void scalar_phase(const BasinDev &b, double tdt, int par
             s = csum_warp(s, true);
             imode[m] = s.value() * b.ftnorm * b.dx * b.dy;
         }
-    } else {
-        // strip sums over the tiles touching rows 0, 1, nyp-2, nyp-1: per
-        // layer the OQG_NQ sums together, so their loads and shuffles overlap
-        // (the additions keep warp_sum's order)
-        const int ntile = b.tiles_x * b.tiles_y;
-#pragma unroll 1
-        for (int k = 0; k < NL; ++k) {
-            double acc[OQG_NQ];
-#pragma unroll
-            for (int q = 0; q < OQG_NQ; ++q) acc[q] = 0.0;
-            for (int t = lane; t < ntile; t += 32) {
-                const int ty0 = (t / b.tiles_x) * b.vty;
-                if (ty0 <= 1 || ty0 + b.vty > b.nyp - 2) {
-                    const double *pt = b.part_tile + ((size_t)t * NL + k) * OQG_NQ;
-#pragma unroll
-                    for (int q = 0; q < OQG_NQ; ++q) acc[q] += pt[q];
-                }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                for (int q = 0; q < OQG_NQ; ++q) acc[q] += __shfl_down_sync(0xffffffffu, acc[q], o);
-            if (lane == 0)
-#pragma unroll
-                for (int q = 0; q < OQG_NQ; ++q) S[k][q] = acc[q];
-        }
-        __syncwarp();
-    }
-    if (lane != 0) return;
-    DevState ns;                                          // the next state
-    const long long nt = st->nt;
-    const double ent_xn = fr->ent_xn;
-    // update_mass_constr (constraint.F90:167-179)
-#pragma unroll
-    for (int l = 0; l < NL - 1; ++l) {
-        ns.dpi[l] = st->dpip[l] - tdt * b.gp[l] * (l == 0 ? ent_xn : 0.0);
-        ns.dpip[l] = st->dpi[l];
-    }
-    const int supp = (b.suppress_period > 0 && (nt % b.suppress_period) == 0) ? 1 : 0;
-    if (!b.cyclic) {
         // box_homog (homog.F90:331-366)
         double ik[NL];
 #pragma unroll
@@ -1140,94 +1124,76 @@ __device__ __noinline__ void scalar_phase(const BasinDev &b, double tdt, int par
 #pragma unroll
         for (int x = 0; x < N * N; ++x) { A[x] = b.cdhoc[x]; LU[x] = b.lu[x]; }
 #pragma unroll
-        for (int x = 0; x < N; ++x) { pv[x] = b.piv[x]; rhs[x] = ns.dpi[x] - (ik[x + 1] - ik[x]); }
+        for (int x = 0; x < N; ++x) { pv[x] = b.piv[x]; rhs[x] = dpi[x] - (ik[x + 1] - ik[x]); }
         solve_ax_b_dev<N>(A, LU, pv, rhs, al);
+        if (lane == 0)
 #pragma unroll
-        for (int l = 0; l < N; ++l) out->alpha[l] = al[l];
+            for (int l = 0; l < N; ++l) out->alpha[l] = al[l];
     } else {
-        double cs[NL], cn[NL], csp[NL], cnp[NL];
+        const int k = lane < NL ? lane : NL - 1;
+        const double dx = b.dx, dy = b.dy, f0 = b.fnot;
+        double cs = st->cs[k], cn = st->cn[k];
+        const double csp = st->csp[k], cnp = st->cnp[k];
+        double S[OQG_NSTRIP], R[OQG_NSTRIP];              // the south's and north's strip integrals
 #pragma unroll
-        for (int k = 0; k < NL; ++k) { cs[k] = st->cs[k]; cn[k] = st->cn[k]; csp[k] = st->csp[k]; cnp[k] = st->cnp[k]; }
-        const double dx = b.dx, dy = b.dy;
-        double rhss[NL], rhsn[NL];
-#pragma unroll
-        for (int k = 0; k < NL; ++k) {
-            rhss[k] = -0.5 * dy * b.fnot * fr->int_Be_s[k];
-            rhsn[k] = -0.5 * dy * b.fnot * fr->int_Be_n[k];
+        for (int q = 0; q < OQG_NSTRIP; ++q) {
+            S[q] = b.part_tile[k * OQG_NSTRIP + q];
+            R[q] = b.part_tile[(NL + k) * OQG_NSTRIP + q];
         }
+        double rhss = -0.5 * dy * f0 * fr->int_Be_s[k], rhsn = -0.5 * dy * f0 * fr->int_Be_n[k];
         // step_constraints (constraint.F90:182-215)
-        rhss[0] = rhss[0] + b.tau_sign * (b.fnot / b.h[0]) * fr->txis;
-        rhsn[0] = rhsn[0] - b.tau_sign * (b.fnot / b.h[0]) * fr->txin;
-        const double dfac = b.fnot * b.delek / (2.0 * fabs(b.fnot));
-        double bs = 0.0, bn = 0.0;
-#pragma unroll
-        for (int k = 0; k < NL; ++k)
-            if (k == b.kt) { bs = S[k][8]; bn = S[k][9]; }
-        const double bdrins = dfac * ((bs * dx) / dy), bdrinn = dfac * ((bn * dx) / dy);
-        rhss[NL - 1] = rhss[NL - 1] + (b.fnot / b.h[NL - 1]) * bdrins;
-        rhsn[NL - 1] = rhsn[NL - 1] - (b.fnot / b.h[NL - 1]) * bdrinn;
-#pragma unroll
-        for (int k = 0; k < NL; ++k) {
-            const double a5s = (S[k][0] * dx) / (2.0 * dx), a9s = (S[k][1] * dx) / (2.0 * dx);
-            const double a5n = (S[k][2] * dx) / (2.0 * dx), a9n = (S[k][3] * dx) / (2.0 * dx);
-            const double ajis = (a5s + 2.0 * a9s) / 6.0, ajin = -(a5n + 2.0 * a9n) / 6.0;
-            const double ap3s = b.ah2[k] * (S[k][4] * dx) / dy, ap3n = b.ah2[k] * (S[k][5] * dx) / dy;
-            const double ap5s = b.ah4[k] * (S[k][6] * dx) / dy, ap5n = b.ah4[k] * (S[k][7] * dx) / dy;
-            rhss[k] = rhss[k] + ajis - ap3s + ap5s;
-            rhsn[k] = rhsn[k] + ajin + ap3n - ap5n;
+        if (k == 0) {
+            rhss = rhss + b.tau_sign * (f0 / b.h[0]) * fr->txis;
+            rhsn = rhsn - b.tau_sign * (f0 / b.h[0]) * fr->txin;
         }
-#pragma unroll
-        for (int k = 0; k < NL; ++k) {
-            const double csn = csp[k] + tdt * rhss[k];
-            const double cnn = cnp[k] + tdt * rhsn[k];
-            csp[k] = cs[k];
-            cnp[k] = cn[k];
-            cs[k] = csn;
-            cn[k] = cnn;
+        const double bs = __shfl_sync(ALL, S[4], b.kt), bn = __shfl_sync(ALL, R[4], b.kt);
+        if (k == NL - 1) {
+            const double dfac = f0 * b.delek / (2.0 * fabs(f0)), fh = f0 / b.h[NL - 1];
+            rhss = rhss + fh * (dfac * ((bs * dx) / dy));
+            rhsn = rhsn - fh * (dfac * ((bn * dx) / dy));
         }
-        // cyclic_homog (homog.F90:280-329).  The x-integral of row j of the
+        const double a5s = (S[0] * dx) / (2.0 * dx), a9s = (S[1] * dx) / (2.0 * dx);
+        const double a5n = (R[0] * dx) / (2.0 * dx), a9n = (R[1] * dx) / (2.0 * dx);
+        const double ajis = (a5s + 2.0 * a9s) / 6.0, ajin = -(a5n + 2.0 * a9n) / 6.0;
+        const double ap3s = b.ah2[k] * (S[2] * dx) / dy, ap3n = b.ah2[k] * (R[2] * dx) / dy;
+        const double ap5s = b.ah4[k] * (S[3] * dx) / dy, ap5n = b.ah4[k] * (R[3] * dx) / dy;
+        rhss = rhss + ajis - ap3s + ap5s;
+        rhsn = rhsn + ajin + ap3n - ap5n;
+        const double csn = csp + tdt * rhss, cnn = cnp + tdt * rhsn;
+        // cyclic_homog (homog.F90:280-329), lane m.  The x-integral of row j of the
         // modal solution is dx times its zero wavenumber (before the 1/N of the
         // inverse transform, which the N-term row sum cancels).
         typedef typename C2<T>::t T2;
-        const T2 *Sp = (const T2 *)b.spec;
-        double clhss[NL], clhsn[NL];
+        const T2 *Sp = (const T2 *)b.spec + (size_t)k * b.ny * b.pk;
+        const double u0s = (double)Sp[0].x, u0n = (double)Sp[(size_t)(b.ny - 1) * b.pk].x;
+        double ss = 0.0, sn = 0.0;
 #pragma unroll
-        for (int m = 0; m < NL; ++m) {
-            double ss = 0.0, sn = 0.0;
-#pragma unroll
-            for (int k = 0; k < NL; ++k) {
-                ss += b.ctl2m[k + NL * m] * cs[k];
-                sn += b.ctl2m[k + NL * m] * cn[k];
-            }
-            const double u0s = (double)Sp[((size_t)m * b.ny) * b.pk].x;
-            const double u0n = (double)Sp[((size_t)m * b.ny + (b.ny - 1)) * b.pk].x;
-            clhss[m] = ss + (u0s * dx) / dy;
-            clhsn[m] = sn + (u0n * dx) / dy;
+        for (int l = 0; l < NL; ++l) {
+            const double c = b.ctl2m[l + NL * k];
+            ss += c * __shfl_sync(ALL, csn, l);
+            sn += c * __shfl_sync(ALL, cnn, l);
         }
-        out->c_bt = clhss[0] * b.hbsi;
-#pragma unroll
-        for (int m = 1; m < NL; ++m) {
-            out->c_bc1[m] = b.hc2n[m] * clhss[m] - b.hc2s[m] * clhsn[m];
-            out->c_bc2[m] = b.hc1s[m] * clhsn[m] - b.hc1n[m] * clhss[m];
+        const double clhss = ss + (u0s * dx) / dy, clhsn = sn + (u0n * dx) / dy;
+        if (lane == 0) out->c_bt = clhss * b.hbsi;
+        else if (lane < NL) {
+            out->c_bc1[k] = b.hc2n[k] * clhss - b.hc2s[k] * clhsn;
+            out->c_bc2[k] = b.hc1s[k] * clhsn - b.hc1n[k] * clhss;
         }
-        // suppress_comp_mode's channel scalars (driver.F90:185-188)
-#pragma unroll
-        for (int k = 0; k < NL; ++k) {
-            if (supp) { cs[k] = 0.5 * (cs[k] + csp[k]); cn[k] = 0.5 * (cn[k] + cnp[k]); }
-            ns.cs[k] = cs[k]; ns.cn[k] = cn[k]; ns.csp[k] = csp[k]; ns.cnp[k] = cnp[k];
+        if (writer && lane < NL) {
+            // suppress_comp_mode's channel scalars (driver.F90:185-188)
+            nx->cs[k] = supp ? 0.5 * (csn + cs) : csn;
+            nx->cn[k] = supp ? 0.5 * (cnn + cn) : cnn;
+            nx->csp[k] = cs;
+            nx->cnp[k] = cn;
         }
     }
-    out->supp = supp;
+    if (lane != 0) return;
+    out->supp = supp ? 1 : 0;
     if (!writer) return;
-    DevState *nx = b.st + (1 - par);
 #pragma unroll
     for (int l = 0; l < NL - 1; ++l) {
-        nx->dpi[l] = supp ? 0.5 * (ns.dpi[l] + ns.dpip[l]) : ns.dpi[l];
-        nx->dpip[l] = ns.dpip[l];
-    }
-    if (b.cyclic) {
-#pragma unroll
-        for (int k = 0; k < NL; ++k) { nx->cs[k] = ns.cs[k]; nx->cn[k] = ns.cn[k]; nx->csp[k] = ns.csp[k]; nx->cnp[k] = ns.cnp[k]; }
+        nx->dpi[l] = supp ? 0.5 * (dpi[l] + dpip[l]) : dpi[l];
+        nx->dpip[l] = dpip[l];
     }
     nx->nt = nt + 1;
 }
@@ -1243,10 +1209,11 @@ __device__ __noinline__ void scalar_phase(const BasinDev &b, double tdt, int par
 template <class T>
 __device__ __forceinline__ bool xinv_scalar_cta(const BasinDev *__restrict__ bas, int scal, int par, double tdt) {
     if (scal <= 0 || (int)blockIdx.x < (int)gridDim.x - scal) return false;
+    const BasinDev &b = bas[blockIdx.x - (gridDim.x - scal)];
     pdl_trigger();
+    if (threadIdx.x < 32) prefetch_basin(b);
     pdl_wait();
     if (threadIdx.x < 32) {
-        const BasinDev &b = bas[blockIdx.x - (gridDim.x - scal)];
         const double dt = tdt != 0.0 ? tdt : b.tdt_m;
         XinvScal *sc = (XinvScal *)b.scal_g;
         if (b.nl == 2) scalar_phase<T, 2>(b, dt, par, true, sc);
@@ -1388,307 +1355,222 @@ k_xinv_rows(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int
 }
 
 // ------------------------------------------------------------------ k_xinv
-// Rows of one CTA: interior rows [jlo, jhi) plus wall row 0 (first CTA) and
-// wall row nyp-1 (last CTA).
-__device__ __forceinline__ void xinv_rows(const BasinDev &b, int rb, int &jlo, int &jhi,
-                                          int &jfirst, int &nra) {
-    jlo = 1 + rb * b.k4_rows;
-    jhi = min(jlo + b.k4_rows, b.nyp - 1);
-    jfirst = (rb == 0) ? 0 : jlo;
-    int jlast = (jhi == b.nyp - 1) ? b.nyp - 1 : jhi - 1;
-    nra = jlast - jfirst + 1;
+// The inverse x-transforms and the assembly as one launch: a CTA transforms
+// one row pair of every mode, then forms the layers of those rows (the first
+// and last CTA the wall rows too).  The last warp runs the scalar phase of the
+// step while the others transform; every CTA computes the same scalars, the
+// first writes the next state.  Threads: NL transforms' (at least 128), and
+// the scalar warp.  Bound by latency: on a 193 x 97 channel the 48 CTAs run one
+// transform and 400 points each.  With the transform's length compiled in, 128
+// threads and a warp that runs the scalars lane by layer, the launch takes 15 us
+// (5 of them the launch's own) where the kernel it replaces, any-length, with
+// its modal rows cleared and rewritten in place, took 27.
+__host__ __device__ __forceinline__ int xinv_tt(int M, int cyclic) { return cyclic ? (M + XINV_E - 1) / XINV_E : odd_tt(M); }
+__host__ __device__ __forceinline__ int xinv_threads(int M, int cyclic, int nl) {
+    const int t = (nl * xinv_tt(M, cyclic) + 31) / 32 * 32;
+    return t > 128 ? t : 128;
+}
+// Dynamic shared bytes: the transforms' buffers; the modal rows take the
+// buffer that the last stage leaves free, or follow an in-place transform's.
+__host__ __device__ __forceinline__ size_t xinv_bytes(int M, int cyclic, int nl, int nxp, int esz) {
+    const size_t buf = (size_t)nl * 2 * esz * (cyclic ? 2 * fft_buf_len(M) : odd_smem_len(M));
+    return buf + (!cyclic && odd_ct_len(M) ? (size_t)nl * 2 * nxp * esz : 0);
 }
 
-// The last warp of the CTA runs the scalar phase of the step while the
-// other nfft = blockDim.x - 32 threads run the inverse transforms; those
-// synchronise among themselves on named barrier 1.
-// out != null: solve-only mode, writes the modal inhomogeneous solutions
-// (FP64, [nl][nyp][px]) and nothing else (no scalar phase).
-// tdt = 0: each member steps with its own b.tdt_m (ensemble launches).
-template <class T, int NL>
-__global__ void __maxnreg__(112)
-k_xinv(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par, double tdt, double *out) {
-    typedef typename C2<T>::t T2;
-    const Work w = work[blockIdx.x];
-    const BasinDev &b = bas[w.member];
-    const int nfft = blockDim.x - 32;
-    const bool fft_thread = (int)threadIdx.x < nfft;
-    const int M = b.M, TT = (M + XINV_E - 1) / XINV_E, G = nfft / TT;
-    const int g = threadIdx.x / TT, t = threadIdx.x - g * TT;
-    int jlo, jhi, jfirst, nra;
-    xinv_rows(b, w.block, jlo, jhi, jfirst, nra);
-    const int nr = jhi - jlo;                    // interior rows
-    const int nxp = b.nxp, n = b.nxin, nyp = b.nyp, px = b.px;
-    const int LB = fft_buf_len(M);
-    const int npr = (nr + 1) >> 1;               // row pairs per mode
-    const int npairs = NL * npr;
-    const bool one_round = G >= npairs;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ XinvScal sS;
-    // Two sets of G transform buffers; each transform starts in the set that
-    // makes its last stage end in set A, and its spectral rows are staged in
-    // the other.  With every row pair in one round the modal rows inh alias
-    // set B once the transforms are done; otherwise they follow both sets.
-    // Grids too wide for the modal rows in shared memory keep them in the
-    // global buffer b.inh_g ([nl][nyp][px], rows of this CTA only).
-    T2 *setA = reinterpret_cast<T2 *>(smem_raw), *setB = setA + (size_t)G * LB;
-    T2 *set_in = (b.nrad & 1) ? setB : setA, *set_st = (b.nrad & 1) ? setA : setB;
-    const bool split = b.xinv_split != 0;
-    const bool alias = one_round && !split;
-    // a row of the spectral buffer: n reals (box) or nk complex (channel)
-    const int rowbytes = b.cyclic ? b.nk * (int)sizeof(T2) : n * (int)sizeof(T);
-    const int RO = round16(rowbytes) / (int)sizeof(T);   // second row offset (T units)
-    T *inh;
-    size_t ms, rs;                               // mode and row strides of inh
-    if (split) { inh = (T *)b.inh_g + (size_t)jfirst * px; ms = (size_t)nyp * px; rs = px; }
-    else {
-        inh = alias ? reinterpret_cast<T *>(setB) : reinterpret_cast<T *>(setA + (size_t)2 * G * LB);
-        ms = (size_t)nra * nxp;
-        rs = nxp;
-    }
-    const T ftn = (T)b.ftnorm;
-
-    pdl_trigger();
-    if (!fft_thread) {
-        pdl_wait();
-        if (!out) scalar_phase<T, NL>(b, tdt != 0.0 ? tdt : b.tdt_m, par, w.block == 0, &sS);
-    } else if (split && b.xinv_sep) {
-        // (solve-only mode) the modal rows come from k_xinv_rows
-        pdl_wait();
-    } else {
-    // zero the wall rows / columns of the modal fields
-    if (!alias)
-        for (int m = 0; m < NL; ++m)
-            for (int lr = 0; lr < nra; ++lr)
-                for (int i = threadIdx.x; i < nxp; i += nfft) inh[m * ms + lr * rs + i] = (T)0;
-    pdl_wait();
-
-    for (int base = 0; base < npairs; base += G) {
-        const int pair = base + g;
-        const bool live = g < G && pair < npairs;
-        const int m = live ? pair / npr : 0;
-        const int r0 = live ? 2 * (pair - m * npr) : 0;     // interior row offset
-        const bool two = live && r0 + 1 < nr;
-        T2 *za = set_in + (size_t)(g < G ? g : 0) * LB;
-        T2 *zb = set_st + (size_t)(g < G ? g : 0) * LB;
-        T *raw = reinterpret_cast<T *>(zb);
-        const int sj = jlo + r0 - 1;                        // spectral row
-        const char *srow = (const char *)b.spec + ((size_t)m * b.ny + sj) * b.pk * (b.cyclic ? sizeof(T2) : sizeof(T));
-        const size_t pitchb = (size_t)b.pk * (b.cyclic ? sizeof(T2) : sizeof(T));
-        if (live) {
-            cp_async_16(raw, srow, round16(rowbytes), t, TT);
-            if (two) cp_async_16(raw + RO, srow + pitchb, round16(rowbytes), t, TT);
-        }
-        cp_async_commit_wait_all();
-        bar_sync(1, nfft);
-        if (live) {
-            if (!b.cyclic) {
-                const T *x = raw, *y = raw + RO;
-                // odd extension: z_0 = z_{n+1} = 0, z_{M-jj} = -z_jj
-                if (t == 0) {
-                    T2 zero;
-                    zero.x = (T)0;
-                    zero.y = (T)0;
-                    za[fpad(0)] = zero;
-                    za[fpad(n + 1)] = zero;
-                }
-                for (int jj = 1 + t; jj <= n; jj += TT) {
-                    T2 v, vm;
-                    v.x = ftn * x[jj - 1];
-                    v.y = two ? ftn * y[jj - 1] : (T)0;
-                    vm.x = -v.x;
-                    vm.y = -v.y;
-                    za[fpad(jj)] = v;
-                    za[fpad(M - jj)] = vm;
-                }
-            } else {
-                const T2 *x = reinterpret_cast<const T2 *>(raw), *y = reinterpret_cast<const T2 *>(raw + RO);
-                for (int kk = t; kk < M; kk += TT) {
-                    T2 X, Y;
-                    const bool lo = kk <= M / 2;
-                    const int ks = lo ? kk : M - kk;
-                    X = x[ks];
-                    if (two) Y = y[ks]; else { Y.x = (T)0; Y.y = (T)0; }
-                    if (!lo) { X.y = -X.y; Y.y = -Y.y; }
-                    if (kk == 0 || 2 * kk == M) { X.y = (T)0; Y.y = (T)0; }
-                    // conj(ftnorm (X + iY))
-                    T2 v;
-                    v.x = ftn * X.x - ftn * Y.y;
-                    v.y = -(ftn * X.y + ftn * Y.x);
-                    za[fpad(kk)] = v;
-                }
-            }
-        }
-        bar_sync(1, nfft);
-        T2 *z = fft_run<T, XINV_E>(za, zb, M, b.rad, b.nrad, (const T2 *)b.tw, live ? t : TT, TT, 1, nfft);
-        if (alias) {
-            // set B is free now: clear it for the modal rows
-            for (int idx = threadIdx.x; idx < NL * nra * nxp; idx += nfft) inh[idx] = (T)0;
-            bar_sync(1, nfft);
-        }
-        if (live) {
-            const int lr = (jlo + r0) - jfirst;
-            T *ox = inh + m * ms + lr * rs;
-            T *oy = ox + rs;
-            if (!b.cyclic) {
-                for (int kk = t; kk < n; kk += TT) {
-                    const T2 v = z[fpad(kk + 1)];
-                    ox[kk + 1] = -v.y;
-                    if (two) oy[kk + 1] = v.x;
-                }
-            } else {
-                for (int i = t; i < M; i += TT) {
-                    const T2 v = z[fpad(i)];
-                    ox[i] = v.x;
-                    if (two) oy[i] = -v.y;
-                }
-                if (t == 0) {
-                    const T2 v = z[fpad(0)];
-                    ox[M] = v.x;
-                    if (two) oy[M] = -v.y;
-                }
-            }
-        }
-        bar_sync(1, nfft);
-    }
-    }   // fft threads
-    __syncthreads();
-
-    if (out) {
-        for (int idx = threadIdx.x; idx < NL * nra * nxp; idx += blockDim.x) {
-            const int m = idx / (nra * nxp), rem = idx - m * nra * nxp;
-            const int lr = rem / nxp, i = rem - lr * nxp;
-            out[((size_t)m * nyp + jfirst + lr) * px + i] = (double)inh[m * ms + lr * rs + i];
-        }
-        return;
-    }
-
-    // homogeneous correction + modes_to_layers, in place (modes -> layers)
-    const XinvScal *sc = &sS;
-    const int supp = sc->supp;
-    double ctm[NL * NL], hc[NL > 1 ? NL - 1 : 1];
-#pragma unroll
-    for (int x = 0; x < NL * NL; ++x) ctm[x] = b.ctm2l[x];
+// The assembly of rows jfirst .. jlast of a basin (see k_xinv_asm): inh(m, j, i)
+// is the modal solution at a point.
+template <class T, int NL, class Inh>
+__device__ __forceinline__ void xinv_assemble(const BasinDev &b, int par, const XinvScal *sc, int jfirst, int jlast, Inh inh) {
+    const int nxp = b.nxp, nyp = b.nyp, px = b.px;
+    const size_t ms = (size_t)nyp * px;
+    const T *__restrict__ H = (const T *)b.hsb;
     const T *__restrict__ Pold = (const T *)b.F[par];
     T *__restrict__ Pnew = (T *)b.F[1 - par];
-    const size_t n2 = (size_t)nyp * px;
-    if (!b.cyclic) {
+    T *__restrict__ Qc = (T *)b.F[3 - par];          // q after this step
+    const T *__restrict__ Qm = (const T *)b.F[2 + par];
+    const bool cyc = b.cyclic != 0, supp = sc->supp != 0;
+    double ctm[NL * NL], hc[2 * NL];
 #pragma unroll
-        for (int m = 1; m < NL; ++m) hc[m - 1] = sc->alpha[m - 1];
+    for (int x = 0; x < NL * NL; ++x) ctm[x] = b.ctm2l[x];
+#pragma unroll
+    for (int m = 0; m < NL; ++m) {
+        hc[m] = !cyc ? (m ? sc->alpha[m - 1] : 0.0) : m ? sc->c_bc1[m] : sc->c_bt;
+        hc[NL + m] = cyc && m ? sc->c_bc2[m] : 0.0;
     }
-    const T *__restrict__ H = (const T *)b.hsb;
-    const FastDiv fdx(nxp);
-    constexpr int U = 4;
-    for (int base = threadIdx.x; base < nra * nxp; base += U * blockDim.x) {
-        // gather the inputs of U points first (independent loads), then compute
-        double hv[U][NL], po[U][NL];
-        int lrs[U], is[U];
+    auto layers = [&](int j, int i, T *pn) {
+        const size_t o2 = (size_t)j * px + i;
+        double pm_[NL];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int idx = base + u * blockDim.x;
-            const bool ok = idx < nra * nxp;
-            const int lr = ok ? fdx.div(idx) : 0, i = ok ? idx - lr * nxp : 0;
-            const int j = jfirst + lr;
-            lrs[u] = ok ? lr : -1;
-            is[u] = i;
-#pragma unroll
-            for (int m = 0; m < NL; ++m) {
-                po[u][m] = (ok && supp) ? (double)Pold[m * n2 + (size_t)j * px + i] : 0.0;
-                if (!b.cyclic) hv[u][m] = (ok && m >= 1) ? (double)H[((size_t)(m - 1) * nyp + j) * px + i] : 0.0;
-                else if (m == 0) hv[u][m] = ok ? b.hbt[j] : 0.0;
-                else hv[u][m] = ok ? b.hbc1[m * nyp + j] : 0.0;
-            }
+        for (int m = 0; m < NL; ++m) {
+            double h = 0.0;
+            if (!cyc) { if (m) h = hc[m] * (double)H[(m - 1) * ms + o2]; }
+            else h = m ? hc[m] * b.hbc1[m * nyp + j] + hc[NL + m] * b.hbc2[m * nyp + j] : hc[0] * b.hbt[j];
+            pm_[m] = inh(m, j, i) + h;
         }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (lrs[u] < 0) continue;
-            const int lr = lrs[u], i = is[u], j = jfirst + lr;
-            double pm_[NL];
-#pragma unroll
-            for (int m = 0; m < NL; ++m) pm_[m] = (double)inh[m * ms + lr * rs + i];
-            if (!b.cyclic) {
-#pragma unroll
-                for (int m = 1; m < NL; ++m) pm_[m] = pm_[m] + hc[m - 1] * hv[u][m];
-            } else {
-                pm_[0] = pm_[0] + sc->c_bt * hv[u][0];
-#pragma unroll
-                for (int m = 1; m < NL; ++m)
-                    pm_[m] = pm_[m] + (sc->c_bc1[m] * hv[u][m] + sc->c_bc2[m] * b.hbc2[m * nyp + j]);
-            }
-#pragma unroll
-            for (int k = 0; k < NL; ++k) {
-                double s2 = 0.0;
-#pragma unroll
-                for (int m = 0; m < NL; ++m) s2 += pm_[m] * ctm[m + NL * k];
-                const T pn = (T)s2;
-                // ocqbdy reads the layer values on and next to the walls
-                // (in shared memory they go back everywhere)
-                if (!split || i <= 1 || i >= nxp - 2 || j <= 1 || j >= nyp - 2) inh[k * ms + lr * rs + i] = pn;
-                Pnew[k * n2 + (size_t)j * px + i] = supp ? (T)((T)0.5 * (pn + (T)po[u][k])) : pn;
-            }
-        }
-    }
-    __syncthreads();
-
-    // ocqbdy (vorsubs.F90:58-114) on the walls of these rows, then the
-    // suppress_comp_mode average of q (driver.F90:180)
-    T *Qc = (T *)b.F[3 - par];        // q after this step (qm buffer of K1)
-    const T *Qm = (const T *)b.F[2 + par];
-    const T fac = (T)b.qb_fac;
-    // the point (lr, i) of these rows: q's average on a suppression step,
-    // ocqbdy's value on a wall
-    auto wall_point = [&](int lr, int i) {
-        const int j = jfirst + lr;
-        const bool zon = (j == 0 || j == nyp - 1);
-        const bool mer = !b.cyclic && (i == 0 || i == nxp - 1);
-        if (!zon && !mer) {
-            if (supp)
-                for (int k = 0; k < NL; ++k) {
-                    const size_t o3 = ((size_t)k * nyp + j) * px + i;
-                    Qc[o3] = (T)0.5 * (Qc[o3] + Qm[o3]);
-                }
-            return;
-        }
-        const int cnt = (zon ? 1 : 0) + (mer ? 1 : 0);
-#define PN(kk, rr, ii) inh[(kk) * ms + (rr) * rs + (ii)]
-        T pv[NL];
-#pragma unroll
-        for (int k = 0; k < NL; ++k) pv[k] = PN(k, lr, i);
 #pragma unroll
         for (int k = 0; k < NL; ++k) {
-            T qv;
-            if (mer) {
-                qv = (i == 0) ? fac * (PN(k, lr, 1) - pv[k]) : fac * (PN(k, lr, nxp - 2) - pv[k]);
-            } else {
-                qv = (j == 0) ? fac * (PN(k, lr + 1, i) - pv[k]) : fac * (PN(k, lr - 1, i) - pv[k]);
-            }
+            double s2 = 0.0;
+#pragma unroll
+            for (int m = 0; m < NL; ++m) s2 += pm_[m] * ctm[m + NL * k];
+            pn[k] = (T)s2;
+        }
+    };
+    const T fac = (T)b.qb_fac;
+    const FastDiv fdx(nxp);
+    const int npts = (jlast - jfirst + 1) * nxp;
+    for (int idx = threadIdx.x; idx < npts; idx += blockDim.x) {
+        const int jr = fdx.div(idx), i = idx - jr * nxp, j = jfirst + jr;
+        const size_t o2 = (size_t)j * px + i;
+        T pn[NL];
+        layers(j, i, pn);
+#pragma unroll
+        for (int k = 0; k < NL; ++k)
+            Pnew[k * ms + o2] = supp ? (T)((T)0.5 * (pn[k] + Pold[k * ms + o2])) : pn[k];
+        const bool zon = (j == 0 || j == nyp - 1), mer = !cyc && (i == 0 || i == nxp - 1);
+        if (!zon && !mer) {
+            if (supp)
+#pragma unroll
+                for (int k = 0; k < NL; ++k) Qc[k * ms + o2] = (T)0.5 * (Qc[k * ms + o2] + Qm[k * ms + o2]);
+            continue;
+        }
+        // ocqbdy (vorsubs.F90:58-114): the inner neighbour across the meridional
+        // wall (a corner takes that one), else across the zonal wall
+        T pnb[NL];
+        layers(mer ? j : (j == 0 ? 1 : nyp - 2), mer ? (i == 0 ? 1 : nxp - 2) : i, pnb);
+        const int cnt = (zon ? 1 : 0) + (mer ? 1 : 0);
+        const T by = (T)(b.beta * b.yprel[j]);
+#pragma unroll
+        for (int k = 0; k < NL; ++k) {
+            T qv = fac * (pnb[k] - pn[k]);
             double mv = 0.0;
 #pragma unroll
-            for (int l = 0; l < NL; ++l) mv += b.amat[k + NL * l] * (double)pv[l];
+            for (int l = 0; l < NL; ++l) mv += b.amat[k + NL * l] * (double)pn[l];
             const T fmv = (T)(b.fnot * mv);
-            const T by = (T)(b.beta * b.yprel[j]);
             for (int c = 0; c < cnt; ++c) qv = qv - fmv;
             // (FP32 storage holds q - beta y: one beta y fewer)
             for (int c = q_anom_stored<T>() ? 1 : 0; c < cnt; ++c) qv = qv + by;
             if (k == b.kt && b.topo_active) {
-                const T dd = (T)b.ddyn[(size_t)j * px + i];
+                const T dd = (T)b.ddyn[o2];
                 for (int c = 0; c < cnt; ++c) qv = qv + dd;
             }
-            const size_t o3 = ((size_t)k * nyp + j) * px + i;
-            Qc[o3] = supp ? (T)((T)0.5 * (qv + Qm[o3])) : qv;
-        }
-#undef PN
-    };
-    // every point on a suppression step and along the zonal walls; else the
-    // two meridional wall points of each row
-    for (int lr = 0; lr < nra; ++lr) {
-        const int j = jfirst + lr;
-        if (supp || j == 0 || j == nyp - 1) {
-            for (int i = threadIdx.x; i < nxp; i += blockDim.x) wall_point(lr, i);
-        } else if (!b.cyclic && threadIdx.x < 2) {
-            wall_point(lr, threadIdx.x == 0 ? 0 : nxp - 1);
+            Qc[k * ms + o2] = supp ? (T)((T)0.5 * (qv + Qm[k * ms + o2])) : qv;
         }
     }
+}
+
+// MC: as in k_xfwd (channels) and odd_fft (boxes).
+template <class T, bool CYC, int MC>
+__global__ void __maxnreg__(112)
+k_xinv(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par, double tdt) {
+    typedef typename C2<T>::t T2;
+    const Work w = work[blockIdx.x];
+    const BasinDev &b = bas[w.member];
+    const int nfft = blockDim.x - 32, M = MC > 0 ? MC : b.M, TT = xinv_tt(M, CYC), nl = b.nl;
+    const int g = threadIdx.x / TT, t = threadIdx.x - g * TT;
+    const bool live = (int)threadIdx.x < nfft && g < nl;
+    const int j = 2 * w.block, n = b.nxin, nxp = b.nxp;
+    const bool two = j + 1 < b.ny;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ XinvScal sS;
+    const int lz = CYC ? 2 * fft_buf_len(M) : odd_smem_len(M);
+    T2 *z0 = reinterpret_cast<T2 *>(smem_raw), *z = z0 + (size_t)(live ? g : 0) * lz;
+    // transform m's two modal rows
+    T *inh0;
+    size_t li;
+    if (!CYC && odd_ct_len(M)) { inh0 = reinterpret_cast<T *>(z0 + (size_t)nl * lz); li = 2 * (size_t)nxp; }
+    else {
+        const int stages = CYC ? b.nrad : max(b.norad - 1, 1);
+        inh0 = reinterpret_cast<T *>(z0 + ((stages & 1) ? 0 : lz / 2));
+        li = 2 * (size_t)lz;
+    }
+    T *ox = inh0 + (live ? g : 0) * li, *oy = ox + nxp;
+    const T ftn = (T)b.ftnorm;
+    pdl_trigger();
+    if ((int)threadIdx.x >= nfft) prefetch_basin(b);
+    pdl_wait();
+    if ((int)threadIdx.x >= nfft) {
+        const double dt = tdt != 0.0 ? tdt : b.tdt_m;
+        if (nl == 2) scalar_phase<T, 2>(b, dt, par, w.block == 0, &sS);
+        else if (nl == 3) scalar_phase<T, 3>(b, dt, par, w.block == 0, &sS);
+        else scalar_phase<T, 4>(b, dt, par, w.block == 0, &sS);
+    } else if constexpr (CYC) {
+        // the Hermitian extension of X + iY, conjugated (inhomog.F90:214-255)
+        constexpr int U = 4;
+        const int nk = b.nk;
+        const FastDiv fd(nk);
+        for (int x0 = threadIdx.x; x0 < nl * nk; x0 += U * nfft) {
+            T2 X[U], Y[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int x = x0 + u * nfft;
+                X[u].x = X[u].y = Y[u].x = Y[u].y = (T)0;
+                if (x < nl * nk) {
+                    const int m = fd.div(x), kk = x - m * nk;
+                    const T2 *r = (const T2 *)b.spec + ((size_t)m * b.ny + j) * b.pk + kk;
+                    X[u] = __ldcg(r);
+                    if (two) Y[u] = __ldcg(r + b.pk);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int x = x0 + u * nfft;
+                if (x >= nl * nk) break;
+                const int m = fd.div(x), kk = x - m * nk;
+                T2 *zm = z0 + (size_t)m * lz;
+                if (kk == 0 || 2 * kk == M) X[u].y = Y[u].y = (T)0;
+                T2 v;
+                v.x = ftn * X[u].x - ftn * Y[u].y;
+                v.y = -(ftn * X[u].y + ftn * Y[u].x);
+                zm[fpad(kk)] = v;
+                if (kk > 0 && 2 * kk < M) {
+                    v.x = ftn * X[u].x + ftn * Y[u].y;
+                    v.y = -(ftn * Y[u].x - ftn * X[u].y);
+                    zm[fpad(M - kk)] = v;
+                }
+            }
+        }
+        bar_sync(1, nfft);
+        const T2 *r = fft_run<T, XINV_E, MC>(z, z + lz / 2, M, b.rad, b.nrad, (const T2 *)b.tw, live ? t : TT, TT, 1, nfft);
+        if (live) {
+            // every column; column nxp-1 = M repeats column 0 (inhomog.F90:250)
+            for (int i = t; i <= M; i += TT) {
+                const T2 v = r[fpad(i == M ? 0 : i)];
+                ox[i] = v.x;
+                oy[i] = -v.y;
+            }
+        }
+    } else {
+        if (live && t == 0) {
+            T2 zero;
+            zero.x = zero.y = (T)0;
+            z[0] = z[zpad<4>(n + 1)] = zero;
+        }
+        const FastDiv fd(n);
+#pragma unroll 4
+        for (int x = threadIdx.x; x < nl * n; x += nfft) {
+            const int m = fd.div(x), i = x - m * n;
+            const T *r = (const T *)b.spec + ((size_t)m * b.ny + j) * b.pk + i;
+            T2 v;
+            v.x = ftn * __ldcg(r);
+            v.y = two ? ftn * __ldcg(r + b.pk) : (T)0;
+            z0[(size_t)m * lz + zpad<4>(i + 1)] = v;
+        }
+        bar_sync(1, nfft);
+        odd_fft<T, MC>(z, M, b.orad, b.norad, (const T2 *)b.otw, t, TT, live, [&](int i, T2 v) {
+            ox[i] = -v.y;
+            oy[i] = v.x;
+        }, nfft);
+        if (live && t == 0) ox[0] = ox[n + 1] = oy[0] = oy[n + 1] = (T)0;
+    }
+    __syncthreads();
+    const int jfirst = j == 0 ? 0 : j + 1, jlast = j + 2 >= b.ny ? b.nyp - 1 : j + 2;
+    auto inh = [&](int m, int jj, int i) {
+        const int lr = jj - j - 1;
+        return lr >= 0 && lr < (two ? 2 : 1) ? (double)inh0[m * li + lr * nxp + i] : 0.0;
+    };
+    if (nl == 2) xinv_assemble<T, 2>(b, par, &sS, jfirst, jlast, inh);
+    else if (nl == 3) xinv_assemble<T, 3>(b, par, &sS, jfirst, jlast, inh);
+    else xinv_assemble<T, 4>(b, par, &sS, jfirst, jlast, inh);
 }
 
 // ------------------------------------------------------------------ k_xinv_asm

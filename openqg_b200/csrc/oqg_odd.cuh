@@ -110,11 +110,11 @@ __device__ __forceinline__ void odd_last(int M, int L, int k, const typename C2<
 
 // The compile-time transform, in place.  z: this transform's buffer with the
 // row pair staged (value i at zpad<4>(i), i = 0 .. N, zero at 0 and N) and a
-// barrier taken since; t: thread of the transform (odd_tt(M) threads); every
-// thread of the CTA calls it.
+// barrier taken since; t: thread of the transform (odd_tt(M) threads); the nbar
+// threads that synchronise on barrier 1 (0: the CTA's) call it.
 template <class T, int M, class Out>
 __device__ __forceinline__ void odd_fft_ct(typename C2<T>::t *z, const typename C2<T>::t *__restrict__ tw, int t,
-                                           bool live, Out out) {
+                                           bool live, Out out, int nbar) {
     typedef typename C2<T>::t T2;
     constexpr int L = M / 16, B = 9, TT = odd_tt(M), SH = odd_sh(M), RA = odd_ra(L), RB = L / RA, NA = L / RA;
     static_assert(RA % 2 == 0, "the first radix splits the extension in halves");
@@ -136,7 +136,7 @@ __device__ __forceinline__ void odd_fft_ct(typename C2<T>::t *z, const typename 
                 }
             }
         }
-        __syncthreads();
+        bar_sync(1, nbar);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int bf = t + u * TT;
@@ -147,7 +147,7 @@ __device__ __forceinline__ void odd_fft_ct(typename C2<T>::t *z, const typename 
                 for (int q = 0; q < RA; ++q) z[zstep<SH, 1>(r * L + j * RA, q)] = v[u][q];
             }
         }
-        __syncthreads();
+        bar_sync(1, nbar);
     }
     if constexpr (RB > 1) {
         constexpr int NB1 = L / RB, NB = B * NB1, U = (NB + TT - 1) / TT;
@@ -166,7 +166,7 @@ __device__ __forceinline__ void odd_fft_ct(typename C2<T>::t *z, const typename 
                 }
             }
         }
-        __syncthreads();
+        bar_sync(1, nbar);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int bf = t + u * TT;
@@ -177,7 +177,7 @@ __device__ __forceinline__ void odd_fft_ct(typename C2<T>::t *z, const typename 
                 for (int q = 0; q < RB; ++q) z[zstep<SH, RA>(r * L + j, q)] = v[u][q];
             }
         }
-        __syncthreads();
+        bar_sync(1, nbar);
     }
     static_assert(TT >= L / 2 + 1, "one last butterfly per thread");
     if (live && t <= L / 2)
@@ -230,7 +230,8 @@ __device__ __forceinline__ void odd_mid_rt(const typename C2<T>::t *src, typenam
 }
 template <class T, class Out>
 __device__ __forceinline__ void odd_fft_rt(typename C2<T>::t *a, int M, const int *rad, int nrad,
-                                           const typename C2<T>::t *__restrict__ tw, int t, int TT, bool live, Out out) {
+                                           const typename C2<T>::t *__restrict__ tw, int t, int TT, bool live, Out out,
+                                           int nbar) {
     typedef typename C2<T>::t T2;
     const int R0 = odd_r0(M), L = M / R0;
     T2 *src = a, *dst = a + odd_buf_len(M);
@@ -261,7 +262,7 @@ __device__ __forceinline__ void odd_fft_rt(typename C2<T>::t *a, int M, const in
                 }
             }
         }
-        __syncthreads();
+        bar_sync(1, nbar);
         T2 *x = src; src = dst; dst = x;
         Ns *= R;
     }
@@ -278,14 +279,15 @@ __device__ __forceinline__ void odd_fft_rt(typename C2<T>::t *a, int M, const in
 
 // MC > 0: an instance of that one length; MC = 0: the compile-time plans
 // chosen by the member's length (ensembles); MC < 0: any other length.
-#define OQG_ODD_CASE(MM) case MM: odd_fft_ct<T, MM>(z, tw, t, live, out); return;
+#define OQG_ODD_CASE(MM) case MM: odd_fft_ct<T, MM>(z, tw, t, live, out, nbar); return;
 template <class T, int MC, class Out>
 __device__ __forceinline__ void odd_fft(typename C2<T>::t *z, int M, const int *rad, int nrad,
-                                        const typename C2<T>::t *__restrict__ tw, int t, int TT, bool live, Out out) {
+                                        const typename C2<T>::t *__restrict__ tw, int t, int TT, bool live, Out out,
+                                        int nbar = 0) {
     if constexpr (MC > 0) {
-        odd_fft_ct<T, MC>(z, tw, t, live, out);
+        odd_fft_ct<T, MC>(z, tw, t, live, out, nbar);
     } else if constexpr (MC < 0) {
-        odd_fft_rt<T>(z, M, rad, nrad, tw, t, TT, live, out);
+        odd_fft_rt<T>(z, M, rad, nrad, tw, t, TT, live, out, nbar);
     } else {
         switch (M) {
             OQG_ODD_CASE(128)
@@ -296,7 +298,7 @@ __device__ __forceinline__ void odd_fft(typename C2<T>::t *z, int M, const int *
             OQG_ODD_CASE(1024)
             OQG_ODD_CASE(2048)
             OQG_ODD_CASE(4096)
-            default: odd_fft_rt<T>(z, M, rad, nrad, tw, t, TT, live, out);
+            default: odd_fft_rt<T>(z, M, rad, nrad, tw, t, TT, live, out, nbar);
         }
     }
 }
