@@ -296,6 +296,13 @@ static void (*xinv_kernel(bool cyclic, int M))(const BasinDev *, const Work *, i
     return k_xinv<T, true, 0>;
 }
 
+// The one-pass assembly's instance: four points per thread in FP32 storage.
+template <class T, int NL>
+static void (*asm_kernel())(const BasinDev *, const Work *, int) {
+    if constexpr (sizeof(T) == 4) return k_xinv_asm4<T, NL>;
+    else return k_xinv_asm<T, NL>;
+}
+
 // The inverse transforms and the one-pass k_xinv_asm as two launches (on), or
 // k_xinv for both.
 static void apply_xinv_sep(oqg_handle *h, bool on) {
@@ -313,7 +320,7 @@ static void launch_step_t(oqg_handle *h, int par, double tdt) {
     launch_ysolve<T>(b.cyclic, h->yg, h->st, h->d_bas, h->d_wy, true);
     if (b.xinv_sep) {
         launch_inv<T, E>(x, 1, par, tdt, nullptr);
-        launch_pdl(k_xinv_asm<T, NL>, h->na, 256, 0, h->st, h->d_bas, (const Work *)h->d_wa, par);
+        launch_pdl(asm_kernel<T, NL>(), h->na, 256, 0, h->st, h->d_bas, (const Work *)h->d_wa, par);
     } else {
         launch_pdl(xinv_kernel<T>(b.cyclic, b.M), h->ni, h->xi_threads, h->smem_i, h->st, h->d_bas, h->d_wi, par, tdt);
     }
@@ -682,7 +689,7 @@ static void launch_phase_t(oqg_handle *h, int phase, int par, double tdt) {
             else
                 xinv_kernel<T>(b.cyclic, b.M)<<<h->ni, h->xi_threads, h->smem_i, h->st>>>(h->d_bas, h->d_wi, par, tdt);
             break;
-        default: k_xinv_asm<T, NL><<<h->na, 256, 0, h->st>>>(h->d_bas, h->d_wa, par); break;
+        default: asm_kernel<T, NL>()<<<h->na, 256, 0, h->st>>>(h->d_bas, h->d_wa, par); break;
     }
 }
 static void launch_phase(oqg_handle *h, int phase, int par, double tdt) {
@@ -743,7 +750,7 @@ static void launch_ens_step_t(oqg_ensemble *e, int par) {
     launch_fwd<T, E>(x);
     launch_ysolve<T>(e->cyclic, e->yg, e->st, e->d_bas, e->d_wy, true);
     launch_inv<T, E>(x, (int)e->m.size(), par, 0.0, nullptr);    // one scalar CTA per member
-    launch_pdl(k_xinv_asm<T, NL>, e->na, 256, 0, e->st, e->d_bas, (const Work *)e->d_wa, par);
+    launch_pdl(asm_kernel<T, NL>(), e->na, 256, 0, e->st, e->d_bas, (const Work *)e->d_wa, par);
 }
 template <class T, int NL, int E>
 static void raise_ens_smem_t(oqg_ensemble *e) {
@@ -1063,9 +1070,10 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     h->xinv_split_needed = !xinv_fits(b.M, b.nl, b.ny, b.nxp);
     h->xi_threads = xinv_threads(b.M, b.cyclic, b.nl) + 32;
     h->smem_i = h->xinv_split_needed ? 0 : xinv_bytes(b.M, b.cyclic, b.nl, b.nxp, (int)h->esz);
-    // one point per thread, at most 8 work items of 256 threads per SM (the
-    // items stride over larger grids)
-    b.asm_items = std::min((b.nxp * b.nyp + 255) / 256, 148 * 8);
+    // at most 8 work items of 256 threads per SM (the items stride over larger
+    // grids)
+    const int avec = h->mixed ? XASM_V : 1;
+    b.asm_items = std::min(((b.nxp + avec - 1) / avec * b.nyp + 255) / 256, 148 * 8);
     h->na = b.asm_items;
     // boxes: the inverse transforms run as a launch of their own, shaped like
     // the forward one, then a one-pass assembly (oqg_set_xinv_sep; the only

@@ -138,6 +138,37 @@ __device__ __forceinline__ CSum csum_block_pair(CSum v, double *red) {
     return r;
 }
 __device__ __forceinline__ double csum_block(CSum v, double *red) { return csum_block_pair(v, red).value(); }
+// K of these reductions at once, each in csum_block_pair's order: the K chains
+// of shuffles and additions overlap and two barriers serve them all.  The
+// totals are valid in thread 0.
+template <int K> __device__ __forceinline__ void csum_block_n(CSum (&v)[K], double (&total)[K]) {
+    __shared__ double rs[K][32], rc[K][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    auto warp = [&](CSum (&x)[K]) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < K; ++q) {
+                const double os = __shfl_down_sync(0xffffffffu, x[q].s, o), oc = __shfl_down_sync(0xffffffffu, x[q].c, o);
+                x[q].merge(os, oc);
+            }
+    };
+    warp(v);
+    __syncthreads();
+    if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < K; ++q) { rs[q][wid] = v[q].s; rc[q][wid] = v[q].c; }
+    __syncthreads();
+    if (wid == 0) {
+        CSum t[K];
+#pragma unroll
+        for (int q = 0; q < K; ++q)
+            if (lane < nw) { t[q].s = rs[q][lane]; t[q].c = rc[q][lane]; }
+        warp(t);
+#pragma unroll
+        for (int q = 0; q < K; ++q) total[q] = t[q].value();
+    }
+}
 
 // ------------------------------------------------------------------ k_vort
 #define VTX 60          // output columns of a vorticity tile
@@ -1580,10 +1611,12 @@ k_xinv(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
 // point from the modal rows in b.inh_g, ocqbdy (vorsubs.F90:58-114) on the
 // walls and the suppress_comp_mode averages (driver.F90:174-189), with the
 // step's scalars from b.scal_g.  The work items of a basin (the work list
-// spans an ensemble's members) take interleaved runs of 256 points, one
-// point per thread in each; a wall point also
-// forms the layer values of its inner neighbour (the same arithmetic as the
-// neighbour's own thread), so no point waits for another.
+// spans an ensemble's members) take interleaved runs of 256 vectors of a row's
+// points, one per thread; a wall point also forms the layer values of its
+// inner neighbour (the same arithmetic as the neighbour's own thread), so no
+// point waits for another.  Bound by the loads in flight: with one FP32 point
+// per thread 24 warps kept 15 KB in flight on an SM, and a 2049^2 launch of
+// FP32 storage ran at 2.3 TB/s (58.6 us; 40.8 with four).
 // hc: the box's alpha (nl-1), or the channel's c_bt, c_bc1[1..], c_bc2[1..]
 // (homog.F90:280-366, by k_xinv_rows' scalar CTA).
 template <class T, int NL>
@@ -1695,6 +1728,161 @@ k_xinv_asm(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int 
                 for (int c = 0; c < cnt; ++c) qv = qv + dd;
             }
             Qc[k * ms + o2] = supp ? (T)((T)0.5 * (qv + Qm[k * ms + o2])) : qv;
+        }
+    }
+}
+
+// The same with four points of a row per thread, for FP32 storage.  (In FP64 two
+// points per thread took 62 us against 75 at 2049^2 but left the whole step as
+// it was, 529 us, and cost the smaller grids their threads, 257^2 29.3 -> 31.9.)
+#define XASM_V 4
+template <class T> struct alignas(sizeof(T) * XASM_V) XasmVec { T v[XASM_V]; };
+template <class T, int NL>
+__global__ void __launch_bounds__(256, 3)
+k_xinv_asm4(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par) {
+    constexpr int V = XASM_V;
+    typedef XasmVec<T> Vec;
+    const Work w = work[blockIdx.x];
+    const BasinDev &b = bas[w.member];
+    __shared__ double sCtm[NL * NL], sAmat[NL * NL], sHc[2 * NL];
+    __shared__ int sSupp;
+    pdl_trigger();
+    // the basin's constant tables before the wait for the previous launch
+    if (threadIdx.x < NL * NL) {
+        sCtm[threadIdx.x] = b.ctm2l[threadIdx.x];
+        sAmat[threadIdx.x] = b.amat[threadIdx.x];
+    }
+    const int nxp = b.nxp, nyp = b.nyp, px = b.px;
+    const bool cyc = b.cyclic != 0;
+    const size_t ms = (size_t)nyp * px;
+    const T *__restrict__ inh = (const T *)b.inh_g;
+    const T *__restrict__ H = (const T *)b.hsb;
+    const T *__restrict__ Pold = (const T *)b.F[par];
+    T *__restrict__ Pnew = (T *)b.F[1 - par];
+    T *__restrict__ Qc = (T *)b.F[3 - par];          // q after this step
+    const T *__restrict__ Qm = (const T *)b.F[2 + par];
+    const T fac = (T)b.qb_fac;
+    const int rv = (nxp + V - 1) / V;                // vectors of a row
+    const FastDiv fdx(rv);
+    const int nvec = rv * nyp;
+    pdl_wait();
+    const XinvScal *sc = (const XinvScal *)b.scal_g;
+    if (!cyc) {
+        if (threadIdx.x < NL - 1) sHc[threadIdx.x] = sc->alpha[threadIdx.x];
+    } else if (threadIdx.x < 2 * NL) {
+        // c_bt, c_bc1[1..NL), then c_bc2 at NL + m
+        const int x = threadIdx.x;
+        sHc[x] = x == 0 ? sc->c_bt : (x < NL ? sc->c_bc1[x] : (x == NL ? 0.0 : sc->c_bc2[x - NL]));
+    }
+    if (threadIdx.x == 0) sSupp = sc->supp;
+    __syncthreads();
+    double ctm[NL * NL], hc[2 * NL];
+#pragma unroll
+    for (int x = 0; x < NL * NL; ++x) ctm[x] = sCtm[x];
+#pragma unroll
+    for (int m = 0; m < 2 * NL; ++m) hc[m] = sHc[m];
+    const bool supp = sSupp != 0;
+    // ocqbdy and the suppression average of q at a wall point with layer
+    // values pn: its inner neighbour across the meridional wall (a corner takes
+    // that one), else across the zonal wall
+    auto wall = [&](int j, int i, const T *pn) {
+        const bool zon = (j == 0 || j == nyp - 1), mer = !cyc && (i == 0 || i == nxp - 1);
+        const size_t o2 = (size_t)j * px + i;
+        const int jn = mer ? j : (j == 0 ? 1 : nyp - 2);
+        const size_t on = mer ? (size_t)j * px + (i == 0 ? 1 : nxp - 2) : (size_t)jn * px + i;
+        T pnb[NL];
+        xinv_layers<T, NL>(b, inh, H, ctm, hc, on, jn, pnb);
+        const int cnt = (zon ? 1 : 0) + (mer ? 1 : 0);
+        const T by = (T)(b.beta * b.yprel[j]);
+#pragma unroll
+        for (int k = 0; k < NL; ++k) {
+            T qv = fac * (pnb[k] - pn[k]);
+            double mv = 0.0;
+#pragma unroll
+            for (int l = 0; l < NL; ++l) mv += sAmat[k + NL * l] * (double)pn[l];
+            const T fmv = (T)(b.fnot * mv);
+            for (int c = 0; c < cnt; ++c) qv = qv - fmv;
+            // (FP32 storage holds q - beta y: one beta y fewer)
+            for (int c = q_anom_stored<T>() ? 1 : 0; c < cnt; ++c) qv = qv + by;
+            if (k == b.kt && b.topo_active) {
+                const T dd = (T)b.ddyn[o2];
+                for (int c = 0; c < cnt; ++c) qv = qv + dd;
+            }
+            Qc[k * ms + o2] = supp ? (T)((T)0.5 * (qv + Qm[k * ms + o2])) : qv;
+        }
+    };
+    // the basin's b.asm_items work items interleave: item w.block takes the
+    // vectors w.block * 256 + t, then every b.asm_items * 256 further
+    const int stride = b.asm_items * 256;
+    for (int idx = w.block * 256 + threadIdx.x; idx < nvec; idx += stride) {
+        const int j = fdx.div(idx), i0 = (idx - j * rv) * V;
+        const size_t o2 = (size_t)j * px + i0;
+        Vec x[NL], h[NL];
+#pragma unroll
+        for (int m = 0; m < NL; ++m) {
+            x[m] = *(const Vec *)(inh + m * ms + o2);
+            if (!cyc && m) h[m] = *(const Vec *)(H + (m - 1) * ms + o2);
+        }
+        double hr[NL];                               // a channel's corrections of the row
+        if (cyc) {
+            hr[0] = hc[0] * b.hbt[j];
+#pragma unroll
+            for (int m = 1; m < NL; ++m) hr[m] = hc[m] * b.hbc1[m * nyp + j] + hc[NL + m] * b.hbc2[m * nyp + j];
+        }
+        Vec pn[NL];
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+            double pm_[NL];
+#pragma unroll
+            for (int m = 0; m < NL; ++m) {
+                pm_[m] = (double)x[m].v[e];
+                if (cyc) pm_[m] = pm_[m] + hr[m];
+                else if (m) pm_[m] = pm_[m] + hc[m - 1] * (double)h[m].v[e];
+            }
+#pragma unroll
+            for (int k = 0; k < NL; ++k) {
+                double s2 = 0.0;
+#pragma unroll
+                for (int m = 0; m < NL; ++m) s2 += pm_[m] * ctm[m + NL * k];
+                pn[k].v[e] = (T)s2;
+            }
+        }
+        const bool whole = i0 + V <= nxp;
+#pragma unroll
+        for (int k = 0; k < NL; ++k) {
+            Vec r = pn[k];
+            if (supp) {
+                const Vec old = *(const Vec *)(Pold + k * ms + o2);
+#pragma unroll
+                for (int e = 0; e < V; ++e) r.v[e] = (T)0.5 * (r.v[e] + old.v[e]);
+            }
+            if (whole) *(Vec *)(Pnew + k * ms + o2) = r;
+            else
+#pragma unroll
+                for (int e = 0; e < V; ++e)
+                    if (i0 + e < nxp) Pnew[k * ms + o2 + e] = r.v[e];
+        }
+        const bool zon = (j == 0 || j == nyp - 1);
+        if (!supp && !zon && (cyc || (i0 > 0 && i0 + V < nxp))) continue;
+#pragma unroll 1
+        for (int e = 0; e < V && i0 + e < nxp; ++e) {
+            const int i = i0 + e;
+            if (zon || (!cyc && (i == 0 || i == nxp - 1))) {
+                T q[NL];
+#pragma unroll
+                for (int k = 0; k < NL; ++k) {
+                    q[k] = pn[k].v[0];
+#pragma unroll
+                    for (int f = 1; f < V; ++f)
+                        if (f == e) q[k] = pn[k].v[f];
+                }
+                wall(j, i, q);
+            } else if (supp) {
+                for (int k = 0; k < NL; ++k) {
+                    const size_t o3 = k * ms + o2 + e;
+                    Qc[o3] = (T)0.5 * (Qc[o3] + Qm[o3]);
+                }
+            }
         }
     }
 }
@@ -1814,10 +2002,20 @@ __device__ __forceinline__ double trap_x(const BasinDev &b, int i) {
 // int_P_dA (numerics.F90:165-204), compensated; red: >= 64 doubles.
 template <class T>
 __device__ double area_integral(const BasinDev &b, const T *f, double *red) {
+    // eight loads in flight per thread (one at a time, a 257^2 field took 39 us)
+    constexpr int U = 8;
+    const FastDiv fd(b.nxp);
+    const int n = b.nyp * b.nxp;
     CSum s;
-    for (int idx = threadIdx.x; idx < b.nyp * b.nxp; idx += blockDim.x) {
-        int j = idx / b.nxp, i = idx - j * b.nxp;
-        s.add(trap_w(b, i, j) * (double)f[(size_t)j * b.px + i]);
+    for (int x0 = threadIdx.x; x0 < n; x0 += U * blockDim.x) {
+        double v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int idx = x0 + u * blockDim.x, j = fd.div(idx < n ? idx : 0), i = idx - j * b.nxp;
+            v[u] = idx < n ? trap_w(b, i, j) * (double)f[(size_t)j * b.px + i] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) s.add(v[u]);
     }
     return csum_block(s, red) * b.dx * b.dy;
 }
@@ -1971,9 +2169,10 @@ __device__ void forcing_integrals_cta(const BasinDev &b, const T *E, double *red
             }
         }
     }
-    double v[5];
-#pragma unroll
-    for (int q = 0; q < 5; ++q) v[q] = csum_block(cv[q], red);
+    // (the five reductions one after the other were 5 of the 13 us of a
+    // channel's k_aml_post, whose last CTA ends with them)
+    double v[5] = {};
+    csum_block_n<5>(cv, v);
     const double exn = v[0] * b.dx * b.dy;
     const double s1 = v[1] * b.dx, n1 = v[2] * b.dx, s2 = v[3] * b.dx, n2v = v[4] * b.dx;
     if (threadIdx.x != 0) return;
