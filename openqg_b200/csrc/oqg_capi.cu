@@ -267,20 +267,35 @@ static XGeo xgeo(oqg_handle *h, bool fp64, bool pdl) {
                 fp64 ? h->d_bas64 : h->d_bas, h->d_wx, pdl};
 }
 
-// The vorticity kernel instance of a tile height and its threads.  wide: no
-// more CTAs than SMs at the least height (us per step: 129^2 25.1 -> 22.5,
-// 193 x 97 channel 29.9 -> 26.7).
+// The vorticity kernel's form.  Grids with few tiles (of the least height) give
+// a tile to a cluster of one CTA per layer, as long as all are resident at once
+// (two CTAs per SM), or, past that, to one CTA of twice the threads, as long as
+// every SM has at most one.  us per step, plain / double / cluster: 65^2 21.3 /
+// 20.2 / 19.0, 129^2 25.1 / 22.5 / 22.3 (three such basins at once 9.65 / 9.02 /
+// 8.58), 193 x 97 channel 29.9 / 26.7 / 24.6.
 typedef void (*VortFn)(const BasinDev *, const Work *, int, double);
+enum VortForm { VORT_PLAIN, VORT_WIDE, VORT_SPLIT };
 template <class T, int NL>
-static VortFn vort_kernel(int vt, bool wide) {
+static VortFn vort_kernel(int vt, VortForm f) {
     switch (vt) {
-        case 8: return wide ? k_vort<T, NL, 8, VWIDE> : k_vort<T, NL, 8, VSTRIPS>;
-        case 12: return k_vort<T, NL, 12, VSTRIPS>;
-        default: return k_vort<T, NL, 16, VSTRIPS>;
+        case 8:
+            return f == VORT_SPLIT ? k_vort<T, NL, 8, VSTRIPS, true>
+                 : f == VORT_WIDE ? k_vort<T, NL, 8, VWIDE, false> : k_vort<T, NL, 8, VSTRIPS, false>;
+        case 12: return k_vort<T, NL, 12, VSTRIPS, false>;
+        default: return k_vort<T, NL, 16, VSTRIPS, false>;
     }
 }
-static bool vort_wide(int vt, int ctas) { return vt == 8 && ctas <= 148; }
-static int vort_threads(int vt, bool wide) { return 64 * (vt == 8 && wide ? VWIDE : VSTRIPS); }
+struct VortGeo {
+    VortForm form;
+    int grid, block, cluster;
+};
+// A single basin's launch; ctas: its strips and tiles.
+static VortGeo vort_geo(const BasinDev &b, int ctas) {
+    const int strips = vort_strips(b.nl, b.cyclic), split = strips + (ctas - strips) * b.nl;
+    if (b.vty == 8 && split <= 2 * 148) return VortGeo{VORT_SPLIT, split, 64 * VSTRIPS, b.nl};
+    if (b.vty == 8 && ctas <= 148) return VortGeo{VORT_WIDE, ctas, 64 * VWIDE, 1};
+    return VortGeo{VORT_PLAIN, ctas, 64 * VSTRIPS, 1};
+}
 
 // The one-kernel inverse's instance: a channel's length (FP64), or any.
 template <class T>
@@ -310,12 +325,37 @@ static void apply_xinv_sep(oqg_handle *h, bool on) {
     h->hb64.xinv_sep = h->hb.xinv_sep;
 }
 
+template <class T, int NL>
+static void launch_vort(oqg_handle *h, int par, double tdt, bool pdl) {
+    const VortGeo g = vort_geo(h->hb, h->nv);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(g.grid);
+    cfg.blockDim = dim3(g.block);
+    cfg.dynamicSmemBytes = h->smem_v;
+    cfg.stream = h->st;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (g.cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = g.cluster;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    cudaLaunchKernelEx(&cfg, vort_kernel<T, NL>(h->hb.vty, g.form), (const BasinDev *)h->d_bas, (const Work *)h->d_wv, par,
+                       tdt);
+}
+
 template <class T, int NL, int E>
 static void launch_step_t(oqg_handle *h, int par, double tdt) {
     const BasinDev &b = h->hb;
     const XGeo x = xgeo(h, false, true);
-    const bool vw = vort_wide(b.vty, h->nv);
-    launch_pdl(vort_kernel<T, NL>(b.vty, vw), h->nv, vort_threads(b.vty, vw), h->smem_v, h->st, h->d_bas, h->d_wv, par, tdt);
+    launch_vort<T, NL>(h, par, tdt, true);
     launch_fwd<T, E>(x);
     launch_ysolve<T>(b.cyclic, h->yg, h->st, h->d_bas, h->d_wy, true);
     if (b.xinv_sep) {
@@ -371,8 +411,9 @@ static void raise_x_smem(bool cyclic, int M, size_t x) {
 }
 template <class T, int NL, int E>
 static void raise_step_smem(bool cyclic, int M, size_t v, size_t x, size_t i) {
-    for (int vt : {8, 12, 16}) raise_smem((const void *)vort_kernel<T, NL>(vt, false), v);
-    raise_smem((const void *)vort_kernel<T, NL>(8, true), v);
+    for (int vt : {8, 12, 16}) raise_smem((const void *)vort_kernel<T, NL>(vt, VORT_PLAIN), v);
+    raise_smem((const void *)vort_kernel<T, NL>(8, VORT_WIDE), v);
+    raise_smem((const void *)vort_kernel<T, NL>(8, VORT_SPLIT), v);
     raise_x_smem<T, E>(cyclic, M, x);
     if (i) raise_smem((const void *)xinv_kernel<T>(cyclic, M), i);
 }
@@ -677,11 +718,7 @@ template <class T, int NL, int E>
 static void launch_phase_t(oqg_handle *h, int phase, int par, double tdt) {
     const BasinDev &b = h->hb;
     switch (phase) {
-        case 0: {
-            const bool vw = vort_wide(b.vty, h->nv);
-            vort_kernel<T, NL>(b.vty, vw)<<<h->nv, vort_threads(b.vty, vw), h->smem_v, h->st>>>(h->d_bas, h->d_wv, par, tdt);
-            break;
-        }
+        case 0: launch_vort<T, NL>(h, par, tdt, false); break;
         case 1: launch_fwd<T, E>(xgeo(h, false, false)); break;
         case 2: launch_ysolve<T>(b.cyclic, h->yg, h->st, h->d_bas, h->d_wy, false); break;
         case 3:
@@ -743,7 +780,7 @@ struct oqg_ensemble {
 // descriptor (tdt = 0).
 template <class T, int NL, int E>
 static void launch_ens_step_t(oqg_ensemble *e, int par) {
-    launch_pdl(vort_kernel<T, NL>(e->hb[0].vty, false), e->nv, vort_threads(e->hb[0].vty, false), e->smem_v, e->st, e->d_bas, e->d_wv, par, 0.0);
+    launch_pdl(vort_kernel<T, NL>(e->hb[0].vty, VORT_PLAIN), e->nv, 64 * VSTRIPS, e->smem_v, e->st, e->d_bas, e->d_wv, par, 0.0);
     // members of one transform length take that length's instance; each
     // member's transforms per CTA follow from the CTA's threads (G = 0)
     const XGeo x{e->cyclic != 0, e->Mu, e->nx, e->xthreads, 0, e->smem_x, e->st, e->d_bas, e->d_wx, true};
@@ -1706,7 +1743,8 @@ __global__ void k_chain_empty() {
 int oqg_launch_floor(oqg_handle *h, int nsteps, double *us_per_step) {
     if (!h || !us_per_step || nsteps < 1) return fail(OQG_EINVAL, "bad argument");
     struct Shape { int grid, block; size_t smem; };
-    std::vector<Shape> sh = {{h->nv, vort_threads(h->hb.vty, vort_wide(h->hb.vty, h->nv)), h->smem_v}, {h->nx, h->xthreads, h->smem_x},
+    const VortGeo vg = vort_geo(h->hb, h->nv);
+    std::vector<Shape> sh = {{vg.grid, vg.block, h->smem_v}, {h->nx, h->xthreads, h->smem_x},
                              {h->yg.grid, h->yg.block, 0}};
     if (h->hb.xinv_sep) {
         sh.push_back({h->nx + 1, rup(h->xthreads, 32), h->smem_x});

@@ -170,6 +170,18 @@ template <int K> __device__ __forceinline__ void csum_block_n(CSum (&v)[K], doub
     }
 }
 
+// Barrier of the CTAs of a cluster (release and acquire), and a value of CTA
+// rank's shared memory at the place of this CTA's p.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ double ld_cluster(const double *p, int rank) {
+    double v;
+    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f64 %0, [a];\n\t}\n"
+                 : "=d"(v) : "r"(smem_u32(p)), "r"(rank) : "memory");
+    return v;
+}
+
 // ------------------------------------------------------------------ k_vort
 #define VTX 60          // output columns of a vorticity tile
 #define VTYMAX 17       // output rows of a vorticity tile (at most)
@@ -376,7 +388,11 @@ __device__ __forceinline__ void vort_strip(const BasinDev &b, int side, int k, i
 // NS row strips of 64 threads: VSTRIPS, or VWIDE where the tiles are no more
 // than the SMs, so that a CTA has its SM to itself: the rows a thread marches
 // in each phase halve.
-template <class T, int NL, int VT, int NS>
+// SPLIT: a tile is shared by a cluster of NL CTAs, one per layer; they exchange
+// the stepped q through distributed shared memory, and CTA m forms mode m's
+// right-hand side.  For single basins with few tiles, where the time is one
+// CTA's chain of NL layers.
+template <class T, int NL, int VT, int NS, bool SPLIT>
 __global__ void __launch_bounds__(64 * NS, NS == VSTRIPS ? 2 : 1)
 k_vort(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par, double tdt) {
     static_assert(VT % NS == 0 && VT >= 8 && VT <= VTYMAX, "tile rows: a multiple of the strips in [8, VTYMAX]");
@@ -385,10 +401,13 @@ k_vort(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
     // rows per strip of each phase; the last strips of d2 and d4 start early
     // and recompute a row or two of their neighbours (the same values)
     constexpr int RMAX = VT / NS, R2MAX = (H2 + NS - 1) / NS, R1MAX = (H1 + NS - 1) / NS;
-    const Work w = work[blockIdx.x];
+    Work w;
+    if constexpr (SPLIT) w = Work{0, (int)blockIdx.x};
+    else w = work[blockIdx.x];
     const BasinDev &b = bas[w.member];
     const int strips = vort_strips(NL, b.cyclic);
     if (w.block < strips) {
+        // (a whole number of clusters: 2 NL)
         pdl_trigger();
         pdl_wait();
         vort_strip<T>(b, w.block / NL, w.block % NL, par);
@@ -416,7 +435,9 @@ k_vort(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
     GeoS<T> g;
     g.nxp = b.nxp; g.nyp = b.nyp; g.cyclic = b.cyclic; g.K = sK;
     const VortLayout LY = vort_layout(VT, (int)sizeof(T));
-    const int tile = w.block - strips, tile_y = tile / b.tiles_x, tile_x = tile - tile_y * b.tiles_x;
+    const int tile = (w.block - strips) / (SPLIT ? NL : 1), tile_y = tile / b.tiles_x, tile_x = tile - tile_y * b.tiles_x;
+    // the layers of this CTA
+    const int kb = SPLIT ? (w.block - strips) % NL : 0, ke = SPLIT ? kb + 1 : NL;
     const int i0 = tile_x * VTX, j0 = tile_y * VT + 1;
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -451,13 +472,13 @@ k_vort(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
     pdl_wait();
 
     auto issue = [&](int k) {
-        T *bf = sm + (k & 1) * LY.nbuf;
+        T *bf = sm + ((k - kb) & 1) * LY.nbuf;
         if (tma) {
             if (threadIdx.x == 0) {
                 fence_proxy_async();
                 unsigned bytes = (unsigned)((HPM * LPQ + 2 * H1 * LPQ + VT * LO) * sizeof(T));
                 if (k == 0) bytes += (unsigned)(VT * LO * sizeof(T));
-                unsigned long long *bar = &bars[k & 1];
+                unsigned long long *bar = &bars[(k - kb) & 1];
                 mbar_expect_tx(bar, bytes);
                 tma_load_3d(bf + LY.pm, tm + (OQG_TMAP_PM + 1 - par) * OQG_TMAP_BYTES, i0 - 4, j0 - 3, k, bar);
                 tma_load_3d(bf + LY.p, tm + (OQG_TMAP_PQ + par) * OQG_TMAP_BYTES, i0 - 4, j0 - 1, k, bar);
@@ -474,7 +495,7 @@ k_vort(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
             cp_async_commit();
         }
     };
-    issue(0);
+    issue(kb);
 
     // strips of rows: [ty*R, ty*R + R) of each region
     constexpr int R2 = R2MAX, R1 = R1MAX, R0 = RMAX;
@@ -492,33 +513,40 @@ k_vort(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
     const bool interior = (j0 - 2 >= 1 && j0 + VT + 1 <= nyp - 2) &&
                           (g.cyclic ? (i0 + VTX <= nxp) : (i0 - 2 >= 1 && i0 + VTX + 1 <= nxp - 2));
 
+    // SPLIT: the stepped q less the planetary and topographic parts, for the
+    // cluster; otherwise summed over the layers in registers
+    __shared__ double sQL[SPLIT ? VT * LO : 1];
+    bool lost = false;
 #pragma unroll 1
-    for (int k = 0; k < NL; ++k) {
-        if (k + 1 < NL) issue(k + 1);
+    for (int k = kb; k < ke; ++k) {
+        if (k + 1 < ke) issue(k + 1);
         if (tma) {
             // one thread polls the barrier; the CTA barrier then publishes
             // the tile to the others without spinning warps taking issue slots
             bool ok = true;
-            if (threadIdx.x == 0) ok = mbar_wait_bounded(&bars[k & 1], (k >> 1) & 1, b.wait_limit);
+            if (threadIdx.x == 0) ok = mbar_wait_bounded(&bars[(k - kb) & 1], ((k - kb) >> 1) & 1, b.wait_limit);
             if (__syncthreads_or(!ok)) {
                 // a tile never arrived: report, drain what is in flight, stop
                 if (threadIdx.x == 0) {
                     atomicOr(b.err, OQG_DERR_TIMEOUT);
-                    mbar_wait_bounded(&bars[k & 1], (k >> 1) & 1, OQG_WAIT_LIMIT);
-                    if (k + 1 < NL) mbar_wait_bounded(&bars[(k + 1) & 1], ((k + 1) >> 1) & 1, OQG_WAIT_LIMIT);
+                    mbar_wait_bounded(&bars[(k - kb) & 1], ((k - kb) >> 1) & 1, OQG_WAIT_LIMIT);
+                    if (k + 1 < ke) mbar_wait_bounded(&bars[(k + 1 - kb) & 1], ((k + 1 - kb) >> 1) & 1, OQG_WAIT_LIMIT);
                 }
                 __syncthreads();
-                return;
+                // (a cluster's other CTAs wait at its barriers below)
+                if constexpr (!SPLIT) return;
+                lost = true;
+                break;
             }
         } else {
-            if (k + 1 < NL) cp_async_wait<1>();
+            if (k + 1 < ke) cp_async_wait<1>();
             else cp_async_wait<0>();
             __syncthreads();
         }
-        const T *sPM = sm + (k & 1) * LY.nbuf + LY.pm;
-        const T *sP = sm + (k & 1) * LY.nbuf + LY.p;
-        const T *sQ = sm + (k & 1) * LY.nbuf + LY.q;
-        const T *sQM = sm + (k & 1) * LY.nbuf + LY.qm;
+        const T *sPM = sm + ((k - kb) & 1) * LY.nbuf + LY.pm;
+        const T *sP = sm + ((k - kb) & 1) * LY.nbuf + LY.p;
+        const T *sQ = sm + ((k - kb) & 1) * LY.nbuf + LY.q;
+        const T *sQM = sm + ((k - kb) & 1) * LY.nbuf + LY.qm;
         // The layer's stencils; I: every point of the tile and its halo is
         // off the walls, so the wall rules and range tests drop out.
         auto layer = [&](auto inner) {
@@ -645,8 +673,10 @@ k_vort(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
                             // modal right-hand side, FP64 (p_modes_rhs)
                             double ql = QA ? (double)qn : (double)qn - sBY[r];
                             if (k == kt && topo) ql -= DD[o2];
+                            if constexpr (SPLIT) sQL[r * LO + tx] = ql;
+                            else
     #pragma unroll
-                            for (int m = 0; m < NL; ++m) acc[u][m] += ql * sCtl[k + NL * m];
+                                for (int m = 0; m < NL; ++m) acc[u][m] += ql * sCtl[k + NL * m];
                         }
                         d4s = d4c;
                         d4c = d4n;
@@ -663,6 +693,27 @@ k_vort(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
     T *RHS = (T *)b.rhs;
     const int ioff = g.cyclic ? 0 : 1;
     const double f0 = b.fnot;
+    if constexpr (SPLIT) {
+        cluster_sync();
+        if (tx < VTX && !lost) {
+            double v[RMAX][NL];
+#pragma unroll
+            for (int l = 0; l < NL; ++l)
+#pragma unroll
+                for (int u = 0; u < RMAX; ++u) v[u][l] = ld_cluster(&sQL[(r0 + u) * LO + tx], l);
+#pragma unroll
+            for (int u = 0; u < RMAX; ++u) {
+                const int r = r0 + u, gj = j0 + r, xi = i0 + tx - ioff;
+                if (gj < 1 || gj > nyp - 2 || xi < 0 || xi >= b.nxin) continue;
+                double s = 0.0;
+#pragma unroll
+                for (int l = 0; l < NL; ++l) s += v[u][l] * sCtl[l + NL * kb];
+                RHS[((size_t)kb * b.ny + (gj - 1)) * b.pr + xi] = (T)(f0 * s);
+            }
+        }
+        cluster_sync();               // no CTA leaves while its tile may be read
+        return;
+    }
     if (tx < VTX) {
 #pragma unroll
         for (int u = 0; u < RMAX; ++u) {
