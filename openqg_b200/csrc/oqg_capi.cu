@@ -171,18 +171,36 @@ static bool ysolve_fits(int ny, int W, int vsz) {
     return (size_t)std::max((ny + 32) | 1, (L * (s + 1) + 1) | 1) * 4 * vsz <= 227 * 1024;
 }
 
+// The fewest radices of odd_fft_rt whose product is L, of those the least sum.
+static void odd_split(int L, std::vector<int> &cur, std::vector<int> &best) {
+    if (L == 1) {
+        auto sum = [](const std::vector<int> &v) { int s = 0; for (int x : v) s += x; return s; };
+        if (best.empty() || cur.size() < best.size() || (cur.size() == best.size() && sum(cur) < sum(best))) best = cur;
+        return;
+    }
+    if (!best.empty() && cur.size() + 1 > best.size()) return;
+#define OQG_ODD_S(RR)                                                                    \
+    if (L % RR == 0 && (cur.empty() || RR <= cur.back())) {                              \
+        cur.push_back(RR);                                                               \
+        odd_split(L / RR, cur, best);                                                    \
+        cur.pop_back();                                                                  \
+    }
+    OQG_ODD_RADICES(OQG_ODD_S)
+#undef OQG_ODD_S
+}
 // The stages of a box transform of length M (oqg_odd.cuh): the radices of the
-// L = M / R0 points of a subsequence, then R0.
-static bool odd_radices(int M, std::vector<int> &rad) {
+// L = M / R0 points of a subsequence, then R0.  M factors into 2, 3 and 5.
+static void odd_radices(int M, std::vector<int> &rad) {
     const int r0 = odd_r0(M), L = M / r0;
+    rad.clear();
     if (odd_ct_len(M)) {
         rad = {odd_ra(L)};
         if (L > rad[0]) rad.push_back(L / rad[0]);
-    } else if (!fft_radices(L, rad)) {
-        return false;
+    } else if (L > 1) {
+        std::vector<int> cur;
+        odd_split(L, cur, rad);
     }
     rad.push_back(r0);
-    return true;
 }
 
 // The transform kernels' instance for a basin's transform length: one built
@@ -930,7 +948,13 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
         return bail(OQG_EUNSUPPORTED, "x-transform length must factor into 2, 3 and 5");
     if (b.M > 4096) return bail(OQG_EUNSUPPORTED, "x-transform length above 4096");
     b.nrad = (int)rad.size();
-    for (int i = 0; i < b.nrad; ++i) b.rad[i] = rad[i];
+    for (int i = 0, Ns = 1; i < b.nrad; Ns *= rad[i++]) {
+        b.rad[i] = rad[i];
+        b.fd_ns[i] = FastDiv(Ns);
+    }
+    b.fd_nxp = FastDiv(b.nxp);
+    b.fd_nxin = FastDiv(b.nxin);
+    b.fd_nk = FastDiv(b.nk);
     b.pr = rup(b.nxin, 32);
     b.pk = rup(b.nk, 32);
     // vorticity tiles: VTX columns by vty rows, vty chosen so that the tiles
@@ -1024,10 +1048,14 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     double *d_otw64 = nullptr;
     if (!b.cyclic) {
         std::vector<int> orad;
-        if (!odd_radices(b.M, orad) || (int)orad.size() > OQG_MAXRAD)
-            return bail(OQG_EUNSUPPORTED, "x-transform length must factor into 2, 3 and 5");
+        odd_radices(b.M, orad);
         b.norad = (int)orad.size();
         std::copy(orad.begin(), orad.end(), b.orad);
+        const int L = b.M / orad.back();
+        for (int s = 0, Ns = 1; s < b.norad - 1 || s == 0; Ns *= b.orad[s++]) {
+            b.fd_obf[s] = FastDiv(b.norad > 1 ? L / b.orad[s] : L);
+            b.fd_ons[s] = FastDiv(Ns);
+        }
         fft_stage_twiddles(b.M, orad, tw);
         d_otw64 = dalloc<double>(h, tw.size());
         CK(cudaMemcpy(d_otw64, tw.data(), tw.size() * sizeof(double), cudaMemcpyHostToDevice));

@@ -40,6 +40,24 @@ struct DevForcing {
 // Channel strip quantities per wall and layer (vorticity kernel)
 #define OQG_NSTRIP 5
 
+// Division of ints in [0, 2^31) by a divisor d >= 1 fixed for a loop, by a
+// multiply-high and a shift (Granlund and Montgomery's method with a 33-bit
+// multiplier 2^32 + m): q = (umulhi(m, n) + n) >> s, s = ceil(log2 d),
+// m = floor(2^32 (2^s - d) / d) + 1.
+struct FastDiv {
+    unsigned m = 1;
+    int s = 0;
+    FastDiv() = default;
+    __host__ __device__ __forceinline__ explicit FastDiv(int d) {
+        s = 0;
+        while ((1u << s) < (unsigned)d) ++s;
+        m = (unsigned)(((1ull << 32) * ((1ull << s) - (unsigned long long)d)) / (unsigned long long)d + 1ull);
+    }
+    __device__ __forceinline__ int div(int n) const {
+        return (int)((__umulhi(m, (unsigned)n) + (unsigned)n) >> s);
+    }
+};
+
 struct BasinDev {
     // geometry
     int nxp, nyp, nl, cyclic;
@@ -86,6 +104,11 @@ struct BasinDev {
     const void *tw;             // [M] T2 per-stage FFT twiddles (fft_stage_twiddles)
     const void *otw;            // box: [M] T2 twiddles of the pruned plan (oqg_odd.cuh)
     int norad, orad[OQG_MAXRAD];   // its radices, the outer one last
+    // divisions of the transforms' index arithmetic (the magic numbers cost a
+    // 64-bit division, so the host forms them): by a row's points, a row's
+    // transform inputs, a channel's wavenumbers, and per stage of the plans by
+    // the butterflies of a subsequence and by the span
+    FastDiv fd_nxp, fd_nxin, fd_nk, fd_obf[OQG_MAXRAD], fd_ons[OQG_MAXRAD], fd_ns[OQG_MAXRAD];
     // Thomas pivots 1/(b - a gam) of blocks of 8 adjacent wavenumbers of a mode:
     // [piv_len][8] from piv_off, up to the longest column's fixed point
     const double *piv_tab;
@@ -116,24 +139,6 @@ struct BasinDev {
                                 // passes tdt = 0 (ensembles: one per member)
     unsigned wait_limit;        // polls of a first wait for a tile load before
                                 // it reports a timeout (drains use the full limit)
-};
-
-// Division of ints in [0, 2^31) by a divisor d >= 1 fixed for a loop, by a
-// multiply-high and a shift (Granlund and Montgomery's method with a 33-bit
-// multiplier 2^32 + m): q = (umulhi(m, n) + n) >> s, s = ceil(log2 d),
-// m = floor(2^32 (2^s - d) / d) + 1.
-struct FastDiv {
-    unsigned m = 1;
-    int s = 0;
-    FastDiv() = default;
-    __host__ __device__ __forceinline__ explicit FastDiv(int d) {
-        s = 0;
-        while ((1u << s) < (unsigned)d) ++s;
-        m = (unsigned)(((1ull << 32) * ((1ull << s) - (unsigned long long)d)) / (unsigned long long)d + 1ull);
-    }
-    __device__ __forceinline__ int div(int n) const {
-        return (int)((__umulhi(m, (unsigned)n) + (unsigned)n) >> s);
-    }
 };
 
 // One entry of a launch's work list: which basin and which block of it.

@@ -186,6 +186,72 @@ template <class T> struct Dft<T, 16> {
     }
 };
 
+// Composite sizes with coprime factors by the prime-factor algorithm (Good and
+// Thomas: no twiddles): n = R2 n1 + R1 n2, k = k1 mod R1, k2 mod R2.
+__host__ __device__ constexpr int inv_mod(int a, int m) {
+    for (int x = 1; x < m; ++x)
+        if (a * x % m == 1) return x;
+    return 1;
+}
+template <class T, int R1, int R2> struct DftPfa {
+    typedef typename C2<T>::t T2;
+    static __device__ __forceinline__ void run(T2 *v) {
+        constexpr int R = R1 * R2, E1 = R2 * inv_mod(R2 % R1, R1), E2 = R1 * inv_mod(R1 % R2, R2);
+        T2 a[R1][R2];
+#pragma unroll
+        for (int n2 = 0; n2 < R2; ++n2) {
+            T2 t[R1];
+#pragma unroll
+            for (int n1 = 0; n1 < R1; ++n1) t[n1] = v[(R2 * n1 + R1 * n2) % R];
+            Dft<T, R1>::run(t);
+#pragma unroll
+            for (int k1 = 0; k1 < R1; ++k1) a[k1][n2] = t[k1];
+        }
+#pragma unroll
+        for (int k1 = 0; k1 < R1; ++k1) {
+            Dft<T, R2>::run(a[k1]);
+#pragma unroll
+            for (int k2 = 0; k2 < R2; ++k2) v[(k1 * E1 + k2 * E2) % R] = a[k1][k2];
+        }
+    }
+};
+template <class T> struct Dft<T, 6> : DftPfa<T, 2, 3> {};
+template <class T> struct Dft<T, 10> : DftPfa<T, 2, 5> {};
+template <class T> struct Dft<T, 12> : DftPfa<T, 4, 3> {};
+template <class T> struct Dft<T, 15> : DftPfa<T, 3, 5> {};
+// 9 = 3 x 3: length-3 DFTs over n1 (n = 3 n1 + n2), twiddles W9^(n2 k1),
+// length-3 DFTs over n2 (k = k1 + 3 k2).
+template <class T> struct Dft<T, 9> {
+    typedef typename C2<T>::t T2;
+    static __device__ __forceinline__ T2 rot(T2 z, double c, double s) {
+        T2 r;
+        r.x = (T)c * z.x + (T)s * z.y;
+        r.y = (T)c * z.y - (T)s * z.x;
+        return r;
+    }
+    static __device__ __forceinline__ void run(T2 *v) {
+        T2 a[3][3];
+#pragma unroll
+        for (int n2 = 0; n2 < 3; ++n2) {
+            T2 t[3] = {v[n2], v[3 + n2], v[6 + n2]};
+            Dft<T, 3>::run(t);
+#pragma unroll
+            for (int k1 = 0; k1 < 3; ++k1) a[k1][n2] = t[k1];
+        }
+        // cos and sin of 2 pi e / 9, e = 1, 2, 4
+        a[1][1] = rot(a[1][1], 0.76604444311897803520, 0.64278760968653932632);
+        a[1][2] = rot(a[1][2], 0.17364817766693034885, 0.98480775301220805937);
+        a[2][1] = rot(a[2][1], 0.17364817766693034885, 0.98480775301220805937);
+        a[2][2] = rot(a[2][2], -0.93969262078590838405, 0.34202014332566873304);
+#pragma unroll
+        for (int k1 = 0; k1 < 3; ++k1) {
+            Dft<T, 3>::run(a[k1]);
+#pragma unroll
+            for (int k2 = 0; k2 < 3; ++k2) v[k1 + 3 * k2] = a[k1][k2];
+        }
+    }
+};
+
 // Shared work buffers hold element i at fpad(i) = i + i/8: with one pad per 8
 // complex values the stride-R stores of the early Stockham stages and the
 // unit-stride loads both spread over all banks.
@@ -255,7 +321,7 @@ __device__ __forceinline__ void bar_sync(int id, int n) {
 // the barriers.
 template <class T>
 __device__ typename C2<T>::t *fft_smem(typename C2<T>::t *a, typename C2<T>::t *b, int M,
-                                       const int *rad, int nrad,
+                                       const int *rad, int nrad, const FastDiv *fds,
                                        const typename C2<T>::t *__restrict__ tw, int t, int TT,
                                        int bar_id, int nbar) {
     typedef typename C2<T>::t T2;
@@ -265,8 +331,7 @@ __device__ typename C2<T>::t *fft_smem(typename C2<T>::t *a, typename C2<T>::t *
         const int R = rad[s];
         const int lg = (Ns & (Ns - 1)) == 0 ? __ffs(Ns) - 1 : -1;
         const T2 *tws = tw + (Ns - 1);
-        FastDiv fd;
-        if (lg < 0) fd = FastDiv(Ns);
+        const FastDiv fd = fds[s];               // by Ns
         switch (R) {
             case 16: fft_stage<T, 16>(src, dst, M, Ns, lg, fd, tws, t, TT); break;
             case 8: fft_stage<T, 8>(src, dst, M, Ns, lg, fd, tws, t, TT); break;
@@ -348,7 +413,7 @@ __device__ __forceinline__ typename C2<T>::t *fft_ct_from(typename C2<T>::t *src
         break;
 template <class T, int E, int MC = 0>
 __device__ __forceinline__ typename C2<T>::t *fft_run(typename C2<T>::t *a, typename C2<T>::t *b, int M,
-                                                      const int *rad, int nrad,
+                                                      const int *rad, int nrad, const FastDiv *fds,
                                                       const typename C2<T>::t *__restrict__ tw, int t, int TT,
                                                       int bar_id, int nbar) {
     if constexpr (MC > 0 && MC % E == 0) {
@@ -365,7 +430,7 @@ __device__ __forceinline__ typename C2<T>::t *fft_run(typename C2<T>::t *a, type
             OQG_FFT_CT(4096)
             default: break;
         }
-        return fft_smem<T>(a, b, M, rad, nrad, tw, t, TT, bar_id, nbar);
+        return fft_smem<T>(a, b, M, rad, nrad, fds, tw, t, TT, bar_id, nbar);
     }
 }
 #undef OQG_FFT_CT

@@ -782,7 +782,7 @@ k_xfwd(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int G) {
         }
     }
     __syncthreads();
-    const T2 *z = fft_run<T, E, MC>(za, zb, M, b.rad, b.nrad, (const T2 *)b.tw, live ? t : TT, TT, 0, 0);
+    const T2 *z = fft_run<T, E, MC>(za, zb, M, b.rad, b.nrad, b.fd_ns, (const T2 *)b.tw, live ? t : TT, TT, 0, 0);
     if (!live) return;
     T2 *S = (T2 *)b.spec;
     T2 *sx = S + ((size_t)m * b.ny + j) * b.pk;
@@ -857,7 +857,7 @@ k_bfwd(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int G) {
     pdl_wait();
     if (live) odd_stage_rows<T>(z, x, x + b.pr, two, b.nxin, (T)1, t, TT);
     __syncthreads();
-    odd_fft<T, MC>(z, M, b.orad, b.norad, (const T2 *)b.otw, t, TT, live, [&](int i, T2 v) {
+    odd_fft<T, MC>(z, M, b, (const T2 *)b.otw, t, TT, live, [&](int i, T2 v) {
         sx[i - 1] = -v.y;
         if (two) sy[i - 1] = v.x;
     });
@@ -1346,7 +1346,7 @@ k_binv(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int G, i
     pdl_wait();
     if (live) odd_stage_rows<T>(z, x, x + b.pk, two, n, (T)b.ftnorm, t, TT);
     __syncthreads();
-    odd_fft<T, MC>(z, M, b.orad, b.norad, (const T2 *)b.otw, t, TT, live, [&](int i, T2 v) {
+    odd_fft<T, MC>(z, M, b, (const T2 *)b.otw, t, TT, live, [&](int i, T2 v) {
         ox[i] = -v.y;
         if (two) oy[i] = v.x;
     });
@@ -1418,7 +1418,7 @@ k_xinv_rows(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int
         }
     }
     __syncthreads();
-    const T2 *z = fft_run<T, E, MC>(za, zb, M, b.rad, b.nrad, (const T2 *)b.tw, live ? t : TT, TT, 0, 0);
+    const T2 *z = fft_run<T, E, MC>(za, zb, M, b.rad, b.nrad, b.fd_ns, (const T2 *)b.tw, live ? t : TT, TT, 0, 0);
     if (!live) return;
     T *ox = inh + ((size_t)m * b.nyp + j + 1) * px;
     T *oy = ox + px;
@@ -1498,7 +1498,7 @@ __device__ __forceinline__ void xinv_assemble(const BasinDev &b, int par, const 
         }
     };
     const T fac = (T)b.qb_fac;
-    const FastDiv fdx(nxp);
+    const FastDiv fdx = b.fd_nxp;
     const int npts = (jlast - jfirst + 1) * nxp;
     for (int idx = threadIdx.x; idx < npts; idx += blockDim.x) {
         const int jr = fdx.div(idx), i = idx - jr * nxp, j = jfirst + jr;
@@ -1579,7 +1579,7 @@ k_xinv(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
         // the Hermitian extension of X + iY, conjugated (inhomog.F90:214-255)
         constexpr int U = 4;
         const int nk = b.nk;
-        const FastDiv fd(nk);
+        const FastDiv fd = b.fd_nk;
         for (int x0 = threadIdx.x; x0 < nl * nk; x0 += U * nfft) {
             T2 X[U], Y[U];
 #pragma unroll
@@ -1612,7 +1612,7 @@ k_xinv(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
             }
         }
         bar_sync(1, nfft);
-        const T2 *r = fft_run<T, XINV_E, MC>(z, z + lz / 2, M, b.rad, b.nrad, (const T2 *)b.tw, live ? t : TT, TT, 1, nfft);
+        const T2 *r = fft_run<T, XINV_E, MC>(z, z + lz / 2, M, b.rad, b.nrad, b.fd_ns, (const T2 *)b.tw, live ? t : TT, TT, 1, nfft);
         if (live) {
             // every column; column nxp-1 = M repeats column 0 (inhomog.F90:250)
             for (int i = t; i <= M; i += TT) {
@@ -1627,7 +1627,7 @@ k_xinv(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
             zero.x = zero.y = (T)0;
             z[0] = z[zpad<4>(n + 1)] = zero;
         }
-        const FastDiv fd(n);
+        const FastDiv fd = b.fd_nxin;
 #pragma unroll 4
         for (int x = threadIdx.x; x < nl * n; x += nfft) {
             const int m = fd.div(x), i = x - m * n;
@@ -1638,7 +1638,7 @@ k_xinv(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
             z0[(size_t)m * lz + zpad<4>(i + 1)] = v;
         }
         bar_sync(1, nfft);
-        odd_fft<T, MC>(z, M, b.orad, b.norad, (const T2 *)b.otw, t, TT, live, [&](int i, T2 v) {
+        odd_fft<T, MC>(z, M, b, (const T2 *)b.otw, t, TT, live, [&](int i, T2 v) {
             ox[i] = -v.y;
             oy[i] = v.x;
         }, nfft);
@@ -1735,7 +1735,7 @@ k_xinv_asm(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int 
     T *__restrict__ Qc = (T *)b.F[3 - par];          // q after this step
     const T *__restrict__ Qm = (const T *)b.F[2 + par];
     const T fac = (T)b.qb_fac;
-    const FastDiv fdx(nxp);
+    const FastDiv fdx = b.fd_nxp;
     const int npts = nxp * nyp;
     // the basin's b.asm_items work items interleave: item w.block takes the
     // points w.block * 256 + t, then every b.asm_items * 256 further
@@ -2055,7 +2055,7 @@ template <class T>
 __device__ double area_integral(const BasinDev &b, const T *f, double *red) {
     // eight loads in flight per thread (one at a time, a 257^2 field took 39 us)
     constexpr int U = 8;
-    const FastDiv fd(b.nxp);
+    const FastDiv fd = b.fd_nxp;
     const int n = b.nyp * b.nxp;
     CSum s;
     for (int x0 = threadIdx.x; x0 < n; x0 += U * blockDim.x) {

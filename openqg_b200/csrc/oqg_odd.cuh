@@ -3,8 +3,8 @@
 // The DST-I of n = N - 1 values (inhomog.F90:170-212; FFTW RODFT00) is the FFT
 // of their odd extension to M = 2N points, and two real rows share one complex
 // transform.  The odd extension makes almost half of that FFT redundant.  With
-// the decimation x[r + R0 j] (r < R0, L = M / R0, R0 the largest power of two
-// up to 16 in M) the length-L transform S_r of subsequence r satisfies
+// the decimation x[r + R0 j] (r < R0, L = M / R0, R0 an even divisor of M up to
+// 16) the length-L transform S_r of subsequence r satisfies
 //     S_{R0-r}(k) = -W_L^{-k} S_r(L - k),
 // so only the R0/2 + 1 subsequences r <= R0/2 are transformed (9 of 16), and
 // the last radix-R0 stage runs for k <= L/2 only: its outputs X(k + L k1) give
@@ -29,8 +29,11 @@ template <class T> struct Dft<T, 1> {
     static __device__ __forceinline__ void run(T2 *) {}
 };
 
-// The outer (last) radix of a box length M = 2 (nxp - 1).
-__host__ __device__ constexpr int odd_r0(int M) { return M % 16 == 0 ? 16 : M % 8 == 0 ? 8 : M % 4 == 0 ? 4 : 2; }
+// The outer (last) radix of a box length M = 2 (nxp - 1): the one that leaves
+// the smallest part, (R0/2 + 1) / R0, of the extension to transform.
+__host__ __device__ constexpr int odd_r0(int M) {
+    return M % 16 == 0 ? 16 : M % 12 == 0 ? 12 : M % 10 == 0 ? 10 : M % 8 == 0 ? 8 : M % 6 == 0 ? 6 : M % 4 == 0 ? 4 : 2;
+}
 // Lengths with a compile-time plan: R0 = 16 and L = RA RB in two stages.
 __host__ __device__ constexpr bool odd_ct_len(int M) {
     return M == 128 || M == 192 || M == 256 || M == 384 || M == 512 || M == 1024 || M == 2048 || M == 4096;
@@ -44,7 +47,7 @@ __host__ __device__ constexpr int odd_tt(int M) {
     const int r0 = odd_r0(M), L = M / r0, B = r0 / 2 + 1;
     if (odd_ct_len(M)) return L == 8 ? 9 : L == 12 ? 9 : L == 24 ? 18 : B * L / 16;
     const int a = (B * L + 15) / 16, c = L / 2 + 1;
-    return r0 == 16 && c > a ? c : a;
+    return r0 >= 10 && c > a ? c : a;
 }
 // Padding of the staged rows (one slot per 16 values) and of the subsequences
 // (one per first radix), so that strided butterfly accesses spread over the
@@ -184,13 +187,15 @@ __device__ __forceinline__ void odd_fft_ct(typename C2<T>::t *z, const typename 
         odd_last<T, 16>(M, L, t, tw + (L - 1), [&](int r, int k) { return z[zpad<SH>(r * L + k)]; }, out);
 }
 
-// ---- any length: the same plan at run time, between two buffers.
+// ---- any length: the same plan at run time, between two buffers, with radices
+// up to 16 so that most subsequences take two stages (a barrier and a pass over
+// shared memory each).  The stages are out of line: a length runs two or three
+// of them, and inlined they spilled the kernel's registers.
 template <class T, int R>
-__device__ __forceinline__ void odd_first_rt(const typename C2<T>::t *src, typename C2<T>::t *dst, int M, int R0, int L,
-                                             int t, int TT) {
+__device__ __noinline__ void odd_first_rt(const typename C2<T>::t *src, typename C2<T>::t *dst, int M, int R0, int L,
+                                          FastDiv fd, int t, int TT) {
     typedef typename C2<T>::t T2;
     const int nA = L / R, S = M / R, N = M / 2, nb = (R0 / 2 + 1) * nA;
-    const FastDiv fd(nA);
     for (int bf = t; bf < nb; bf += TT) {
         const int r = fd.div(bf), j = bf - r * nA, i0 = r + R0 * j;
         T2 v[R];
@@ -208,11 +213,10 @@ __device__ __forceinline__ void odd_first_rt(const typename C2<T>::t *src, typen
     }
 }
 template <class T, int R>
-__device__ __forceinline__ void odd_mid_rt(const typename C2<T>::t *src, typename C2<T>::t *dst, int R0, int L, int Ns,
-                                           const typename C2<T>::t *__restrict__ tws, int t, int TT) {
+__device__ __noinline__ void odd_mid_rt(const typename C2<T>::t *src, typename C2<T>::t *dst, int R0, int L, int Ns,
+                                        FastDiv fd, FastDiv fn, const typename C2<T>::t *__restrict__ tws, int t, int TT) {
     typedef typename C2<T>::t T2;
     const int nb1 = L / R, nb = (R0 / 2 + 1) * nb1;
-    const FastDiv fd(nb1), fn(Ns);
     for (int bf = t; bf < nb; bf += TT) {
         const int r = fd.div(bf), j = bf - r * nb1, q0 = fn.div(j), jm = j - q0 * Ns;
         T2 v[R];
@@ -228,37 +232,33 @@ __device__ __forceinline__ void odd_mid_rt(const typename C2<T>::t *src, typenam
         for (int q = 0; q < R; ++q) dst[zpad<3>(d + q * Ns)] = v[q];
     }
 }
+#define OQG_ODD_RADICES(X) X(16) X(15) X(12) X(10) X(9) X(8) X(6) X(5) X(4) X(3) X(2)
 template <class T, class Out>
-__device__ __forceinline__ void odd_fft_rt(typename C2<T>::t *a, int M, const int *rad, int nrad,
+__device__ __forceinline__ void odd_fft_rt(typename C2<T>::t *a, int M, const BasinDev &b,
                                            const typename C2<T>::t *__restrict__ tw, int t, int TT, bool live, Out out,
                                            int nbar) {
     typedef typename C2<T>::t T2;
-    const int R0 = odd_r0(M), L = M / R0;
+    const int R0 = odd_r0(M), L = M / R0, nrad = b.norad;
     T2 *src = a, *dst = a + odd_buf_len(M);
     int Ns = 1;
     // the length's radices, the last of which is R0's own stage below
     for (int s = 0; s < nrad - 1 || s == 0; ++s) {
-        const int R = nrad == 1 ? 1 : rad[s];
+        const int R = nrad == 1 ? 1 : b.orad[s];
         if (live) {
+            const FastDiv fd = b.fd_obf[s], fn = b.fd_ons[s];
             if (s == 0) {
                 switch (R) {
-                    case 16: odd_first_rt<T, 16>(src, dst, M, R0, L, t, TT); break;
-                    case 8: odd_first_rt<T, 8>(src, dst, M, R0, L, t, TT); break;
-                    case 4: odd_first_rt<T, 4>(src, dst, M, R0, L, t, TT); break;
-                    case 2: odd_first_rt<T, 2>(src, dst, M, R0, L, t, TT); break;
-                    case 3: odd_first_rt<T, 3>(src, dst, M, R0, L, t, TT); break;
-                    case 5: odd_first_rt<T, 5>(src, dst, M, R0, L, t, TT); break;
-                    default: odd_first_rt<T, 1>(src, dst, M, R0, L, t, TT); break;
+#define OQG_ODD_F(RR) case RR: odd_first_rt<T, RR>(src, dst, M, R0, L, fd, t, TT); break;
+                    OQG_ODD_RADICES(OQG_ODD_F)
+#undef OQG_ODD_F
+                    default: odd_first_rt<T, 1>(src, dst, M, R0, L, fd, t, TT); break;
                 }
             } else {
                 const T2 *tws = tw + (Ns - 1);
                 switch (R) {
-                    case 16: odd_mid_rt<T, 16>(src, dst, R0, L, Ns, tws, t, TT); break;
-                    case 8: odd_mid_rt<T, 8>(src, dst, R0, L, Ns, tws, t, TT); break;
-                    case 4: odd_mid_rt<T, 4>(src, dst, R0, L, Ns, tws, t, TT); break;
-                    case 2: odd_mid_rt<T, 2>(src, dst, R0, L, Ns, tws, t, TT); break;
-                    case 3: odd_mid_rt<T, 3>(src, dst, R0, L, Ns, tws, t, TT); break;
-                    default: odd_mid_rt<T, 5>(src, dst, R0, L, Ns, tws, t, TT); break;
+#define OQG_ODD_M(RR) case RR: odd_mid_rt<T, RR>(src, dst, R0, L, Ns, fd, fn, tws, t, TT); break;
+                    OQG_ODD_RADICES(OQG_ODD_M)
+#undef OQG_ODD_M
                 }
             }
         }
@@ -270,10 +270,15 @@ __device__ __forceinline__ void odd_fft_rt(typename C2<T>::t *a, int M, const in
     auto get = [&](int r, int k) { return src[zpad<3>(r * L + k)]; };
     const T2 *twl = tw + (L - 1);
     for (int k = t; k <= L / 2; k += TT) {
-        if (R0 == 16) odd_last<T, 16>(M, L, k, twl, get, out);
-        else if (R0 == 8) odd_last<T, 8>(M, L, k, twl, get, out);
-        else if (R0 == 4) odd_last<T, 4>(M, L, k, twl, get, out);
-        else odd_last<T, 2>(M, L, k, twl, get, out);
+        switch (R0) {
+            case 16: odd_last<T, 16>(M, L, k, twl, get, out); break;
+            case 12: odd_last<T, 12>(M, L, k, twl, get, out); break;
+            case 10: odd_last<T, 10>(M, L, k, twl, get, out); break;
+            case 8: odd_last<T, 8>(M, L, k, twl, get, out); break;
+            case 6: odd_last<T, 6>(M, L, k, twl, get, out); break;
+            case 4: odd_last<T, 4>(M, L, k, twl, get, out); break;
+            default: odd_last<T, 2>(M, L, k, twl, get, out);
+        }
     }
 }
 
@@ -281,13 +286,13 @@ __device__ __forceinline__ void odd_fft_rt(typename C2<T>::t *a, int M, const in
 // chosen by the member's length (ensembles); MC < 0: any other length.
 #define OQG_ODD_CASE(MM) case MM: odd_fft_ct<T, MM>(z, tw, t, live, out, nbar); return;
 template <class T, int MC, class Out>
-__device__ __forceinline__ void odd_fft(typename C2<T>::t *z, int M, const int *rad, int nrad,
+__device__ __forceinline__ void odd_fft(typename C2<T>::t *z, int M, const BasinDev &b,
                                         const typename C2<T>::t *__restrict__ tw, int t, int TT, bool live, Out out,
                                         int nbar = 0) {
     if constexpr (MC > 0) {
         odd_fft_ct<T, MC>(z, tw, t, live, out, nbar);
     } else if constexpr (MC < 0) {
-        odd_fft_rt<T>(z, M, rad, nrad, tw, t, TT, live, out, nbar);
+        odd_fft_rt<T>(z, M, b, tw, t, TT, live, out, nbar);
     } else {
         switch (M) {
             OQG_ODD_CASE(128)
@@ -298,7 +303,7 @@ __device__ __forceinline__ void odd_fft(typename C2<T>::t *z, int M, const int *
             OQG_ODD_CASE(1024)
             OQG_ODD_CASE(2048)
             OQG_ODD_CASE(4096)
-            default: odd_fft_rt<T>(z, M, rad, nrad, tw, t, TT, live, out, nbar);
+            default: odd_fft_rt<T>(z, M, b, tw, t, TT, live, out, nbar);
         }
     }
 }
