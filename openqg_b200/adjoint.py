@@ -160,8 +160,7 @@ class QGRun(torch.autograd.Function):
         run = AdjointRun(qg, every, device=psi0.device)
         run.forward(nsteps, tdt)
         ctx.run, ctx.f0, ctx.cdtype = run, f0, curl.dtype
-        p = qg.get_state()[0]
-        return torch.as_tensor(p, dtype=torch.float64, device=psi0.device)
+        return torch.as_tensor(qg.p, dtype=torch.float64, device=psi0.device)
 
     @staticmethod
     def backward(ctx, gp: torch.Tensor):

@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(OQG_ADJ_THREADS) k_adj_wall(const BasinDev *__
     for (int m = 0; m < N; ++m) dot[m] = 0.0;
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < (size_t)nyp * nxp;
          idx += (size_t)gridDim.x * blockDim.x) {
-        const int j = (int)(idx / nxp), i = (int)(idx - (size_t)j * nxp);
+        const int j = b.fd_nxp.div((int)idx), i = (int)idx - j * nxp;
         const size_t o = (size_t)j * px + i;
         const bool zon = (j == 0 || j == nyp - 1), mer = (i == 0 || i == nxp - 1);
         const int cnt = (zon ? 1 : 0) + (mer ? 1 : 0);
@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(OQG_ADJ_THREADS) k_adj_init(const BasinDev *__
     const size_t n2 = (size_t)nyp * px;
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < (size_t)nyp * nxp;
          idx += (size_t)gridDim.x * blockDim.x) {
-        const int j = (int)(idx / nxp), i = (int)(idx - (size_t)j * nxp);
+        const int j = b.fd_nxp.div((int)idx), i = (int)idx - j * nxp;
         const size_t o = (size_t)j * px + i;
         const double w = ((i == 0 || i == nxp - 1) ? 0.5 : 1.0) * ((j == 0 || j == nyp - 1) ? 0.5 : 1.0) * b.dx * b.dy;
         for (int f = 0; f < 2; ++f) {

@@ -1970,7 +1970,7 @@ __global__ void k_qcomp(const BasinDev *__restrict__ bas, int member, const doub
     const double afac = b.fx_bc / b.fx;   // alpha/(alpha/2+1)
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < (size_t)b.nyp * b.nxp;
          idx += (size_t)gridDim.x * blockDim.x) {
-        const int j = (int)(idx / b.nxp), i = (int)(idx - (size_t)j * b.nxp);
+        const int j = b.fd_nxp.div((int)idx), i = (int)idx - j * b.nxp;
         const size_t o2 = (size_t)j * b.px + i;
         double pv[NL];
 #pragma unroll
@@ -2025,7 +2025,7 @@ template <class T>
 __global__ void k_rows_in(const double *src, T *dst, int nxp, int px, size_t nrows) {
     const size_t n = nrows * (size_t)nxp;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t r = i / (size_t)nxp, c = i - r * nxp;
+        const size_t r = (unsigned)i / (unsigned)nxp, c = i - r * nxp;    // n < 2^31
         dst[r * px + c] = (T)src[i];
     }
 }
@@ -2033,7 +2033,7 @@ template <class T>
 __global__ void k_rows_out(const T *src, double *dst, int nxp, int px, size_t nrows) {
     const size_t n = nrows * (size_t)nxp;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t r = i / (size_t)nxp, c = i - r * nxp;
+        const size_t r = (unsigned)i / (unsigned)nxp, c = i - r * nxp;    // n < 2^31
         dst[i] = (double)src[r * px + c];
     }
 }
