@@ -604,6 +604,8 @@ def time_batches(g, tdt, msteps, steps, flush):
 
 PHASES = ["k_vort", "k_xfwd", "k_ysolve", "k_xinv"]
 # a closed box runs the inverse transforms and the assembly as two launches
+# (its transforms are k_bfwd and k_binv, a channel's k_xfwd and k_xinv_rows; the
+# phases keep one name)
 PHASES_SEP = ["k_vort", "k_xfwd", "k_ysolve", "k_xinv_rows", "k_xinv_asm"]
 
 

@@ -301,22 +301,22 @@ int oqg_autotune(oqg_handle *h, double tdt, int nsteps, int *best_vty, double *m
 /* Current tile height of the vorticity kernel. */
 int oqg_get_vty(oqg_handle *h, int *vty);
 
-/* The y-solve's warps per column (1, 2 or 4): oqg_create picks enough for
- * about 20 warps per SM while each lane keeps 4 to 8 rows; this measures the
- * three on the device like oqg_autotune (nsteps steps of tdt from the
- * current state, restored) and keeps the fastest.  ms[0..2]: ms per step
- * with 1, 2 and 4 warps.  Results agree to rounding (the scan's
- * association changes with the split). */
+/* The spread of a y-solve column over threads (1, 2 or 4: fewer and longer to
+ * more and shorter chunks of rows; "warps"): oqg_create starts with 2; this
+ * measures the three on the device like oqg_autotune (nsteps steps of tdt from
+ * the current state, restored) and keeps the fastest.  ms[0..2]: ms per step
+ * with 1, 2 and 4.  Results agree to rounding (the scan's association changes
+ * with the split). */
 int oqg_autotune_ysolve(oqg_handle *h, double tdt, int nsteps, int *best_warps, double *ms);
-/* Current warps per y-solve column. */
+/* Current spread of a y-solve column. */
 int oqg_get_ysolve_warps(oqg_handle *h, int *warps);
-/* Fix the vorticity tile height (8, 12 or 16) or the y-solve's warps per
+/* Fix the vorticity tile height (8, 12 or 16) or the y-solve's spread per
  * column (1, 2 or 4) without measuring, e.g. from an earlier oqg_autotune
  * on the same GPU; OQG_EINVAL for other values. */
 int oqg_set_vty(oqg_handle *h, int vty);
 int oqg_set_ysolve_warps(oqg_handle *h, int warps);
 /* The inverse transforms as a launch shaped like the forward
- * one (k_xinv_rows, which also runs the step's scalar phase once) and a
+ * one (k_binv, k_xinv_rows; it also runs the step's scalar phase once) and a
  * one-pass assembly (k_xinv_asm), instead of one kernel that transforms and
  * assembles in shared memory.  On by default for boxes, off for channels;
  * it cannot be turned off where the modal rows do not fit in shared memory

@@ -336,8 +336,9 @@ class QG:
         return best.value, {v: float(ms[v]) for v in range(8, 18) if np.isfinite(ms[v])}
 
     def autotune_ysolve(self, tdt: float, nsteps: int = 20):
-        """Measures the y-solve with 1, 2 and 4 warps per column and keeps the
-        fastest; returns (warps, {warps: ms per step})."""
+        """Measures the y-solve with its columns spread 1, 2 and 4 wide (about
+        25, 50 and 100 chunks of rows) and keeps the fastest; returns
+        (spread, {spread: ms per step})."""
         best = ctypes.c_int()
         ms = (ctypes.c_double * 3)()
         _check(lib().oqg_autotune_ysolve(self.h, float(tdt), int(nsteps), ctypes.byref(best), ms),
@@ -349,7 +350,7 @@ class QG:
         _check(lib().oqg_set_vty(self.h, int(rows)), "oqg_set_vty")
 
     def set_ysolve_warps(self, warps: int):
-        """Fixes the y-solve's warps per column (1, 2 or 4) without measuring."""
+        """Fixes the spread of the y-solve's columns (1, 2 or 4) without measuring."""
         _check(lib().oqg_set_ysolve_warps(self.h, int(warps)), "oqg_set_ysolve_warps")
 
     def set_xinv_sep(self, on: bool):
