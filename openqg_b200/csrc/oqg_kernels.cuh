@@ -243,24 +243,26 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// Queues the copy of rows [jlo, jlo+nr) x cols [ilo, ilo+nc) of layer k of a
-// channel's f into s (leading dimension nc); outside the basin -> 0.  Columns
+// Queues the copy of rows [jlo, jlo+nr) x cols [ilo, ilo+nc) of layer k of f
+// into s (leading dimension nc); outside the basin -> 0.  A channel's columns
 // of a halo tile wrap with period nxp-1 as far as the last output column's
 // halo; an `own` tile (the CTA's output columns only) reads columns < nxp as
 // stored, including the duplicate column nxp-1, and zeros beyond, so it never
-// reads a column that another CTA writes.
+// reads a column that another CTA writes.  A box (whose tiles come so when
+// there are no tensor maps) has no column outside 0 .. nxp-1.
 // Thread layout: 64 columns x blockDim / 64 rows.
 template <class T, class G>
 __device__ __forceinline__ void load_tile_async(T *s, const T *__restrict__ f, const G &g, int px,
                                                 int k, int jlo, int nr, int ilo, int nc,
                                                 bool own = false) {
     const int N = g.nxp - 1;
+    const bool wrap = g.cyclic && !own;
     const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
     const T *fk = f + (size_t)k * g.nyp * px;
     for (int c = tx; c < nc; c += 64) {
         const int gi = ilo + c;
-        const bool cv = own ? gi < g.nxp : gi < g.nxp + 3;
-        const int i = !cv ? 0 : own ? gi : gi < 0 ? gi + N : gi >= N ? gi - N : gi;
+        const bool cv = wrap ? gi < g.nxp + 3 : gi >= 0 && gi < g.nxp;
+        const int i = !cv ? 0 : !wrap ? gi : gi < 0 ? gi + N : gi >= N ? gi - N : gi;
         for (int r = ty; r < nr; r += blockDim.x >> 6) {
             const int j = jlo + r;
             const bool v = cv && j >= 0 && j < g.nyp;
