@@ -628,6 +628,15 @@ static bool make_tmaps(oqg_handle *h) {
     return true;
 }
 
+// The maps of a new tile height, where the handle has maps.  A channel steps
+// without them (its tiles all come by cp.async) when they cannot be encoded.
+static bool retile_tmaps(oqg_handle *h) {
+    BasinDev &b = h->hb;
+    if (!b.tmaps || make_tmaps(h)) return true;
+    if (b.cyclic) b.tmaps = nullptr;
+    return b.cyclic != 0;
+}
+
 // ----------------------------------------------------------- homogeneous solutions
 // homsol_box (homog.F90:214-278) and homsol_cyclic (homog.F90:128-212); the
 // Helmholtz solves run on the device.
@@ -2480,7 +2489,7 @@ static int set_vty(oqg_handle *h, int vt) {
     std::vector<Work> wv(h->nv);
     for (int i = 0; i < h->nv; ++i) wv[i] = Work{0, i};
     CK(cudaMemcpy(h->d_wv, wv.data(), wv.size() * sizeof(Work), cudaMemcpyHostToDevice));
-    if (b.tmaps && !make_tmaps(h)) return fail(OQG_ECUDA, "tensor maps could not be encoded");
+    if (!retile_tmaps(h)) return fail(OQG_ECUDA, "tensor maps could not be encoded");
     h->smem_v = vort_smem_bytes(vt, (int)h->esz);
     set_attrs(h);
     h->hb64.vty = b.vty;
@@ -2664,7 +2673,7 @@ static int ens_set_vty(oqg_ensemble *e, int vt) {
         BasinDev &b = h->hb;
         b.vty = vt;
         b.tiles_y = vort_tile_rows(b.nyp, vt);
-        if (b.tmaps && !make_tmaps(h)) return fail(OQG_ECUDA, "tensor maps could not be encoded");
+        if (!retile_tmaps(h)) return fail(OQG_ECUDA, "tensor maps could not be encoded");
         h->hb64.vty = b.vty;
         h->hb64.tiles_y = b.tiles_y;
         h->hb64.tmaps = b.tmaps;

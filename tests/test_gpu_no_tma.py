@@ -84,3 +84,26 @@ def test_ensemble_without_tensor_maps(monkeypatch, precision, tol):
     for i, b in enumerate(bs):
         _check(e.get_state(i), b, tol)
     e.close()
+
+
+def test_channel_retiles_without_tensor_maps(monkeypatch):
+    """A channel created with tensor maps takes another tile height, alone and in
+    an ensemble's tuner, where they can no longer be encoded."""
+    b = _basin(181, 101, True, 0)
+    monkeypatch.delenv("OQG_NO_TMA", raising=False)
+    g, e = QG(b), Ensemble([b, b])
+    p, pm, w = _state(b)
+    for i in range(2):
+        e.set_state(i, p, pm)
+        e.set_forcing(i, w)
+    monkeypatch.setenv("OQG_NO_TMA", "1")
+    for rows in (12, 8, 16):
+        g.set_tile_rows(rows)
+    _check(_step(g, b), b, 1e-12)
+    e.autotune(600.0, 2)
+    e.step(600.0, 2)
+    e.sync()
+    for i in range(2):
+        _check(e.get_state(i), b, 1e-12)
+    g.close()
+    e.close()
