@@ -134,7 +134,9 @@ static void launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem,
 template <class T, bool CPLX>
 static void (*ysolve_kernel(int R, int KB))(const BasinDev *, const Work *) {
     constexpr int K = CPLX ? 4 : 8;
-    if (KB == 1) return k_ysolve<T, CPLX, YS_ROWS, 1>;
+    if constexpr (!CPLX) {
+        if (KB == 1) return k_ysolve<T, CPLX, YS_ROWS, 1>;      // (a channel has at most 3584 rows)
+    }
     if (KB == 2) return k_ysolve<T, CPLX, YS_ROWS, 2>;
     if (KB < K) return k_ysolve<T, CPLX, YS_ROWS, K / 2>;
     return R == 4 ? k_ysolve<T, CPLX, 4, K> : R == 8 ? k_ysolve<T, CPLX, 8, K> : k_ysolve<T, CPLX, YS_ROWS, K>;

@@ -835,8 +835,8 @@ __device__ __forceinline__ void odd_stage_rows(typename C2<T>::t *z, const T *__
 }
 
 // A box's forward transform: DST-I of the modal right-hand side's row pairs
-// (oqg_odd.cuh).  A CTA holds G = b.xg transforms (an ensemble: as many as
-// its threads serve, G <= 0), numbered with the mode fastest.
+// (oqg_odd.cuh).  A CTA holds G transforms (G <= 0, an ensemble: as many as
+// its threads serve), numbered with the mode fastest.
 template <class T, int MC = 0>
 __global__ void __launch_bounds__(256, 2)
 k_bfwd(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int G) {
@@ -2196,7 +2196,7 @@ __device__ __forceinline__ void block_sum_n(double (&v)[K]) {
 }
 
 template <class T>
-__device__ void forcing_integrals_cta(const BasinDev &b, const T *E, double *red) {
+__device__ void forcing_integrals_cta(const BasinDev &b, const T *E) {
     DevForcing *sc = b.frc;
     const size_t n2 = (size_t)b.nyp * b.px;
     // ent_rows' trapezoidal sum, and for a channel the trapezoidal x-sums of
@@ -2242,9 +2242,8 @@ __device__ void forcing_integrals_cta(const BasinDev &b, const T *E, double *red
 // descriptor's entrainment, one CTA.
 template <class T>
 __global__ void k_forcing_integrals(const BasinDev *__restrict__ bas, int member) {
-    __shared__ double red[64];
     const BasinDev &b = bas[member];
-    forcing_integrals_cta<T>(b, (const T *)b.ent, red);
+    forcing_integrals_cta<T>(b, (const T *)b.ent);
 }
 
 // Whether this CTA is the last of its grid to arrive (a ticket counter that

@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(128) k_oml_post(OmlDev o, T *wekp, T *ent, dou
     // boundary stress integrals (ekman.F90:60-70)
     if (!last_cta(ticket)) return;
     __syncthreads();
-    forcing_integrals_cta<T>(bas[0], ent_after, red);
+    forcing_integrals_cta<T>(bas[0], ent_after);
     if (threadIdx.x == 0) {
         bas[0].frc->txis = 0.0;
         bas[0].frc->txin = 0.0;
@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(128) k_aml_post(AmlDev o, const T *__restrict_
     __syncthreads();
     aml_strips_cta(o, bas[0].frc, red);
     __syncthreads();
-    forcing_integrals_cta<T>(bas[0], ent_after, red);
+    forcing_integrals_cta<T>(bas[0], ent_after);
 }
 
 // The atmosphere's wind stress from its lagged layer-1 pressure (xforc,

@@ -30,9 +30,10 @@ template <class T> struct Dft<T, 1> {
 };
 
 // The outer (last) radix of a box length M = 2 (nxp - 1): the one that leaves
-// the smallest part, (R0/2 + 1) / R0, of the extension to transform.
+// the smallest part, (R0/2 + 1) / R0, of the extension to transform.  (M is even,
+// at least 8 and has no prime factor above 5: one of these divides it.)
 __host__ __device__ constexpr int odd_r0(int M) {
-    return M % 16 == 0 ? 16 : M % 12 == 0 ? 12 : M % 10 == 0 ? 10 : M % 8 == 0 ? 8 : M % 6 == 0 ? 6 : M % 4 == 0 ? 4 : 2;
+    return M % 16 == 0 ? 16 : M % 12 == 0 ? 12 : M % 10 == 0 ? 10 : M % 8 == 0 ? 8 : 6;
 }
 // Lengths with a compile-time plan: R0 = 16 and L = RA RB in two stages.
 __host__ __device__ constexpr bool odd_ct_len(int M) {
@@ -232,7 +233,10 @@ __device__ __noinline__ void odd_mid_rt(const typename C2<T>::t *src, typename C
         for (int q = 0; q < R; ++q) dst[zpad<3>(d + q * Ns)] = v[q];
     }
 }
+// The radices of a subsequence, largest first; those of later stages (2 and 16
+// never are: a plan has the fewest stages, of those the least sum).
 #define OQG_ODD_RADICES(X) X(16) X(15) X(12) X(10) X(9) X(8) X(6) X(5) X(4) X(3) X(2)
+#define OQG_ODD_LATER(X) X(15) X(12) X(10) X(9) X(8) X(6) X(5) X(4) X(3)
 template <class T, class Out>
 __device__ __forceinline__ void odd_fft_rt(typename C2<T>::t *a, int M, const BasinDev &b,
                                            const typename C2<T>::t *__restrict__ tw, int t, int TT, bool live, Out out,
@@ -257,7 +261,7 @@ __device__ __forceinline__ void odd_fft_rt(typename C2<T>::t *a, int M, const Ba
                 const T2 *tws = tw + (Ns - 1);
                 switch (R) {
 #define OQG_ODD_M(RR) case RR: odd_mid_rt<T, RR>(src, dst, R0, L, Ns, fd, fn, tws, t, TT); break;
-                    OQG_ODD_RADICES(OQG_ODD_M)
+                    OQG_ODD_LATER(OQG_ODD_M)
 #undef OQG_ODD_M
                 }
             }
@@ -275,9 +279,7 @@ __device__ __forceinline__ void odd_fft_rt(typename C2<T>::t *a, int M, const Ba
             case 12: odd_last<T, 12>(M, L, k, twl, get, out); break;
             case 10: odd_last<T, 10>(M, L, k, twl, get, out); break;
             case 8: odd_last<T, 8>(M, L, k, twl, get, out); break;
-            case 6: odd_last<T, 6>(M, L, k, twl, get, out); break;
-            case 4: odd_last<T, 4>(M, L, k, twl, get, out); break;
-            default: odd_last<T, 2>(M, L, k, twl, get, out);
+            default: odd_last<T, 6>(M, L, k, twl, get, out);
         }
     }
 }

@@ -76,6 +76,7 @@ WIDTHS = [
 def test_widths_cover_the_plans():
     every = set().union(*map(_features, _admitted()))
     assert {f[1] for f in every if f[0] == "outer"} == {16, 12, 10, 8, 6}
+    assert {f[1] for f in every if f[0] in (1, 2)} == set(RADICES) - {16, 2}      # OQG_ODD_LATER
     assert set().union(*map(_features, WIDTHS)) == every
 
 
