@@ -312,15 +312,17 @@ int oqg_autotune_ysolve(oqg_handle *h, double tdt, int nsteps, int *best_warps, 
 int oqg_get_ysolve_warps(oqg_handle *h, int *warps);
 /* Fix the vorticity tile height (8, 12 or 16) or the y-solve's spread per
  * column (1, 2 or 4) without measuring, e.g. from an earlier oqg_autotune
- * on the same GPU; OQG_EINVAL for other values. */
+ * on the same GPU; OQG_EINVAL for other values.  A box may have 7200, 7168
+ * or 7040 interior rows at spread 1, 2 or 4, a channel 3584, 3520 or 3456
+ * (OQG_EUNSUPPORTED; oqg_create takes any grid that spread 1 does). */
 int oqg_set_vty(oqg_handle *h, int vty);
 int oqg_set_ysolve_warps(oqg_handle *h, int warps);
 /* The inverse transforms as a launch shaped like the forward
  * one (k_binv, k_xinv_rows; it also runs the step's scalar phase once) and a
  * one-pass assembly (k_xinv_asm), instead of one kernel that transforms and
  * assembles in shared memory.  On by default for boxes, off for channels;
- * it cannot be turned off where the modal rows do not fit in shared memory
- * (1025 points wide and more: OQG_EUNSUPPORTED). */
+ * it cannot be turned off (OQG_EUNSUPPORTED) above 1601, 1025 and 801 points
+ * across for boxes of 2, 3 and 4 layers, 2701, 1801 and 1351 for channels. */
 int oqg_set_xinv_sep(oqg_handle *h, int on);
 int oqg_get_xinv_sep(oqg_handle *h, int *on);
 /* Measures the two forms of the inverse transform and assembly (one kernel,

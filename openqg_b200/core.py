@@ -359,9 +359,10 @@ class QG:
         _check(lib().oqg_set_xinv_sep(self.h, 1 if on else 0), "oqg_set_xinv_sep")
 
     def autotune_xinv(self, tdt: float, nsteps: int = 20):
-        """Grids below 1025 points: measures the inverse transform and
-        assembly as one kernel and as two launches and keeps the faster;
-        returns (two_launches, {False: ms, True: ms}) for the forms measured."""
+        """Measures the inverse transform and assembly as one kernel (where
+        the grid is narrow enough, oqg_set_xinv_sep) and as two launches and
+        keeps the faster; returns (two_launches, {False: ms, True: ms}) for
+        the forms measured."""
         best = ctypes.c_int()
         ms = (ctypes.c_double * 2)()
         _check(lib().oqg_autotune_xinv(self.h, float(tdt), int(nsteps), ctypes.byref(best), ms),

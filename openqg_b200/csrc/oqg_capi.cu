@@ -67,7 +67,7 @@ struct oqg_handle {
     int E = 8, xthreads = 128, xi_threads = 64;
     int yW = 1;                          // spread of a y-solve column as set or tuned
     YGeo yg{};                           // the y-solve's launch
-    bool xinv_split_needed = false;      // the modal rows do not fit in shared memory
+    bool xinv_split_needed = false;      // too wide for the one-kernel inverse (xinv_most)
     int na = 0;                          // CTAs of k_xinv_asm
     int xg = 1;                          // transforms per CTA of k_xfwd and k_xinv_rows
     size_t smem_v = 0, smem_x = 0, smem_x64 = 0, smem_i = 0;
@@ -104,13 +104,12 @@ static X *dalloc(oqg_handle *h, size_t count) {
 
 // ----------------------------------------------------------- launch helpers
 
-// Whether a grid may take the one-kernel inverse (oqg_set_xinv_sep): two
-// buffers of nl transforms of M FP64 values, threads for them, and the modal
-// rows of a row pair and a wall row in shared memory.
-static bool xinv_fits(int M, int nl, int ny, int nxp) {
-    const int tt = (M + XINV_E - 1) / XINV_E, nfft = std::max(std::min(512, rup(nl * tt, 32)), rup(tt, 32)), G = nfft / tt;
-    const size_t set = (size_t)G * fft_buf_len(M) * 16, inh = (size_t)nl * (ny > 2 ? 3 : ny + 2) * nxp * 8;
-    return (G >= nl ? std::max(2 * set, set + inh) : 2 * set + inh) <= 227 * 1024;
+// The longest transform that may take the one-kernel inverse (oqg_set_xinv_sep),
+// by layers: a limit of the interface, up to which k_xinv needs at most 191 KB of
+// shared memory (xinv_bytes) and 384 threads.
+static int xinv_most(int nl, bool cyclic) {
+    static const int box[] = {3200, 2048, 1600}, channel[] = {2700, 1800, 1350};
+    return (cyclic ? channel : box)[nl - 2];
 }
 
 // Launch with programmatic stream serialisation: the kernel may be scheduled
@@ -161,16 +160,17 @@ static YGeo ysolve_geo(int ny, int nk, int nl, bool cplx, int W) {
 }
 // Column groups of a basin (the work list has room for one per CTA).
 static int ysolve_groups(const BasinDev &b) { return b.nl * ((b.nk + b.ykb - 1) / b.ykb); }
-// Spread of a y-solve column (oqg_set_ysolve_warps): the middle one.
-static int ysolve_warps(int ny, long long ncols) {
-    (void)ny;
-    (void)ncols;
-    return 2;
-}
-// Whether this build takes columns of ny rows at spread W (values of vsz bytes).
-static bool ysolve_fits(int ny, int W, int vsz) {
-    const int L = 32 * W, s = ny <= 4 * L ? 4 : ny <= 8 * L ? 8 : ny <= 16 * L ? 16 : (ny + L - 1) / L;
-    return (size_t)std::max((ny + 32) | 1, (L * (s + 1) + 1) | 1) * 4 * vsz <= 227 * 1024;
+// Spread of a y-solve column that a handle or an ensemble starts with
+// (oqg_set_ysolve_warps): the middle one.  us per step at 1 / 2 / 4: 129^2 21.9 /
+// 21.6 / 21.9, 257^2 30.4 / 29.3 / 29.0, 513^2 47.3 / 47.4 / 48.2, channels 385 x
+// 193 38.1 / 37.4 / 37.4, 769 x 481 72.2 / 72.1 / 67.2, 1025 x 801 122.0 / 121.9 /
+// 123.9.
+#define YS_SPREAD 2
+// The tallest column at spread W: a limit of the interface (k_ysolve itself holds
+// YS_ROWS * YS_THREADS = 8192 rows).
+static int ysolve_most(bool cyclic, int W) {
+    const int most = W == 1 ? 7200 : W == 2 ? 7168 : 7040;
+    return !cyclic ? most : W == 1 ? 3584 : W == 2 ? 3520 : 3456;
 }
 
 // The fewest radices of odd_fft_rt whose product is L, of those the least sum.
@@ -209,7 +209,8 @@ static void odd_radices(int M, std::vector<int> &rad) {
 // for each length of the configurations' grids (boxes of 65 to 2049 points,
 // the 193-point channel; only that FFT plan in its code), the any-length one
 // otherwise.  M = 0: an ensemble of several lengths.
-#define OQG_XLENS(X) X(128) X(192) X(256) X(384) X(512) X(1024) X(2048) X(4096)
+#define OQG_XINV_LENS(X) X(128) X(192) X(256) X(384) X(512) X(1024) X(2048)     // up to xinv_most
+#define OQG_XLENS(X) OQG_XINV_LENS(X) X(4096)
 template <class T>
 static void (*bfwd_kernel(int M))(const BasinDev *, const Work *, int) {
     switch (M) {
@@ -324,7 +325,7 @@ static void (*xinv_kernel(bool cyclic, int M))(const BasinDev *, const Work *, i
     if constexpr (sizeof(T) == 8) {
         switch (M) {
 #define OQG_XK(MM) case MM: return k_xinv<T, true, MM>;
-            OQG_XLENS(OQG_XK)
+            OQG_XINV_LENS(OQG_XK)
 #undef OQG_XK
         }
     }
@@ -1125,9 +1126,8 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     h->xthreads = GX * TT;
     h->xg = GX;
     h->nx = (b.nl * npm + GX - 1) / GX;
-    h->yW = ysolve_warps(b.ny, (long long)b.nl * b.nk);
-    if (!ysolve_fits(b.ny, 1, b.cyclic ? 16 : 8))
-        return bail(OQG_EUNSUPPORTED, "grid too large for this build's shared-memory tiling");
+    h->yW = YS_SPREAD;
+    if (b.ny > ysolve_most(b.cyclic, 1)) return bail(OQG_EUNSUPPORTED, "grid taller than the y-solve's limit");
     h->yg = ysolve_geo(b.ny, b.nk, b.nl, b.cyclic, h->yW);
     b.ykb = h->yg.KB;
     h->ni = npm;
@@ -1143,7 +1143,7 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     b.inh_g = dalloc<char>(h, (size_t)b.nl * b.nyp * b.px * 8);
     b.scal_g = dalloc<char>(h, sizeof(XinvScal));
     if (!b.inh_g || !b.scal_g) return bail(OQG_ECUDA, "out of device memory");
-    h->xinv_split_needed = !xinv_fits(b.M, b.nl, b.ny, b.nxp);
+    h->xinv_split_needed = b.M > xinv_most(b.nl, b.cyclic);
     h->xi_threads = xinv_threads(b.M, b.cyclic, b.nl) + 32;
     h->smem_i = h->xinv_split_needed ? 0 : xinv_bytes(b.M, b.cyclic, b.nl, b.nxp, (int)h->esz);
     // at most 8 work items of 256 threads per SM (the items stride over larger
@@ -1153,8 +1153,7 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     h->na = b.asm_items;
     // boxes: the inverse transforms run as a launch of their own, shaped like
     // the forward one, then a one-pass assembly (oqg_set_xinv_sep; the only
-    // form once the modal rows leave shared memory); channels start with the
-    // one-kernel form
+    // form of wide grids); channels start with the one-kernel form
     apply_xinv_sep(h, !b.cyclic || h->xinv_split_needed);
     if (h->smem_x64 > 227 * 1024)
         return bail(OQG_EUNSUPPORTED, "grid too large for this build's shared-memory tiling");
@@ -1930,10 +1929,9 @@ int oqg_ensemble_create(const oqg_params *members, int nmembers, oqg_ensemble **
     for (oqg_handle *h : e->m)
         if (h->hb.M != e->Mu) e->Mu = 0;
     {
-        long long cols = 0;
         int ny_max = 0;
-        for (oqg_handle *h : e->m) { cols += (long long)h->hb.nl * h->hb.nk; ny_max = std::max(ny_max, h->hb.ny); }
-        e->yW = ysolve_warps(ny_max, cols);
+        for (oqg_handle *h : e->m) ny_max = std::max(ny_max, h->hb.ny);
+        e->yW = YS_SPREAD;
         // one shape for every member: the tallest's, with CTAs of its threads
         // (shorter columns pack several groups into one)
         e->yg = ysolve_geo(ny_max, 1, 1, e->cyclic, e->yW);
@@ -2503,7 +2501,8 @@ static int set_vty(oqg_handle *h, int vt) {
 
 // The y-solve's columns spread by W: the launch shape, the graphs.
 static int set_ysolve_w(oqg_handle *h, int W) {
-    if (!ysolve_fits(h->hb.ny, W, h->hb.cyclic ? 16 : 8)) return fail(OQG_EUNSUPPORTED, "y-solve tile too large");
+    if (h->hb.ny > ysolve_most(h->hb.cyclic, W))
+        return fail(OQG_EUNSUPPORTED, "grid taller than the y-solve's limit at this spread");
     h->yW = W;
     h->yg = ysolve_geo(h->hb.ny, h->hb.nk, h->hb.nl, h->hb.cyclic, W);
     drop_graphs(h);
@@ -2600,7 +2599,7 @@ int oqg_get_xinv_sep(oqg_handle *h, int *on) {
 int oqg_autotune_xinv(oqg_handle *h, double tdt, int nsteps, int *best_sep, double *ms) {
     if (!h || nsteps < 2 || !(tdt > 0.0)) return fail(OQG_EINVAL, "bad argument");
     if (ms) ms[0] = ms[1] = -1.0;
-    // grids whose modal rows leave shared memory have the two-launch form only
+    // wide grids have the two-launch form only
     if (h->xinv_split_needed) {
         if (best_sep) *best_sep = h->hb.xinv_sep;
         return OQG_OK;

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import oracle
-from openqg_b200.core import QG, Ensemble
+from openqg_b200.core import QG, Ensemble, OqgError
 from openqg_b200.params import OQG_MIXED, Basin
 from tests.qg_numpy import rel_l2
 
@@ -75,3 +75,39 @@ def test_ensemble_of_tall_and_short_boxes(precision, tol):
             assert rel_l2(a, r) <= tol, i
         o.close()
     e.close()
+
+
+def _takes(call):
+    try:
+        call()
+    except OqgError as e:
+        assert "OQG_EUNSUPPORTED" in str(e)
+        return False
+    return True
+
+
+@pytest.mark.parametrize("cyclic,most", [(False, (7200, 7168, 7040)), (True, (3584, 3520, 3456))], ids=["box", "channel"])
+def test_height_limits(cyclic, most):
+    def basin(ny):
+        return Basin(nxp=9, nyp=ny + 2, dx=1e4, dy=1e4, h=[500.0, 3500.0], gp=[0.03], ah4=[1e9] * 2, ah2=[0.0] * 2,
+                     cyclic=cyclic, dz_sign=1 if cyclic else -1, k_topo=1 if cyclic else 2)
+
+    for ny in sorted({m + d for m in most for d in (0, 1)}):
+        if ny > most[0]:
+            assert not _takes(lambda: QG(basin(ny)).close())
+            continue
+        g = QG(basin(ny))
+        assert [_takes(lambda: g.set_ysolve_warps(w)) for w in (1, 2, 4)] == [ny <= m for m in most], ny
+        g.close()
+
+
+# nxp at the one-kernel inverse's limit and the next admitted length
+@pytest.mark.parametrize("nl,cyclic,nxp,beyond", [(2, False, 1601, 1621), (3, False, 1025, 1081), (4, False, 801, 811),
+                                                  (2, True, 2701, 2881), (3, True, 1801, 1876),
+                                                  (4, True, 1351, 1441)])
+def test_one_kernel_inverse_limits(nl, cyclic, nxp, beyond):
+    for n, ok in ((nxp, True), (beyond, False)):
+        g = QG(Basin(nxp=n, nyp=9, dx=1e4, dy=1e4, h=[300.0, 500.0, 1000.0, 2200.0][:nl], gp=[0.05, 0.025, 0.015][:nl - 1],
+                     ah4=[1e9] * nl, ah2=[0.0] * nl, cyclic=cyclic, dz_sign=1 if cyclic else -1, k_topo=1 if cyclic else nl))
+        assert _takes(lambda: g.set_xinv_sep(False)) == ok
+        g.close()
