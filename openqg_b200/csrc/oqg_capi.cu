@@ -231,27 +231,32 @@ static void (*binv_kernel(int M))(const BasinDev *, const Work *, int, int, int,
         default: return k_binv<T, -1>;
     }
 }
+// A channel's.  FP32 storage takes the any-length instances: us per step of a
+// channel in two inverse launches, any-length / per-length, 129 x 97 25.4 / 25.2,
+// 193 x 97 27.4 / 28.0, 385 x 193 35.2 / 37.8, 513 x 257 38.1 / 40.4, 1025 x 401
+// 56.6 / 59.2.  (2049 x 513 113.6 / 105.6 and 4097 x 257 113.1 / 104.3 go the other
+// way; nothing takes them apart so far.)
 template <class T, int E>
 static void (*xfwd_kernel(int M))(const BasinDev *, const Work *, int) {
-    // FP32 storage keeps the any-length instances: at 513 points the step
-    // measured 44.5 us with them against 48.1 us with the per-length ones
-    if (std::is_same<T, float>::value) M = 0;
-    switch (M) {
+    if constexpr (sizeof(T) == 8) {
+        switch (M) {
 #define OQG_XF(MM) case MM: return k_xfwd<T, E, MM>;
-        OQG_XLENS(OQG_XF)
+            OQG_XLENS(OQG_XF)
 #undef OQG_XF
-        default: return k_xfwd<T, E>;
+        }
     }
+    return k_xfwd<T, E>;
 }
 template <class T, int E>
 static void (*xinv_rows_kernel(int M))(const BasinDev *, const Work *, int, int, int, double, T *) {
-    if (std::is_same<T, float>::value) M = 0;      // as xfwd_kernel
-    switch (M) {
+    if constexpr (sizeof(T) == 8) {
+        switch (M) {
 #define OQG_XI(MM) case MM: return k_xinv_rows<T, E, MM>;
-        OQG_XLENS(OQG_XI)
+            OQG_XLENS(OQG_XI)
 #undef OQG_XI
-        default: return k_xinv_rows<T, E>;
+        }
     }
+    return k_xinv_rows<T, E>;
 }
 
 // The launches of the x-transforms.  cyclic: a channel's kernels; M: the
