@@ -867,10 +867,12 @@ k_bfwd(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int G) {
 
 // ------------------------------------------------------------------ k_ysolve
 // Thomas solves in y (inhomog.F90:187-199), one column per (mode, wavenumber).
-// The lanes of a warp lie along the wavenumber: KB adjacent columns (64 bytes of
-// FP64) times 32 / KB chunks of R rows, so every load and store of a row is
-// whole sectors and a column's values stay in the registers of its threads
-// from load to store.  Both substitutions are affine recurrences with the same
+// The lanes of a warp lie along the wavenumber: KB adjacent columns times 32 / KB
+// chunks of R rows, and a column's values stay in the registers of its threads
+// from load to store.  A row's access is KB values: 64 bytes of FP64 (32 of FP32)
+// up to 1024 rows of a box, half of that up to 2048, where an FP32 row is then
+// half of its 32-byte sector, a quarter up to 4096, and one value above; a
+// channel's complex values are 64 bytes (32) up to 2048 rows, half above.  Both substitutions are affine recurrences with the same
 // coefficients e_j = -a beta_j:
 //   down   u_j = beta_j f_j + e_j u_{j-1},   up   w_j = u_j + e_j w_{j+1}.
 // A thread runs its R rows from a zero input (v_j) and keeps the products
@@ -879,10 +881,11 @@ k_bfwd(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int G) {
 // The chunk maps are scanned across the lanes by shuffles and across the warps
 // of a column group through shared memory (two barriers in all).
 //
-// Bound by latency.  The kernel this replaces staged four columns per CTA in
-// shared memory (32-byte rows; 16-byte ones in FP32 storage, half of each
-// sector unused) with the lanes along y: strided pivot loads and six passes
-// over the tile.
+// Bound by latency: a thread's two serial passes over its rows and the scans;
+// above 1024 rows one CTA of 512 threads fills an SM, and no load overlaps
+// another group's passes.  Per launch 11.2 us at 513^2 and 93 us at 2049^2 FP64
+// (91 in FP32 storage); staging four columns per CTA in shared memory with the
+// lanes along y took 14.5 and 147 us (132).
 template <class T, bool CPLX> struct YT;
 template <class T> struct YT<T, false> { typedef double v; typedef T g; };
 template <class T> struct YT<T, true> { typedef double2 v; typedef typename C2<T>::t g; };
@@ -925,7 +928,10 @@ __host__ __device__ __forceinline__ int ysolve_kb(int ny, int cplx) {
 // the length of a thread's chain for threads.  At W = 2 a step took (us, rows
 // 4 / 8 / 16): 257^2 29.8 / 30.0 / 30.6, 361 x 287 - / 42.7 / 43.7, 513^2
 // - / 51.4 / 50.2; 32 rows do not fit the registers (1025^2: 168 against 147
-// with 16).
+// with 16).  A channel's complex values spill 160-240 bytes per thread at 16
+// rows: 8 against 16 rows 67.2 / 72.1 at 769 x 481 (FP32 storage 53.3 / 56.4),
+// 81.2 / 83.9 at 641^2, but 123.9 / 121.9 at 1025 x 801 (93.5 / 95.3), so the
+// boxes' rule serves both, and oqg_autotune_ysolve finds the 8 rows of spread 4.
 __host__ __device__ __forceinline__ int ysolve_rows(int ny, int cplx, int W) {
     const int kb = ysolve_kb(ny, cplx);
     int R = 4;
@@ -1445,10 +1451,10 @@ k_xinv_rows(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int
 // step while the others transform; every CTA computes the same scalars, the
 // first writes the next state.  Threads: NL transforms' (at least 128), and
 // the scalar warp.  Bound by latency: on a 193 x 97 channel the 48 CTAs run one
-// transform and 400 points each.  With the transform's length compiled in, 128
-// threads and a warp that runs the scalars lane by layer, the launch takes 15 us
-// (5 of them the launch's own) where the kernel it replaces, any-length, with
-// its modal rows cleared and rewritten in place, took 27.
+// transform and 400 points each.  The launch takes 15 us there (5 of them the
+// launch's own) with the transform's length compiled in, 128 threads and the
+// scalars lane by layer; with an any-length transform, the modal rows cleared
+// and rewritten in place and the scalars in one lane it took 27.
 __host__ __device__ __forceinline__ int xinv_tt(int M, int cyclic) { return cyclic ? (M + XINV_E - 1) / XINV_E : odd_tt(M); }
 __host__ __device__ __forceinline__ int xinv_threads(int M, int cyclic, int nl) {
     const int t = (nl * xinv_tt(M, cyclic) + 31) / 32 * 32;
@@ -1816,7 +1822,7 @@ k_xinv_asm4(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int
     const T *__restrict__ Qm = (const T *)b.F[2 + par];
     const T fac = (T)b.qb_fac;
     const int rv = (nxp + V - 1) / V;                // vectors of a row
-    const FastDiv fdx(rv);
+    const FastDiv fdx(rv);                           // (formed while the previous launch drains)
     const int nvec = rv * nyp;
     pdl_wait();
     const XinvScal *sc = (const XinvScal *)b.scal_g;
