@@ -675,7 +675,7 @@ def measure_basin(workload, prec, steps, warmup, msteps, flush, rank, pg, seed=N
     g = QG(b)
     g.set_state(p, p)
     g.set_forcing(w, None, ts, tn)
-    # the vorticity tile height and the y-solve's warps per column, measured
+    # the vorticity tile height and the spread of the y-solve's columns, measured
     # on this GPU (oqg_autotune, oqg_autotune_ysolve), unless fixed
     if PINNED.get("tile_rows"):
         g.set_tile_rows(PINNED["tile_rows"])
@@ -930,7 +930,7 @@ def main():
                     help="the inverse transforms as a launch of their own (1) or inside the assembly "
                          "kernel (0); default: measured")
     ap.add_argument("--ysolve-warps", type=int, default=0, choices=[0, 1, 2, 4],
-                    help="fix the y-solve's warps per column instead of measuring them")
+                    help="fix the spread of the y-solve's columns instead of measuring it")
     ap.add_argument("--adjoint-only", action="store_true",
                     help="time only the adjoint configuration (one repetition of 40 steps) and "
                          "print its figures; for profiling")

@@ -295,8 +295,8 @@ int oqg_launch_floor(oqg_handle *h, int nsteps, double *us_per_step);
  * state, and records the height for the basin's shape and precision, so
  * handles created afterwards in this process start from it.  *best_vty
  * (may be NULL) gets the height; ms (NULL or >= 18 doubles) gets the time
- * per step of each height at index height.  Results do not depend on the
- * height (each point is computed the same way in any tile). */
+ * per step of each height at index height.  Results of the heights agree to
+ * rounding. */
 int oqg_autotune(oqg_handle *h, double tdt, int nsteps, int *best_vty, double *ms);
 /* Current tile height of the vorticity kernel. */
 int oqg_get_vty(oqg_handle *h, int *vty);

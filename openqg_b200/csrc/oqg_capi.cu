@@ -69,7 +69,7 @@ struct oqg_handle {
     YGeo yg{};                           // the y-solve's launch
     bool xinv_split_needed = false;      // too wide for the one-kernel inverse (xinv_most)
     int na = 0;                          // CTAs of k_xinv_asm
-    int xg = 1;                          // transforms per CTA of k_xfwd and k_xinv_rows
+    int xg = 1;                          // transforms per CTA of the transform launches
     size_t smem_v = 0, smem_x = 0, smem_x64 = 0, smem_i = 0;
     double *stage[2] = {nullptr, nullptr};
     double *hrow = nullptr;     // contiguous host-order copy buffer [nl][nyp][nxp]

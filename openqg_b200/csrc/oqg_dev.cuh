@@ -126,15 +126,15 @@ struct BasinDev {
     double *ent_rows;           // [nyp][2] row sums of the ent area integral and their
                                 // compensations
     void *inh_g;                // modal rows in global memory, [nl][nyp][px] (8-byte
-                                // slots): wide grids, and every box (k_xinv_rows)
+                                // slots): with xinv_sep
     int *err;                   // device error bits
     // launch bookkeeping
-    int xinv_sep;               // the inverse transforms run as k_xinv_rows and the
+    int xinv_sep;               // the inverse transforms run as k_binv or k_xinv_rows and the
                                 // assembly as k_xinv_asm (boxes; always when wide)
     int asm_items;              // k_xinv_asm work items of this basin (256-point runs
                                 // interleaved over them)
     void *scal_g;               // with xinv_sep: the step's scalar phase results,
-                                // written once per step by k_xinv_rows
+                                // written once per step by k_binv or k_xinv_rows
     double tdt_m;               // leapfrog step of this member when a launch
                                 // passes tdt = 0 (ensembles: one per member)
     unsigned wait_limit;        // polls of a first wait for a tile load before

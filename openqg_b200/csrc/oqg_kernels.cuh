@@ -5,8 +5,8 @@
 //   k_vort   vort_step (qg/vorticity.F90:14-103) + p_modes_rhs (qg/modes.F90:248-266)
 //            2-D tiles staged in shared memory; the layer loop runs inside the
 //            CTA so the modal right-hand side is formed in registers.
-//   k_xfwd   forward x-transform of solve_inhomog_box / _cyclic
-//            (qg/inhomog.F90:170-255): DST-I (box) or r2c FFT (channel).
+//   k_bfwd   forward x-transform of solve_inhomog_box (qg/inhomog.F90:170-212),
+//            DST-I; k_xfwd, of solve_inhomog_cyclic (inhomog.F90:214-255), r2c FFT.
 //   k_ysolve Thomas solve in y per (mode, wavenumber) (inhomog.F90:187-199),
 //            chunks of rows in registers, their affine maps scanned.
 //   k_xinv   inverse x-transform + homogeneous correction + modes_to_layers
@@ -18,8 +18,9 @@
 //            homog.F90:280-329), and the suppress_comp_mode schedule
 //            (openqg.F90:485-487).
 //   or, as two launches (the default for boxes, measured for channels):
-//   k_xinv_rows  the inverse x-transforms alone, shaped like k_xfwd, with one
-//            extra CTA per basin for the scalar phase;
+//   k_binv, k_xinv_rows  the inverse x-transforms alone (a box's, a channel's),
+//            shaped like the forward ones, with one extra CTA per basin for the
+//            scalar phase;
 //   k_xinv_asm   the homogeneous correction, modes_to_layers, ocqbdy and the
 //            suppression averages, one thread per point.
 // Every launch takes a work list, so one launch serves one basin or an
@@ -658,7 +659,7 @@ k_vort(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
                             if (QA) {
                                 // + J(beta y, p): the Arakawa sum of a field linear in y is
                                 // -dy (4 (pE - pW) + (pNE - pNW) + (pSE - pSW)); explicit FMAs
-                                // keep the rounding the same in every tile instance
+                                // fix this part's rounding
                                 const T py = fma((T)4, pxc, (pw[2][2] - pw[2][0]) + (pw[0][2] - pw[0][0]));
                                 jac = fma(-sK[10 + 2 * NL], py, jac);
                             }
@@ -928,7 +929,7 @@ __host__ __device__ __forceinline__ int ysolve_kb(int ny, int cplx) {
 // the length of a thread's chain for threads.  At W = 2 a step took (us, rows
 // 4 / 8 / 16): 257^2 29.8 / 30.0 / 30.6, 361 x 287 - / 42.7 / 43.7, 513^2
 // - / 51.4 / 50.2; 32 rows do not fit the registers (1025^2: 168 against 147
-// with 16).  A channel's complex values spill 160-240 bytes per thread at 16
+// with 16).  A channel's complex values spill 160-224 bytes per thread at 16
 // rows: 8 against 16 rows 67.2 / 72.1 at 769 x 481 (FP32 storage 53.3 / 56.4),
 // 81.2 / 83.9 at 641^2, but 123.9 / 121.9 at 1025 x 801 (93.5 / 95.3), so the
 // boxes' rule serves both, and oqg_autotune_ysolve finds the 8 rows of spread 4.
@@ -1288,7 +1289,7 @@ __device__ __noinline__ void scalar_phase(const BasinDev &b, double tdt, int par
     nx->nt = nt + 1;
 }
 
-// ------------------------------------------------------------------ k_xinv_rows
+// ------------------------------------------------------------------ k_binv, k_xinv_rows
 // The inverse x-transforms of the y-solved spectral rows as a launch of
 // their own, shaped like the forward one, into the modal rows b.inh_g, which
 // k_xinv_asm assembles (into out instead when out != null: the solve-only
@@ -1665,7 +1666,7 @@ k_xinv(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
 
 // ------------------------------------------------------------------ k_xinv_asm
 #define XASM_ENS_POINTS 1024   // points per assembly work item of an ensemble's member
-// The assembly of a basin whose inverse transforms ran as k_xinv_rows: the
+// The assembly of a basin whose inverse transforms ran as a launch of their own: the
 // homogeneous correction and modes_to_layers (modes.F90:268-284) of every
 // point from the modal rows in b.inh_g, ocqbdy (vorsubs.F90:58-114) on the
 // walls and the suppress_comp_mode averages (driver.F90:174-189), with the
@@ -1677,7 +1678,7 @@ k_xinv(const BasinDev *__restrict__ bas, const Work *__restrict__ work, int par,
 // per thread 24 warps kept 15 KB in flight on an SM, and a 2049^2 launch of
 // FP32 storage ran at 2.3 TB/s (58.6 us; 40.8 with four).
 // hc: the box's alpha (nl-1), or the channel's c_bt, c_bc1[1..], c_bc2[1..]
-// (homog.F90:280-366, by k_xinv_rows' scalar CTA).
+// (homog.F90:280-366, by that launch's scalar CTA).
 template <class T, int NL>
 __device__ __forceinline__ void xinv_layers(const BasinDev &b, const T *__restrict__ inh, const T *__restrict__ H,
                                             const double *ctm, const double *hc, size_t o2, int j, T *pn) {
