@@ -93,13 +93,22 @@ struct oqg_handle {
     double frc_host[2] = {0.0, 0.0};   // txis, txin as last queued for the device
 };
 
+// Fills and copies of host arrays run on the stream whose kernels read them.
+// On the legacy stream they would not be ordered with a handle's (non-blocking)
+// stream, and may still be under way when the call returns: a fill of the
+// descriptor could land on the descriptor that the handle's stream had copied
+// there, and the first kernels would read null pointers.
 template <class X>
 static X *dalloc(oqg_handle *h, size_t count) {
     void *p = nullptr;
     if (cudaMalloc(&p, count * sizeof(X) + 16) != cudaSuccess) return nullptr;
-    cudaMemset(p, 0, count * sizeof(X) + 16);
+    cudaMemsetAsync(p, 0, count * sizeof(X) + 16, h->st);
     h->allocs.push_back(p);
     return (X *)p;
+}
+// (src is pageable: it has been read when this returns)
+static cudaError_t copy_in(cudaStream_t st, void *dst, const void *src, size_t bytes) {
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
 }
 
 // ----------------------------------------------------------- launch helpers
@@ -630,7 +639,7 @@ static bool make_tmaps(oqg_handle *h) {
     if (!ok) return false;
     void *d = b.tmaps ? const_cast<void *>(b.tmaps) : dalloc<unsigned char>(h, (size_t)OQG_NTMAP * OQG_TMAP_BYTES);
     if (!d) return false;
-    if (cudaMemcpy(d, maps.data(), (size_t)OQG_NTMAP * sizeof(CUtensorMap), cudaMemcpyHostToDevice) != cudaSuccess)
+    if (copy_in(h->st, d, maps.data(), (size_t)OQG_NTMAP * sizeof(CUtensorMap)) != cudaSuccess)
         return false;
     b.tmaps = d;
     return true;
@@ -687,9 +696,9 @@ static int homsol(oqg_handle *h) {
         if (h->mixed) {
             std::vector<float> f(hsb.size());
             for (size_t x = 0; x < f.size(); ++x) f[x] = (float)hsb[x];
-            CK(cudaMemcpy(dst, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice));
+            CK(copy_in(h->st, dst, f.data(), f.size() * sizeof(float)));
         } else {
-            CK(cudaMemcpy(dst, hsb.data(), hsb.size() * sizeof(double), cudaMemcpyHostToDevice));
+            CK(copy_in(h->st, dst, hsb.data(), hsb.size() * sizeof(double)));
         }
     } else {
         std::vector<double> hbt(nyp), hbc1((size_t)nl * nyp, 0.0), hbc2((size_t)nl * nyp, 0.0);
@@ -723,9 +732,9 @@ static int homsol(oqg_handle *h) {
             b.hc1n[m] = p1n / det;
             b.hc2n[m] = p2n / det;
         }
-        CK(cudaMemcpy(const_cast<double *>(b.hbt), hbt.data(), nyp * sizeof(double), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(const_cast<double *>(b.hbc1), hbc1.data(), hbc1.size() * sizeof(double), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(const_cast<double *>(b.hbc2), hbc2.data(), hbc2.size() * sizeof(double), cudaMemcpyHostToDevice));
+        CK(copy_in(h->st, const_cast<double *>(b.hbt), hbt.data(), nyp * sizeof(double)));
+        CK(copy_in(h->st, const_cast<double *>(b.hbc1), hbc1.data(), hbc1.size() * sizeof(double)));
+        CK(copy_in(h->st, const_cast<double *>(b.hbc2), hbc2.data(), hbc2.size() * sizeof(double)));
     }
     // the FP64 solve descriptor shares the constants
     std::memcpy(h->hb64.cdhoc, b.cdhoc, sizeof b.cdhoc);
@@ -1043,8 +1052,9 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     if (P.ddyn) {
         double *d_dd = dalloc<double>(h, n2);
         if (!d_dd) return bail(OQG_ECUDA, "out of device memory");
-        CK(cudaMemcpy2D(d_dd, b.px * sizeof(double), P.ddyn, P.nxp * sizeof(double), P.nxp * sizeof(double),
-                        P.nyp, cudaMemcpyHostToDevice));
+        // (the caller's array, which may be pinned: the setup's solves wait for the copy)
+        CK(cudaMemcpy2DAsync(d_dd, b.px * sizeof(double), P.ddyn, P.nxp * sizeof(double), P.nxp * sizeof(double),
+                             P.nyp, cudaMemcpyHostToDevice, h->st));
         b.ddyn = d_dd;
         b.topo_active = 1;
     }
@@ -1057,10 +1067,10 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     if (h->mixed) {
         float *d_tw32 = dalloc<float>(h, tw.size());
         std::vector<float> tf(tw.begin(), tw.end());
-        CK(cudaMemcpy(d_tw32, tf.data(), tf.size() * sizeof(float), cudaMemcpyHostToDevice));
+        CK(copy_in(h->st, d_tw32, tf.data(), tf.size() * sizeof(float)));
         d_tw = d_tw32;
     }
-    CK(cudaMemcpy(d_tw64, tw.data(), tw.size() * sizeof(double), cudaMemcpyHostToDevice));
+    CK(copy_in(h->st, d_tw64, tw.data(), tw.size() * sizeof(double)));
     b.tw = d_tw;
     double *d_otw64 = nullptr;
     if (!b.cyclic) {
@@ -1075,27 +1085,27 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
         }
         fft_stage_twiddles(b.M, orad, tw);
         d_otw64 = dalloc<double>(h, tw.size());
-        CK(cudaMemcpy(d_otw64, tw.data(), tw.size() * sizeof(double), cudaMemcpyHostToDevice));
+        CK(copy_in(h->st, d_otw64, tw.data(), tw.size() * sizeof(double)));
         b.otw = d_otw64;
         if (h->mixed) {
             float *d_otw32 = dalloc<float>(h, tw.size());
             std::vector<float> tf(tw.begin(), tw.end());
-            CK(cudaMemcpy(d_otw32, tf.data(), tf.size() * sizeof(float), cudaMemcpyHostToDevice));
+            CK(copy_in(h->st, d_otw32, tf.data(), tf.size() * sizeof(float)));
             b.otw = d_otw32;
         }
     }
     pt = pivot_blocks(pt, b.nl, b.nk);
     double *d_pt = dalloc<double>(h, pt.tab.size());
     int *d_po = dalloc<int>(h, pt.off.size()), *d_pl = dalloc<int>(h, pt.len.size());
-    CK(cudaMemcpy(d_pt, pt.tab.data(), pt.tab.size() * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(d_po, pt.off.data(), pt.off.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(d_pl, pt.len.data(), pt.len.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CK(copy_in(h->st, d_pt, pt.tab.data(), pt.tab.size() * sizeof(double)));
+    CK(copy_in(h->st, d_po, pt.off.data(), pt.off.size() * sizeof(int)));
+    CK(copy_in(h->st, d_pl, pt.len.data(), pt.len.size() * sizeof(int)));
     b.piv_tab = d_pt; b.piv_off = d_po; b.piv_len = d_pl;
     if (!b.cyclic) {
         std::vector<double> dw;
         dst_row_sums(b.nk, dw);
         double *d_dw = dalloc<double>(h, dw.size());
-        CK(cudaMemcpy(d_dw, dw.data(), dw.size() * sizeof(double), cudaMemcpyHostToDevice));
+        CK(copy_in(h->st, d_dw, dw.data(), dw.size() * sizeof(double)));
         b.dst_w = d_dw;
         b.hsb = dalloc<char>(h, (size_t)(b.nl - 1) * n2 * h->esz);
     } else {
@@ -1115,7 +1125,7 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     h->d_bad = dalloc<unsigned long long>(h, 1);
     h->d_diag = dalloc<double>(h, 4 * (size_t)b.nl);
     if (!b.st || !b.frc || !b.err || !h->stage[1] || !h->d_diag) return bail(OQG_ECUDA, "out of device memory");
-    CK(cudaMemcpy(d_yp, yp.data(), yp.size() * sizeof(double), cudaMemcpyHostToDevice));
+    CK(copy_in(h->st, d_yp, yp.data(), yp.size() * sizeof(double)));
 
     // ---- launch geometry
     // 16 values per transform thread: one radix-16 butterfly per stage
@@ -1174,11 +1184,11 @@ static int create_impl(const oqg_params *prm, oqg_handle **out, bool batched) {
     h->d_wy = dalloc<Work>(h, wy.size());
     h->d_wi = dalloc<Work>(h, wi.size());
     h->d_wa = dalloc<Work>(h, wa.size());
-    CK(cudaMemcpy(h->d_wv, wv.data(), wv.size() * sizeof(Work), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(h->d_wx, wx.data(), wx.size() * sizeof(Work), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(h->d_wy, wy.data(), wy.size() * sizeof(Work), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(h->d_wi, wi.data(), wi.size() * sizeof(Work), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(h->d_wa, wa.data(), wa.size() * sizeof(Work), cudaMemcpyHostToDevice));
+    CK(copy_in(h->st, h->d_wv, wv.data(), wv.size() * sizeof(Work)));
+    CK(copy_in(h->st, h->d_wx, wx.data(), wx.size() * sizeof(Work)));
+    CK(copy_in(h->st, h->d_wy, wy.data(), wy.size() * sizeof(Work)));
+    CK(copy_in(h->st, h->d_wi, wi.data(), wi.size() * sizeof(Work)));
+    CK(copy_in(h->st, h->d_wa, wa.data(), wa.size() * sizeof(Work)));
 
     b.tmaps = nullptr;
     make_tmaps(h);
@@ -1250,7 +1260,7 @@ int oqg_set_state_full(oqg_handle *h, const double *p, const double *pm, const d
         if (csp) sc.csp[k] = csp[k];
         if (cnp) sc.cnp[k] = cnp[k];
     }
-    CK(cudaMemcpy(b.st + par, &sc, sizeof sc, cudaMemcpyHostToDevice));
+    CK(copy_in(h->st, b.st + par, &sc, sizeof sc));
     return OQG_OK;
 }
 
@@ -1430,11 +1440,11 @@ int oqg_suppress(oqg_handle *h) {
 // Reads and clears the device error word of a basin after its stream has
 // drained: a timeout of a bounded wait is OQG_ETIMEOUT, any other bit
 // OQG_ECUDA.  `who` names the basin in the message.
-static int take_device_error(const BasinDev &b, const std::string &who) {
+static int take_device_error(const BasinDev &b, cudaStream_t st, const std::string &who) {
     int err = 0;
     CK(cudaMemcpy(&err, b.err, sizeof(int), cudaMemcpyDeviceToHost));
     if (!err) return OQG_OK;
-    CK(cudaMemset(b.err, 0, sizeof(int)));
+    CK(cudaMemsetAsync(b.err, 0, sizeof(int), st));
     if (err & OQG_DERR_TIMEOUT)
         return fail(OQG_ETIMEOUT, "a bounded device wait ran out" + who + "; the step's results are invalid");
     return fail(OQG_ECUDA, "device error flag set" + who);
@@ -1443,7 +1453,7 @@ static int take_device_error(const BasinDev &b, const std::string &who) {
 int oqg_sync(oqg_handle *h) {
     if (!h) return fail(OQG_EINVAL, "null handle");
     CK(cudaStreamSynchronize(h->st));
-    return take_device_error(h->hb, "");
+    return take_device_error(h->hb, h->st, "");
 }
 
 int oqg_set_wait_limit(oqg_handle *h, long long polls) {
@@ -1970,7 +1980,7 @@ int oqg_ensemble_create(const oqg_params *members, int nmembers, oqg_ensemble **
         void *d = nullptr;
         if (cudaMalloc(&d, bytes) != cudaSuccess) return nullptr;
         e->allocs.push_back(d);
-        if (cudaMemcpy(d, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
+        if (copy_in(e->st, d, src, bytes) != cudaSuccess) return nullptr;
         return d;
     };
     e->hb.resize(nmembers);
@@ -2094,7 +2104,7 @@ int oqg_ensemble_sync(oqg_ensemble *e) {
     if (!e) return fail(OQG_EINVAL, "null ensemble");
     CK(cudaStreamSynchronize(e->st));
     for (size_t i = 0; i < e->m.size(); ++i) {
-        int rc = take_device_error(e->m[i]->hb, " in member " + std::to_string(i));
+        int rc = take_device_error(e->m[i]->hb, e->st, " in member " + std::to_string(i));
         if (rc) return rc;
     }
     return OQG_OK;
@@ -2493,7 +2503,7 @@ static int set_vty(oqg_handle *h, int vt) {
     h->nv = vort_ctas(b);
     std::vector<Work> wv(h->nv);
     for (int i = 0; i < h->nv; ++i) wv[i] = Work{0, i};
-    CK(cudaMemcpy(h->d_wv, wv.data(), wv.size() * sizeof(Work), cudaMemcpyHostToDevice));
+    CK(copy_in(h->st, h->d_wv, wv.data(), wv.size() * sizeof(Work)));
     if (!retile_tmaps(h)) return fail(OQG_ECUDA, "tensor maps could not be encoded");
     h->smem_v = vort_smem_bytes(vt, (int)h->esz);
     set_attrs(h);
@@ -2699,11 +2709,11 @@ static int ens_set_vty(oqg_ensemble *e, int vt) {
         e->d_wv = (Work *)d;
         e->wv_cap = wv.size();
     }
-    CK(cudaMemcpy(e->d_wv, wv.data(), wv.size() * sizeof(Work), cudaMemcpyHostToDevice));
+    CK(copy_in(e->st, e->d_wv, wv.data(), wv.size() * sizeof(Work)));
     e->nv = (int)wv.size();
     e->smem_v = vort_smem_bytes(vt, (int)e->m[0]->esz);
     OQG_DISPATCH_E(raise_ens_smem_t, e, e);
-    CK(cudaMemcpy(e->d_bas, e->hb.data(), n * sizeof(BasinDev), cudaMemcpyHostToDevice));
+    CK(copy_in(e->st, e->d_bas, e->hb.data(), n * sizeof(BasinDev)));
     for (int i = 0; i < 2; ++i)
         if (e->gexec[i]) { cudaGraphExecDestroy(e->gexec[i]); e->gexec[i] = nullptr; }
     return OQG_OK;
